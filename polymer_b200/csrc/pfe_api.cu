@@ -220,6 +220,10 @@ static void reset_context(pfe_context* ctx) {
   ctx->d_gr_start = ctx->d_gr_n = ctx->d_bk_list = nullptr;
   ctx->d_gr_max = nullptr;
   ctx->d_prec = nullptr;
+  ctx->d_raw = nullptr;
+  ctx->d_raw_steps = ctx->d_raw_cost = nullptr;
+  ctx->d_raw_pair = nullptr;
+  ctx->nraw = 0;
   ctx->ngroups = 0;
   ctx->d_pp = ctx->d_pph = ctx->d_out_c = ctx->d_out_x = nullptr;
   ctx->pp_bytes = ctx->pph_bytes = ctx->out_bytes = 0;
@@ -606,6 +610,7 @@ int32_t pfe_batch_setup(pfe_batch* b, const pfe_args* args, int32_t n) {
     pfe_context* c = nullptr;
     if ((rc = pfe_context_create(b->device, &c)) != PFE_OK) break;
     b->inst.push_back(c);
+    c->in_batch = true;   // its chunk lists are joined, cut and sorted with the others'
     if ((rc = pfe_context_setup(c, &args[k])) != PFE_OK) break;
     if (!c->molecular) {
       set_error("pfe_batch_setup: batches hold molecules only");

@@ -51,12 +51,24 @@ struct PairArrays {
   double* gmax;     // largest bound in the pair's block-pair group (molecules)
 };
 
+// A piece of work of the molecular quartet kernels: bra group G against the ket
+// groups [first, end) of the bucketed list, of which the bra pairs [p0, p1) and
+// the ket pairs [q0, q1) (positions in their groups; q1 beyond a ket group's end
+// means its end).  A group quartet cut into several pieces is digested piece by
+// piece: J and K are linear in its integrals.
+struct __align__(16) Chunk {
+  int G, first, end, inst;   // inst: the instance of a batch (0 otherwise)
+  int p0, p1, q0, q1;
+};
+constexpr int kAllPairs = 1 << 30;   // q1 of a chunk that takes the ket groups whole
+constexpr int kClassPairs = 21;      // (bra class, ket class) pairs, bra class >= ket class
+
 // One launch of the quartet kernel: a (bra class, ket class) pair and its chunks.
 struct ClassLaunch {
   int cb, ck;
   int nchunks_host;
   int* d_nchunks;
-  int4* chunks;  // (bra pair, first ket, end ket, 0)
+  Chunk* chunks;             // costliest first
   double quartets;
   // execution variant: 0 = straight-line thread per quartet, 1 = warp per
   // quartet on the op table, 2 = block per quartet on the op table, 3 = warp
@@ -87,7 +99,6 @@ struct ClassLaunch {
   int wide_wpb, wide_per_warp, wide_vmax, wide_xmax;
   size_t smem_wide;
   int* queue;                // device work queue: one chunk counter per launch (pass), zeroed before each
-  unsigned int* cost;        // screened primitive quartets per chunk (chunks are sorted by it, descending)
   int npass;                 // register passes of the straight-line variant
   int npass_live;            // of which launched: the others keep no component with a coefficient
   int gmul = 32;             // straight-line variant: persistent grid of up to gmul blocks per SM
@@ -169,6 +180,16 @@ struct pfe_context {
   int nlaunch = 0;
   int* d_queue = nullptr;    // 64 chunk counters per class launch (the work queues of launches[])
   double census_quartets = 0.0, census_flops = 0.0, census_ref = 0.0, census_fp32 = 0.0;
+  // the chunks of every class pair before they are cut into pieces and sorted
+  // (molecular set-up; a batch joins those of its instances): per chunk its class
+  // pair, its screened quartets and its length in steps, per class pair the sum of the lengths
+  bool in_batch = false;     // set before set-up: the batch finishes the chunk lists
+  int nraw = 0;
+  pfe::Chunk* d_raw = nullptr;
+  unsigned int* d_raw_steps = nullptr;
+  unsigned int* d_raw_cost = nullptr;
+  unsigned char* d_raw_pair = nullptr;
+  double pair_steps[pfe::kClassPairs] = {};
 
   // host-path staging (pfe_fourindex_eri)
   double* d_pp = nullptr;

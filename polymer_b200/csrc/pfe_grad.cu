@@ -119,9 +119,9 @@ __global__ void __launch_bounds__(256) k_grad(MolLaunch ql, GradTables tabs, Gra
   const int nt = ql.nt;
   const int nchunks = *ql.nchunks;
   for (int c = blockIdx.x; c < nchunks; c += gridDim.x) {
-    const int4 ch = ql.chunks[c];
-    const int G = ch.x;
-    const int g0 = ql.gr_start[G], gn = ql.gr_n[G];
+    const Chunk ch = ql.chunks[c];
+    const int G = ch.G;
+    const int g0 = ql.gr_start[G];
     const PairRec* __restrict__ rec = ql.rec;
     const int2 ij0 = __ldg(reinterpret_cast<const int2*>(&rec[g0].si));
     __syncthreads();   // the previous chunk is done with the shared lists
@@ -138,7 +138,7 @@ __global__ void __launch_bounds__(256) k_grad(MolLaunch ql, GradTables tabs, Gra
     __syncthreads();
     const int na = cnt[0], nb = cnt[1], nab = na * nb;
     for (int t = tid; t < nab; t += blockDim.x) P[GL::OAB + t] = dt_at(D, nt, tA[t / nb], tB[t % nb]);
-    for (int k = ch.y; k < ch.z; ++k) {
+    for (int k = ch.first; k < ch.end; ++k) {
       const int H = ql.bk_list[k];
       const int h0 = ql.gr_start[H], hn = ql.gr_n[H];
       const double hmax = ql.gr_max[H];
@@ -165,12 +165,12 @@ __global__ void __launch_bounds__(256) k_grad(MolLaunch ql, GradTables tabs, Gra
       for (int t = tid; t < nb * nd; t += blockDim.x) P[GL::OBD + t] = dt_at(D, nt, tB[t / nd], tD[t % nd]);
       // this group quartet's gradient, per centre (A, C, D) and axis, J and K (thread 0)
       double g[3][3][2] = {};
-      for (int p = g0; p < g0 + gn; ++p) {
+      for (int p = g0 + ch.p0; p < g0 + ch.p1; ++p) {
         const double sp = pair_bound(rec, p);
         if (sp * hmax < thr) break;
         const PairView bp = load_pair(rec, p);
-        const int qe = (G == H) ? p + 1 : h0 + hn;
-        for (int q = h0; q < qe; ++q) {
+        const int qe = min((G == H) ? p + 1 : h0 + hn, h0 + min(hn, ch.q1));
+        for (int q = h0 + ch.q0; q < qe; ++q) {
           const double sq = pair_bound(rec, q);
           if (sp * sq < thr) break;
           const PairView kq = load_pair(rec, q);

@@ -217,68 +217,219 @@ __device__ __forceinline__ int reach_end(const double* __restrict__ gr_max, cons
   return e;
 }
 
-__global__ void k_chunk_count(const double* __restrict__ gr_max, const int* __restrict__ bk_list, int g0, int ng,
-                              Segs sg, bool same, double inttol, int* __restrict__ nchunk) {
-  const int i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= ng) return;
-  const int G = g0 + i;
+// The class pairs of one set-up: rows are the (class pair, bra group) combinations,
+// those of pair i at [row0[i], row0[i + 1]).
+struct PairRows {
+  int n;
+  int row0[kClassPairs + 1];
+  int cg0[kClassPairs];          // first bra group of the pair
+  unsigned char code[kClassPairs];   // index of the class pair (pair_code)
+  unsigned char same[kClassPairs];   // bra class == ket class
+  Segs seg[kClassPairs];         // the ket class's buckets
+};
+
+__host__ __device__ inline int pair_code(int cb, int ck) { return cb * (cb + 1) / 2 + ck; }
+
+__device__ __forceinline__ int row_pair(const PairRows& pr, int row) {
+  int i = 0;
+  while (i + 1 < pr.n && row >= pr.row0[i + 1]) ++i;
+  return i;
+}
+
+__global__ void k_chunk_count(const double* __restrict__ gr_max, const int* __restrict__ bk_list,
+                              const __grid_constant__ PairRows pr, double inttol, int* __restrict__ nchunk) {
+  const int r = blockIdx.x * blockDim.x + threadIdx.x;
+  if (r >= pr.row0[pr.n]) return;
+  const int i = row_pair(pr, r);
+  const Segs& sg = pr.seg[i];
+  const int G = pr.cg0[i] + r - pr.row0[i];
   const double gmx = gr_max[G];
   int n = 0;
   for (int b = 0; b < NBUCKET; ++b) {
     if (sg.s0[b] >= sg.s1[b]) continue;
-    const int e = reach_end(gr_max, bk_list, sg.s0[b], sg.s1[b], gmx, G, same, inttol);
+    const int e = reach_end(gr_max, bk_list, sg.s0[b], sg.s1[b], gmx, G, pr.same[i], inttol);
     n += (e - sg.s0[b] + 31) >> 5;
   }
-  nchunk[i] = n;
+  nchunk[r] = n;
 }
 
-__global__ void k_chunk_fill(const double* __restrict__ gr_max, const int* __restrict__ bk_list, int g0, int ng,
-                             Segs sg, bool same, double inttol, const int* __restrict__ off, int4* __restrict__ chunks) {
-  const int i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= ng) return;
-  const int G = g0 + i;
+__global__ void k_chunk_fill(const double* __restrict__ gr_max, const int* __restrict__ bk_list,
+                             const int* __restrict__ gr_n, const __grid_constant__ PairRows pr, double inttol,
+                             const int* __restrict__ off, Chunk* __restrict__ chunks,
+                             unsigned char* __restrict__ pair) {
+  const int r = blockIdx.x * blockDim.x + threadIdx.x;
+  if (r >= pr.row0[pr.n]) return;
+  const int i = row_pair(pr, r);
+  const Segs& sg = pr.seg[i];
+  const int G = pr.cg0[i] + r - pr.row0[i];
   const double gmx = gr_max[G];
-  int o = off[i];
+  int o = off[r];
   for (int b = 0; b < NBUCKET; ++b) {
     if (sg.s0[b] >= sg.s1[b]) continue;
-    const int e = reach_end(gr_max, bk_list, sg.s0[b], sg.s1[b], gmx, G, same, inttol);
-    for (int k = sg.s0[b]; k < e; k += 32) chunks[o++] = make_int4(G, k, min(k + 32, e), 0);
+    const int e = reach_end(gr_max, bk_list, sg.s0[b], sg.s1[b], gmx, G, pr.same[i], inttol);
+    for (int k = sg.s0[b]; k < e; k += 32) {
+      chunks[o] = Chunk{G, k, min(k + 32, e), 0, 0, gr_n[G], 0, kAllPairs};
+      pair[o++] = pr.code[i];
+    }
   }
 }
 
-// Primitive quartets of every chunk that pass the screen (the census): lane per
-// ket group, binary search over each ket group's bound-sorted pairs.
-// Screened primitive quartets of every chunk (its cost, also the sort key of
-// the work queue) and their total.
-__global__ void k_chunk_census(const int4* __restrict__ chunks, int nchunks, const int* __restrict__ bk_list,
-                               const int* __restrict__ gr_start, const int* __restrict__ gr_n,
-                               const double* __restrict__ sch, double inttol, unsigned long long* __restrict__ total,
-                               unsigned int* __restrict__ cost) {
+// What the set-up kernels read of a molecule's groups.
+struct GroupView {
+  const int* bk_list;
+  const int* gr_start;
+  const int* gr_n;
+  const double* sch;
+  double inttol;
+};
+
+// Primitive quartets of group quartet (G|H) that pass the screen with the bra
+// pairs [p0, p1) and the ket pairs [q0, q1): binary searches over the ket group's
+// bound-sorted pairs.
+__device__ __forceinline__ unsigned long long piece_quartets(const GroupView& v, int G, int H, int p0, int p1, int q0,
+                                                             int q1) {
+  const int g0 = v.gr_start[G], h0 = v.gr_start[H], hn = v.gr_n[H];
+  unsigned long long n = 0;
+  for (int p = g0 + p0; p < g0 + p1; ++p) {
+    const double sp = v.sch[p];
+    const int qe = min(G == H ? p + 1 : h0 + hn, h0 + min(hn, q1));
+    int lo = h0 + q0, hi = qe;
+    while (lo < hi) {
+      const int mid = (lo + hi) >> 1;
+      if (sp * v.sch[mid] < v.inttol) hi = mid; else lo = mid + 1;
+    }
+    n += (unsigned long long)max(lo - (h0 + q0), 0);
+  }
+  return n;
+}
+
+// Totals of a class pair over its chunks.
+struct PairStat {
+  unsigned long long quartets, steps;
+  unsigned int live;   // pieces with a quartet
+};
+
+// The census of a set-up's chunks (one warp per chunk, one ket group per lane):
+// the screened quartets of every class pair, and the steps of every chunk -- what
+// its costliest lane walks serially in the straight-line kernels, or all of its
+// quartets where a warp or block takes them one at a time (bit `code` of serial).
+__global__ void k_chunk_census(const Chunk* __restrict__ chunks, const unsigned char* __restrict__ pair, int nchunks,
+                               GroupView v, unsigned int serial, unsigned int* __restrict__ steps,
+                               unsigned int* __restrict__ cost, PairStat* __restrict__ stat) {
   const int c = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
   const int lane = threadIdx.x & 31;
   if (c >= nchunks) return;
-  const int4 ch = chunks[c];
-  unsigned long long n = 0;
-  const int li = ch.y + lane;
-  if (li < ch.z) {
-    const int G = ch.x, H = bk_list[li];
-    const int g0 = gr_start[G], gn = gr_n[G], h0 = gr_start[H], hn = gr_n[H];
-    for (int p = g0; p < g0 + gn; ++p) {
-      const double sp = sch[p];
-      const int qe = (G == H) ? p + 1 : h0 + hn;
-      int lo = h0, hi = qe;
-      while (lo < hi) {
-        const int mid = (lo + hi) >> 1;
-        if (sp * sch[mid] < inttol) hi = mid; else lo = mid + 1;
-      }
-      n += (unsigned long long)(lo - h0);
+  const Chunk ch = chunks[c];
+  const int li = ch.first + lane;
+  unsigned long long n = li < ch.end ? piece_quartets(v, ch.G, v.bk_list[li], ch.p0, ch.p1, ch.q0, ch.q1) : 0ull;
+  unsigned long long longest = n;
+  for (int o = 16; o > 0; o >>= 1) {
+    n += __shfl_xor_sync(0xffffffffu, n, o);
+    longest = max(longest, __shfl_xor_sync(0xffffffffu, longest, o));
+  }
+  if (lane == 0) {
+    const int code = pair[c];
+    const unsigned int st = (unsigned int)min((serial >> code) & 1 ? n : longest, 0xffffffffull);
+    steps[c] = st;
+    cost[c] = (unsigned int)min(n, 0xffffffffull);
+    if (n) {
+      atomicAdd(&stat[code].quartets, n);
+      atomicAdd(&stat[code].steps, (unsigned long long)st);
     }
   }
-  for (int o = 16; o > 0; o >>= 1) n += __shfl_xor_sync(0xffffffffu, n, o);
-  if (lane == 0) {
-    if (n) atomicAdd(total, n);
-    cost[c] = (unsigned int)min(n, 0xffffffffull);
+}
+
+// How a chunk of `steps` steps is cut so that no piece walks many more than
+// `most`: into k runs of ket groups (serial classes), then m runs of bra pairs, then
+// l runs of ket pairs.
+struct PieceCut {
+  int k, m, l;
+};
+
+__device__ __forceinline__ PieceCut cut_chunk(const Chunk& ch, unsigned int steps, unsigned int most, bool serial,
+                                              const GroupView& v) {
+  PieceCut pc{1, 1, 1};
+  unsigned int want = steps / most + (steps % most ? 1 : 0);
+  if (want <= 1) return pc;
+  if (serial) {
+    pc.k = (int)min(want, (unsigned int)(ch.end - ch.first));
+    want = (want + pc.k - 1) / pc.k;
   }
+  pc.m = (int)min(want, (unsigned int)(ch.p1 - ch.p0));
+  want = (want + pc.m - 1) / pc.m;
+  int hmax = 1;
+  for (int i = ch.first; i < ch.end; ++i) hmax = max(hmax, v.gr_n[v.bk_list[i]]);
+  pc.l = (int)min(want, (unsigned int)hmax);
+  return pc;
+}
+
+struct PairMost {
+  unsigned int most[kClassPairs];   // longest piece aimed at
+  unsigned int serial;
+};
+
+__global__ void k_piece_count(const Chunk* __restrict__ chunks, const unsigned char* __restrict__ pair,
+                              const unsigned int* __restrict__ steps, int nchunks, GroupView v,
+                              const __grid_constant__ PairMost pm, int* __restrict__ npiece) {
+  const int c = blockIdx.x * blockDim.x + threadIdx.x;
+  if (c >= nchunks) return;
+  const PieceCut pc = cut_chunk(chunks[c], steps[c], pm.most[pair[c]], (pm.serial >> pair[c]) & 1, v);
+  npiece[c] = pc.k * pc.m * pc.l;
+}
+
+// The pieces of every chunk at its offset (one warp per chunk), tagged with the
+// instance, and the key of each: its class pair, then its screened quartets
+// descending (the work queues hand out the costliest first); pieces without a
+// quartet get the last key and are dropped.
+__global__ void k_piece_fill(const Chunk* __restrict__ chunks, const unsigned char* __restrict__ pair,
+                             const unsigned int* __restrict__ steps, const unsigned int* __restrict__ cost, int nchunks,
+                             GroupView v, const __grid_constant__ PairMost pm, int inst, const int* __restrict__ off,
+                             Chunk* __restrict__ out, unsigned long long* __restrict__ key,
+                             PairStat* __restrict__ stat) {
+  const int c = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
+  const int lane = threadIdx.x & 31;
+  if (c >= nchunks) return;
+  const Chunk ch = chunks[c];
+  const int code = pair[c];
+  const PieceCut pc = cut_chunk(ch, steps[c], pm.most[code], (pm.serial >> code) & 1, v);
+  int hmax = 1;
+  if (pc.l > 1)
+    for (int i = ch.first; i < ch.end; ++i) hmax = max(hmax, v.gr_n[v.bk_list[i]]);
+  const int nk = ch.end - ch.first, np = ch.p1 - ch.p0;
+  int o = off[c];
+  unsigned int live = 0;
+  for (int ik = 0; ik < pc.k; ++ik)
+    for (int im = 0; im < pc.m; ++im)
+      for (int il = 0; il < pc.l; ++il, ++o) {
+        Chunk q = ch;
+        q.inst = inst;
+        q.first = ch.first + (int)((long long)nk * ik / pc.k);
+        q.end = ch.first + (int)((long long)nk * (ik + 1) / pc.k);
+        q.p0 = ch.p0 + (int)((long long)np * im / pc.m);
+        q.p1 = ch.p0 + (int)((long long)np * (im + 1) / pc.m);
+        if (pc.l > 1) {
+          q.q0 = (int)((long long)hmax * il / pc.l);
+          q.q1 = (int)((long long)hmax * (il + 1) / pc.l);
+        }
+        const int li = q.first + lane;
+        unsigned long long n = cost[c];
+        if (pc.k * pc.m * pc.l > 1) n = li < q.end ? piece_quartets(v, q.G, v.bk_list[li], q.p0, q.p1, q.q0, q.q1) : 0ull;
+        if (pc.k * pc.m * pc.l > 1)
+          for (int d = 16; d > 0; d >>= 1) n += __shfl_xor_sync(0xffffffffu, n, d);
+        if (lane == 0) {
+          out[o] = q;
+          key[o] = n ? ((unsigned long long)code << 32) | (0xffffffffull - min(n, 0xffffffffull))
+                     : (unsigned long long)kClassPairs << 32;
+        }
+        live += n ? 1u : 0u;
+      }
+  if (lane == 0 && live) atomicAdd(&stat[code].live, live);
+}
+
+__global__ void k_piece_gather(const Chunk* __restrict__ in, const int* __restrict__ perm, int n,
+                               Chunk* __restrict__ out) {
+  const int t = blockIdx.x * blockDim.x + threadIdx.x;
+  if (t < n) out[t] = in[perm[t]];
 }
 
 // ------------------------------------------------------------------ density in target space
@@ -402,7 +553,7 @@ struct TeamLayout {
 // of the team (a warp, or the block) share one primitive quartet at a time and
 // run the op table level by level; X accumulates in shared (or global) memory.
 template <int LA, int LB, int LC, int LD, bool BLOCK>
-__device__ __forceinline__ void gq_team(const MolLaunch& ql, const OpTableDev& tab, const int4 ch, double* sm,
+__device__ __forceinline__ void gq_team(const MolLaunch& ql, const OpTableDev& tab, const Chunk ch, double* sm,
                                         double* xg, OpGeom& geo, int* prm, double* sw, int tid, int team) {
   constexpr int NA = ncum(LA), NB = ncum(LB), NC = ncum(LC), ND = ncum(LD);
   constexpr int NI = NA * NB * NC * ND;
@@ -421,8 +572,8 @@ __device__ __forceinline__ void gq_team(const MolLaunch& ql, const OpTableDev& t
   const double* __restrict__ scoef = ql.scoef;   // held in registers (ql may live in global memory)
   const double* __restrict__ boys = ql.boys;
   const double c2pi = 2.0 / sqrt(REF_PI);
-  const int G = ch.x;
-  const int g0 = ql.gr_start[G], gn = ql.gr_n[G];
+  const int G = ch.G;
+  const int g0 = ql.gr_start[G];
   {
     const int I0 = pr.si[g0], J0 = pr.sj[g0];
     for (int x = tid; x < NA; x += team) prm[x] = ql.stidx[I0 * MAXCOMP + x];
@@ -443,7 +594,7 @@ __device__ __forceinline__ void gq_team(const MolLaunch& ql, const OpTableDev& t
   pure = pure && tab.ops_p2 != nullptr;   // from here: the bra-and-ket table may apply
   for (int t = tid; t < NA * NB; t += team)
     P[DG::OAB + t] = dt_at(D, nt, prm[t / NB], prm[DG::SB + t % NB]);
-  for (int k = ch.y; k < ch.z; ++k) {
+  for (int k = ch.first; k < ch.end; ++k) {
     const int H = ql.bk_list[k];
     const int h0 = ql.gr_start[H], hn = ql.gr_n[H];
     const double hmax = ql.gr_max[H];
@@ -481,7 +632,7 @@ __device__ __forceinline__ void gq_team(const MolLaunch& ql, const OpTableDev& t
     const unsigned short* __restrict__ t_out = pure2 ? tab.out_p2 : b_out;
     const int t_nlevels = pure2 ? tab.nlevels_p2 : b_nlevels;
     bool any = false;   // team-uniform: every loop decision below is
-    for (int p = g0; p < g0 + gn; ++p) {
+    for (int p = g0 + ch.p0; p < g0 + ch.p1; ++p) {
       const double sp = pr.schwarz[p];
       if (sp * hmax < thr) break;
       const int I = pr.si[p], J = pr.sj[p];
@@ -489,8 +640,8 @@ __device__ __forceinline__ void gq_team(const MolLaunch& ql, const OpTableDev& t
         cab[t] = scoef[I * MAXCOMP + t / NB] * scoef[J * MAXCOMP + t % NB];
       const double zb = pr.zeta[p];
       const double Px = pr.P[0][p], Py = pr.P[1][p], Pz = pr.P[2][p];
-      const int qe = (G == H) ? p + 1 : h0 + hn;
-      for (int q = h0; q < qe; ++q) {
+      const int qe = min((G == H) ? p + 1 : h0 + hn, h0 + min(hn, ch.q1));
+      for (int q = h0 + ch.q0; q < qe; ++q) {
         if (sp * pr.schwarz[q] < thr) break;   // the reference's screen (thr = INTTOL; team-uniform)
         const int K = pr.si[q], L = pr.sj[q];
         const double ze = pr.zeta[q];
@@ -550,8 +701,8 @@ __global__ void __launch_bounds__(256) k_gq_warp(MolLaunch ql, OpTableDev tab, i
   const int nchunks = *ql.nchunks;
   const int stride = gridDim.x * wpb * ql.numprocs;
   for (int c = (blockIdx.x * wpb + wid) * ql.numprocs + ql.myid; c < nchunks; c += stride) {
-    const int4 ch = ql.chunks[c];
-    gq_team<LA, LB, LC, LD, false>(ql.insts ? ql.insts[ch.w] : ql, tab, ch, smem + (size_t)wid * per_warp, nullptr,
+    const Chunk ch = ql.chunks[c];
+    gq_team<LA, LB, LC, LD, false>(ql.insts ? ql.insts[ch.inst] : ql, tab, ch, smem + (size_t)wid * per_warp, nullptr,
                                    s_geo[wid], s_prm[wid], s_w + wid, lane, 32);
   }
 }
@@ -567,7 +718,7 @@ __global__ void __launch_bounds__(256) k_gq_block(MolLaunch ql, OpTableDev tab, 
   __shared__ double s_w[1];
   const int nchunks = *ql.nchunks;
   for (int c = blockIdx.x * ql.numprocs + ql.myid; c < nchunks; c += gridDim.x * ql.numprocs)
-    gq_team<LA, LB, LC, LD, true>(ql.insts ? ql.insts[ql.chunks[c].w] : ql, tab, ql.chunks[c], smem,
+    gq_team<LA, LB, LC, LD, true>(ql.insts ? ql.insts[ql.chunks[c].inst] : ql, tab, ql.chunks[c], smem,
                                   xg ? xg + (size_t)blockIdx.x * (ncum(LA) * ncum(LB) * ncum(LC) * ncum(LD)) : nullptr,
                                   s_geo, s_prm, s_w, threadIdx.x, blockDim.x);
 }
@@ -723,6 +874,136 @@ static int size_wide(ClassLaunch& cl, const int kept_max[3], const bool lower_ke
   return PFE_OK;
 }
 
+static void free_raw(pfe_context* ctx) {
+  for (void* p : {(void*)ctx->d_raw, (void*)ctx->d_raw_steps, (void*)ctx->d_raw_cost, (void*)ctx->d_raw_pair})
+    ctx->free_now(p);
+  ctx->d_raw = nullptr;
+  ctx->d_raw_steps = ctx->d_raw_cost = nullptr;
+  ctx->d_raw_pair = nullptr;
+  ctx->nraw = 0;
+}
+
+static GroupView group_view(const pfe_context* ctx) {
+  return GroupView{ctx->d_bk_list, ctx->d_gr_start, ctx->d_gr_n, ctx->pairs.schwarz, ctx->inttol};
+}
+
+// The chunk lists the kernels run, from the raw chunks of one molecule or of every
+// instance of a batch (`own`, a context or a batch, holds the memory): chunks much
+// longer than an even share of their class's work are cut into pieces, and every
+// class's pieces are sorted costliest first for its work queue.
+//
+// Why cut: a lane walks all primitive quartets of its group quartet in turn (up to
+// thousands where both groups are products of long contractions), so in a small
+// molecule, whose classes have fewer chunks than the GPU has warps, a launch lasts
+// as long as its longest lane.  The aim is a quarter of what each of the resident warps gets
+// on average, but no less than kLeastSteps: a piece pays its own set-up and
+// digestion (about two microseconds).  Ranks of one build must cut alike, so the
+// rule reads the work alone, not the device.
+static unsigned int longest_piece(double steps) {
+  constexpr double kWarps = 148.0 * 8.0;   // resident warps of the 255-register kernels on a B200
+  constexpr unsigned int kLeastSteps = 24;
+  const double share = steps / (4.0 * kWarps);
+  return (unsigned int)std::min(4.0e9, std::max((double)kLeastSteps, share));
+}
+
+template <typename Owner>
+static int finish_chunks(Owner* own, pfe_context* const* inst, int ninst, ClassLaunch* launches, int nlaunch,
+                         cudaStream_t s) {
+  long long nraw = 0;
+  double steps[kClassPairs] = {};
+  PairMost pm{};
+  for (int k = 0; k < ninst; ++k) {
+    nraw += inst[k]->nraw;
+    for (int i = 0; i < kClassPairs; ++i) steps[i] += inst[k]->pair_steps[i];
+  }
+  if (nraw >= (1LL << 31)) { set_error("too many chunks"); return PFE_EINVAL; }
+  for (int cb = 0; cb < 6; ++cb)
+    for (int ck = 0; ck <= cb; ++ck) {
+      pm.most[pair_code(cb, ck)] = longest_piece(steps[pair_code(cb, ck)]);
+      if (!straight_launcher(cb, ck)) pm.serial |= 1u << pair_code(cb, ck);
+    }
+  PairStat stat[kClassPairs] = {};
+  Chunk* sorted = nullptr;
+  if (nraw > 0) {
+    struct Scratch {   // freed on every way out
+      std::vector<void*> p;
+      ~Scratch() { for (void* q : p) cudaFree(q); }
+    } scratch;
+    auto tmp = [&](auto** p, size_t bytes) -> cudaError_t {
+      if (cudaError_t f = injected_alloc_failure()) return f;
+      const cudaError_t e = cudaMalloc((void**)p, bytes ? bytes : 16);
+      if (e == cudaSuccess) scratch.p.push_back((void*)*p);
+      return e;
+    };
+    int *npiece = nullptr, *off = nullptr;
+    PairStat* d_stat = nullptr;
+    void* cub_tmp = nullptr;
+    PFE_CUDA(tmp(&npiece, sizeof(int) * (nraw + 1)));
+    PFE_CUDA(tmp(&off, sizeof(int) * (nraw + 1)));
+    PFE_CUDA(tmp(&d_stat, sizeof(stat)));
+    PFE_CUDA(cudaMemsetAsync(npiece + nraw, 0, sizeof(int), s));
+    PFE_CUDA(cudaMemsetAsync(d_stat, 0, sizeof(stat), s));
+    long long o = 0;
+    for (int k = 0; k < ninst; ++k) {
+      const pfe_context* c = inst[k];
+      if (c->nraw == 0) continue;
+      k_piece_count<<<(c->nraw + 127) / 128, 128, 0, s>>>(c->d_raw, c->d_raw_pair, c->d_raw_steps, c->nraw,
+                                                          group_view(c), pm, npiece + o);
+      o += c->nraw;
+    }
+    PFE_CUDA(cudaGetLastError());
+    size_t tb = 0;
+    cub::DeviceScan::ExclusiveSum(nullptr, tb, npiece, off, (int)nraw + 1, s);
+    PFE_CUDA(tmp(&cub_tmp, tb + 16));
+    PFE_CUDA(cub::DeviceScan::ExclusiveSum(cub_tmp, tb, npiece, off, (int)nraw + 1, s));
+    int total = 0;
+    PFE_CUDA(cudaMemcpyAsync(&total, off + nraw, sizeof(int), cudaMemcpyDeviceToHost, s));
+    PFE_CUDA(cudaStreamSynchronize(s));
+    Chunk* pieces = nullptr;
+    unsigned long long *key = nullptr, *key2 = nullptr;
+    int *iota = nullptr, *perm = nullptr;
+    PFE_CUDA(tmp(&pieces, sizeof(Chunk) * total));
+    PFE_CUDA(tmp(&key, sizeof(unsigned long long) * total));
+    PFE_CUDA(tmp(&key2, sizeof(unsigned long long) * total));
+    PFE_CUDA(tmp(&iota, sizeof(int) * total));
+    PFE_CUDA(tmp(&perm, sizeof(int) * total));
+    PFE_CUDA(own->alloc((void**)&sorted, sizeof(Chunk) * total));
+    o = 0;
+    for (int k = 0; k < ninst; ++k) {
+      const pfe_context* c = inst[k];
+      if (c->nraw == 0) continue;
+      k_piece_fill<<<(c->nraw + 3) / 4, 128, 0, s>>>(c->d_raw, c->d_raw_pair, c->d_raw_steps, c->d_raw_cost, c->nraw,
+                                                     group_view(c), pm, k, off + o, pieces, key, d_stat);
+      o += c->nraw;
+    }
+    k_mol_iota<<<(total + 255) / 256, 256, 0, s>>>(iota, total);
+    PFE_CUDA(cudaGetLastError());
+    cub::DeviceRadixSort::SortPairs(nullptr, tb, key, key2, iota, perm, total, 0, 37, s);
+    void* sort_tmp = nullptr;
+    PFE_CUDA(tmp(&sort_tmp, tb + 16));
+    PFE_CUDA(cub::DeviceRadixSort::SortPairs(sort_tmp, tb, key, key2, iota, perm, total, 0, 37, s));
+    k_piece_gather<<<(total + 255) / 256, 256, 0, s>>>(pieces, perm, total, sorted);
+    PFE_CUDA(cudaGetLastError());
+    PFE_CUDA(cudaMemcpyAsync(stat, d_stat, sizeof(stat), cudaMemcpyDeviceToHost, s));
+    PFE_CUDA(cudaStreamSynchronize(s));
+  }
+  int start[kClassPairs + 1] = {0};
+  for (int i = 0; i < kClassPairs; ++i) start[i + 1] = start[i] + (int)stat[i].live;
+  int n[64] = {0};
+  int* d_n = nullptr;
+  PFE_CUDA(own->alloc((void**)&d_n, sizeof(n)));
+  for (int i = 0; i < nlaunch; ++i) {
+    ClassLaunch& cl = launches[i];
+    const int code = pair_code(cl.cb, cl.ck);
+    n[i] = cl.nchunks_host = (int)stat[code].live;
+    cl.chunks = sorted + start[code];
+    cl.d_nchunks = d_n + i;
+  }
+  PFE_CUDA(cudaMemcpyAsync(d_n, n, sizeof(n), cudaMemcpyHostToDevice, s));
+  PFE_CUDA(cudaStreamSynchronize(s));
+  return PFE_OK;
+}
+
 int molecular_setup(pfe_context* ctx, const pfe_args* a) {
   (void)a;
   cudaStream_t s = ctx->stream;
@@ -857,67 +1138,68 @@ int molecular_setup(pfe_context* ctx, const pfe_args* a) {
     if (seg[c].s1[b] == 0) seg[c].s0[b] = i;
     seg[c].s1[b] = i + 1;
   }
-  // chunk lists for every class pair cb >= ck
+  // the chunks of every class pair cb >= ck in one list, a class pair after another
   ctx->nlaunch = 0;
   ctx->census_quartets = ctx->census_flops = ctx->census_ref = 0.0;
   PFE_CUDA(ctx->alloc((void**)&ctx->d_queue, sizeof(int) * 64 * 64));
   PFE_CUDA(cudaMemsetAsync(ctx->d_queue, 0, sizeof(int) * 64 * 64, s));
-  int maxg = 1;
-  for (int c = 0; c < 6; ++c) maxg = std::max(maxg, cgn[c]);
-  int *nchunk = nullptr, *offs = nullptr;
-  unsigned long long* d_total = nullptr;
-  PFE_CUDA(ctx->alloc((void**)&nchunk, sizeof(int) * (maxg + 1)));
-  PFE_CUDA(ctx->alloc((void**)&offs, sizeof(int) * (maxg + 1)));
-  PFE_CUDA(ctx->alloc((void**)&d_total, sizeof(unsigned long long)));
+  PairRows rows{};
+  unsigned int serial = 0;
   for (int cb = 0; cb < 6; ++cb)
     for (int ck = 0; ck <= cb; ++ck) {
-      const int nbg = cgn[cb];
       bool any = false;
       for (int b = 0; b < NBUCKET; ++b) any = any || seg[ck].s1[b] > seg[ck].s0[b];
-      if (nbg == 0 || !any) continue;
-      k_chunk_count<<<(nbg + 127) / 128, 128, 0, s>>>(ctx->d_gr_max, ctx->d_bk_list, cg0[cb], nbg, seg[ck], cb == ck,
-                                                      ctx->inttol, nchunk);
-      PFE_CUDA(cudaMemsetAsync(nchunk + nbg, 0, sizeof(int), s));
-      if ((rc = exclusive_sum(ctx, nchunk, offs, nbg + 1, s)) != PFE_OK) return rc;
-      int total = 0;
-      PFE_CUDA(cudaMemcpyAsync(&total, offs + nbg, sizeof(int), cudaMemcpyDeviceToHost, s));
+      if (cgn[cb] == 0 || !any) continue;
+      const int i = rows.n++;
+      rows.row0[i + 1] = rows.row0[i] + cgn[cb];
+      rows.cg0[i] = cg0[cb];
+      rows.code[i] = (unsigned char)pair_code(cb, ck);
+      rows.same[i] = cb == ck;
+      rows.seg[i] = seg[ck];
+      if (!straight_launcher(cb, ck)) serial |= 1u << pair_code(cb, ck);
+    }
+  const int nrow = rows.row0[rows.n];
+  PairStat stat[kClassPairs] = {};
+  if (nrow > 0) {
+    int *nchunk = nullptr, *offs = nullptr;
+    PairStat* d_stat = nullptr;
+    PFE_CUDA(ctx->alloc((void**)&nchunk, sizeof(int) * (nrow + 1)));
+    PFE_CUDA(ctx->alloc((void**)&offs, sizeof(int) * (nrow + 1)));
+    PFE_CUDA(ctx->alloc((void**)&d_stat, sizeof(stat)));
+    PFE_CUDA(cudaMemsetAsync(nchunk + nrow, 0, sizeof(int), s));
+    PFE_CUDA(cudaMemsetAsync(d_stat, 0, sizeof(stat), s));
+    k_chunk_count<<<(nrow + 127) / 128, 128, 0, s>>>(ctx->d_gr_max, ctx->d_bk_list, rows, ctx->inttol, nchunk);
+    PFE_CUDA(cudaGetLastError());
+    if ((rc = exclusive_sum(ctx, nchunk, offs, nrow + 1, s)) != PFE_OK) return rc;
+    int total = 0;
+    PFE_CUDA(cudaMemcpyAsync(&total, offs + nrow, sizeof(int), cudaMemcpyDeviceToHost, s));
+    PFE_CUDA(cudaStreamSynchronize(s));
+    ctx->nraw = total;
+    if (total > 0) {
+      PFE_CUDA(ctx->alloc((void**)&ctx->d_raw, sizeof(Chunk) * total));
+      PFE_CUDA(ctx->alloc((void**)&ctx->d_raw_pair, total));
+      PFE_CUDA(ctx->alloc((void**)&ctx->d_raw_steps, sizeof(unsigned int) * total));
+      PFE_CUDA(ctx->alloc((void**)&ctx->d_raw_cost, sizeof(unsigned int) * total));
+      k_chunk_fill<<<(nrow + 127) / 128, 128, 0, s>>>(ctx->d_gr_max, ctx->d_bk_list, ctx->d_gr_n, rows, ctx->inttol,
+                                                      offs, ctx->d_raw, ctx->d_raw_pair);
+      k_chunk_census<<<(total + 3) / 4, 128, 0, s>>>(ctx->d_raw, ctx->d_raw_pair, total, group_view(ctx), serial,
+                                                     ctx->d_raw_steps, ctx->d_raw_cost, d_stat);
+      PFE_CUDA(cudaGetLastError());
+      PFE_CUDA(cudaMemcpyAsync(stat, d_stat, sizeof(stat), cudaMemcpyDeviceToHost, s));
       PFE_CUDA(cudaStreamSynchronize(s));
-      if (total == 0) continue;
+    }
+    for (void* p : {(void*)nchunk, (void*)offs, (void*)d_stat}) ctx->free_now(p);
+  }
+  for (int i = 0; i < kClassPairs; ++i) ctx->pair_steps[i] = (double)stat[i].steps;
+  for (int cb = 0; cb < 6; ++cb)
+    for (int ck = 0; ck <= cb; ++ck) {
+      const double nq = (double)stat[pair_code(cb, ck)].quartets;
+      if (nq == 0.0) continue;
       ClassLaunch cl{};
       cl.gmul = 32;   // what the autotuner picks for most classes on C20H42 and the water batch
       cl.cb = cb;
       cl.ck = ck;
-      cl.nchunks_host = total;
-      PFE_CUDA(ctx->alloc((void**)&cl.chunks, sizeof(int4) * total));
-      PFE_CUDA(ctx->alloc((void**)&cl.d_nchunks, sizeof(int)));
-      PFE_CUDA(cudaMemcpyAsync(cl.d_nchunks, &cl.nchunks_host, sizeof(int), cudaMemcpyHostToDevice, s));
-      k_chunk_fill<<<(nbg + 127) / 128, 128, 0, s>>>(ctx->d_gr_max, ctx->d_bk_list, cg0[cb], nbg, seg[ck], cb == ck,
-                                                     ctx->inttol, offs, cl.chunks);
-      PFE_CUDA(cudaMemsetAsync(d_total, 0, sizeof(unsigned long long), s));
-      unsigned int *cost = nullptr, *cost_sorted = nullptr;
-      int4* sorted = nullptr;
-      PFE_CUDA(ctx->alloc((void**)&cost, sizeof(unsigned int) * total));
-      PFE_CUDA(ctx->alloc((void**)&cost_sorted, sizeof(unsigned int) * total));
-      PFE_CUDA(ctx->alloc((void**)&sorted, sizeof(int4) * total));
-      k_chunk_census<<<(total + 3) / 4, 128, 0, s>>>(cl.chunks, total, ctx->d_bk_list, ctx->d_gr_start, ctx->d_gr_n,
-                                                     ctx->pairs.schwarz, ctx->inttol, d_total, cost);
-      PFE_CUDA(cudaGetLastError());
-      {  // the work queue hands out the costliest chunks first (stable: equal costs keep their order)
-        size_t tb = 0;
-        cub::DeviceRadixSort::SortPairsDescending(nullptr, tb, cost, cost_sorted, cl.chunks, sorted, total, 0, 32, s);
-        void* tmp = nullptr;
-        PFE_CUDA(ctx->alloc(&tmp, tb + 16));
-        PFE_CUDA(cub::DeviceRadixSort::SortPairsDescending(tmp, tb, cost, cost_sorted, cl.chunks, sorted, total, 0, 32,
-                                                           s));
-        PFE_CUDA(cudaMemcpyAsync(cl.chunks, sorted, sizeof(int4) * total, cudaMemcpyDeviceToDevice, s));
-        PFE_CUDA(cudaStreamSynchronize(s));
-        for (void* p : {(void*)tmp, (void*)cost, (void*)sorted}) ctx->free_now(p);
-        cl.cost = cost_sorted;   // kept: a batch sorts its joined chunk list by it
-      }
-      unsigned long long nq = 0;
-      PFE_CUDA(cudaMemcpyAsync(&nq, d_total, sizeof(unsigned long long), cudaMemcpyDeviceToHost, s));
-      PFE_CUDA(cudaStreamSynchronize(s));
-      cl.quartets = (double)nq;
+      cl.quartets = nq;
       cl.has_straight = straight_launcher(cb, ck) != nullptr;
       cl.npass = cl.has_straight ? straight_npass(cb, ck) : 0;
       cl.npass_live = 0;   // register passes actually launched (the rest keep no coefficient)
@@ -993,14 +1275,19 @@ int molecular_setup(pfe_context* ctx, const pfe_args* a) {
       for (int v = 0; v < 4; ++v) cl.tuned_ms[v] = 0.f;
       cl.queue = ctx->d_queue + 64 * ctx->nlaunch;
       ctx->launches[ctx->nlaunch++] = cl;
-      ctx->census_quartets += (double)nq;
-      ctx->census_flops += (double)nq * class_flops(cb, ck);
+      ctx->census_quartets += nq;
+      ctx->census_flops += nq * class_flops(cb, ck);
     }
+  if (!ctx->in_batch) {
+    pfe_context* const self = ctx;
+    if ((rc = finish_chunks(ctx, &self, 1, ctx->launches, ctx->nlaunch, s)) != PFE_OK) return rc;
+    free_raw(ctx);
+  }
   ctx->free_now(d_count);
   free_pairs(ctx, &raw);
   for (void* p : {(void*)gbits, (void*)k_sch, (void*)k_gmax, (void*)k64, (void*)perm_a, (void*)perm_b, (void*)k32,
                   (void*)k32b, (void*)k8, (void*)k8b, (void*)head, (void*)gix, (void*)gr_cls, (void*)bkey,
-                  (void*)bkey_sorted, (void*)giota, (void*)nchunk, (void*)offs, (void*)d_total})
+                  (void*)bkey_sorted, (void*)giota})
     ctx->free_now(p);
   ctx->free_pending();
   return PFE_OK;
@@ -1298,13 +1585,8 @@ int molecular_density_ok(pfe_context* ctx, cudaStream_t s, bool* ok) {
 
 namespace pfe {
 
-__global__ void k_tag_chunks(int4* __restrict__ chunks, int n, int instance) {
-  const int t = blockIdx.x * blockDim.x + threadIdx.x;
-  if (t < n) chunks[t].w = instance;
-}
-
-// Join the instances' chunk lists per (bra class, ket class): device copies and
-// tags queued on one stream, one synchronisation at the end.
+// Join the instances' chunks into one list per (bra class, ket class), every chunk
+// tagged with its instance.
 int batch_setup(pfe_batch* b) {
   b->nlaunch = 0;
   PFE_CUDA(b->alloc((void**)&b->d_queue, sizeof(int) * 64 * 64));
@@ -1316,16 +1598,15 @@ int batch_setup(pfe_batch* b) {
   } guard{st};
   for (int cb = 0; cb < 6; ++cb)
     for (int ck = 0; ck <= cb; ++ck) {
-      long long total = 0;
+      double quartets = 0.0;
       const ClassLaunch* tmpl = nullptr;
       for (pfe_context* c : b->inst)
         for (int i = 0; i < c->nlaunch; ++i)
           if (c->launches[i].cb == cb && c->launches[i].ck == ck) {
-            total += c->launches[i].nchunks_host;
+            quartets += c->launches[i].quartets;
             if (!tmpl) tmpl = &c->launches[i];
           }
-      if (!tmpl || total == 0) continue;
-      if (total >= (1LL << 31)) { set_error("batch: too many chunks in one quartet class"); return PFE_EINVAL; }
+      if (!tmpl) continue;
       ClassLaunch cl = *tmpl;
       {  // launched passes over the whole batch: a pass is skipped only if no instance needs it
         int bits = 0;
@@ -1344,45 +1625,17 @@ int batch_setup(pfe_batch* b) {
         if (rc != PFE_OK) return rc;
         if (!cl.has_wide && cl.variant == 3) cl.variant = cl.has_straight ? 0 : 2;
       }
-      cl.nchunks_host = (int)total;
-      cl.quartets = 0.0;
+      cl.quartets = quartets;
       cl.queue = b->d_queue + 64 * b->nlaunch;
-      PFE_CUDA(b->alloc((void**)&cl.chunks, sizeof(int4) * total));
-      PFE_CUDA(b->alloc((void**)&cl.d_nchunks, sizeof(int)));
-      unsigned int* jcost = nullptr;
-      PFE_CUDA(b->alloc((void**)&jcost, sizeof(unsigned int) * total));
-      PFE_CUDA(cudaMemcpy(cl.d_nchunks, &cl.nchunks_host, sizeof(int), cudaMemcpyHostToDevice));   // pageable: synchronous
-      long long o = 0;
-      for (size_t k = 0; k < b->inst.size(); ++k) {
-        pfe_context* c = b->inst[k];
-        for (int i = 0; i < c->nlaunch; ++i) {
-          const ClassLaunch& li = c->launches[i];
-          if (li.cb != cb || li.ck != ck) continue;
-          PFE_CUDA(cudaMemcpyAsync(cl.chunks + o, li.chunks, sizeof(int4) * li.nchunks_host, cudaMemcpyDeviceToDevice,
-                                   st));
-          PFE_CUDA(cudaMemcpyAsync(jcost + o, li.cost, sizeof(unsigned int) * li.nchunks_host,
-                                   cudaMemcpyDeviceToDevice, st));
-          k_tag_chunks<<<(li.nchunks_host + 255) / 256, 256, 0, st>>>(cl.chunks + o, li.nchunks_host, (int)k);
-          PFE_CUDA(cudaGetLastError());
-          o += li.nchunks_host;
-          cl.quartets += li.quartets;
-        }
-      }
-      {  // one queue over the whole batch, costliest chunks first
-        unsigned int* ks = nullptr;
-        int4* vs = nullptr;
-        PFE_CUDA(b->alloc((void**)&ks, sizeof(unsigned int) * total));
-        PFE_CUDA(b->alloc((void**)&vs, sizeof(int4) * total));
-        size_t tb = 0;
-        cub::DeviceRadixSort::SortPairsDescending(nullptr, tb, jcost, ks, cl.chunks, vs, (int)total, 0, 32, st);
-        void* tmp = nullptr;
-        PFE_CUDA(b->alloc(&tmp, tb + 16));
-        PFE_CUDA(cub::DeviceRadixSort::SortPairsDescending(tmp, tb, jcost, ks, cl.chunks, vs, (int)total, 0, 32, st));
-        PFE_CUDA(cudaMemcpyAsync(cl.chunks, vs, sizeof(int4) * total, cudaMemcpyDeviceToDevice, st));
-        cl.cost = ks;
-      }
       b->launches[b->nlaunch++] = cl;
     }
+  {
+    const int rc = finish_chunks(b, b->inst.data(), (int)b->inst.size(), b->launches, b->nlaunch, st);
+    if (rc != PFE_OK) return rc;
+  }
+  for (pfe_context* c : b->inst) {   // the joined lists replace them
+    free_raw(c);
+  }
   PFE_CUDA(b->alloc(&b->d_insts, sizeof(MolLaunch) * b->inst.size()));
   PFE_CUDA(b->alloc((void**)&b->d_off, sizeof(long long) * b->off.size()));
   PFE_CUDA(cudaMemcpy(b->d_off, b->off.data(), sizeof(long long) * b->off.size(), cudaMemcpyHostToDevice));

@@ -68,13 +68,13 @@ struct MolLaunch {
   double dtol;            // skip quartets with bound * max|P| < dtol (0: the reference's screen only)
   double mcut;            // FP32 recursion where bound * max|P| < mcut (0: FP64 only)
   unsigned long long* n32;  // quartets run in FP32
-  const int4* chunks;     // (bra group, first list entry, end list entry, 0), costliest first
+  const Chunk* chunks;    // costliest first
   const int* nchunks;
   int* queue;             // chunk counters (one per pass), zero at launch: warps take chunks in order
   double inttol;
   int nt;
   int myid, numprocs;
-  const MolLaunch* insts;   // batches: the launch record of every instance (chunk .w), else null
+  const MolLaunch* insts;   // batches: the launch record of every instance (Chunk::inst), else null
   int lower_kept_bits;      // bit L: some shell of top L has a coefficient on a lower component
 };
 
@@ -299,10 +299,10 @@ __global__ void __launch_bounds__(128, GqOccupancy<LA, LB, LC, LD>::blocks) k_gq
     if (lane == 0) t = atomicAdd(lq.queue + PASS, 1);
     const int c = __shfl_sync(0xffffffffu, t, 0) * lq.numprocs + lq.myid;
     if (c >= nchunks) break;
-    const int4 ch = lq.chunks[c];
+    const Chunk ch = lq.chunks[c];
     // this chunk's instance: batches read its launch record from global memory
     const MolLaunch& ql = [&]() -> const MolLaunch& {
-      if constexpr (BATCH) return lq.insts[ch.w];
+      if constexpr (BATCH) return lq.insts[ch.inst];
       else return lq;
     }();
     // the tables the loops read, held in registers (ql may live in global memory)
@@ -312,8 +312,8 @@ __global__ void __launch_bounds__(128, GqOccupancy<LA, LB, LC, LD>::blocks) k_gq
     const int* __restrict__ stidx = ql.stidx;
     const double mcut = ql.mcut;
     const int nt = ql.nt;
-    const int G = ch.x;
-    const int g0 = ql.gr_start[G], gn = ql.gr_n[G];
+    const int G = ch.G;
+    const int g0 = ql.gr_start[G];
     const int2 ijg = __ldg(reinterpret_cast<const int2*>(&rec[g0].si));
     if constexpr (NPASS > 1) {
       // a pass whose bra components all lack a coefficient (the lower components of a
@@ -324,10 +324,10 @@ __global__ void __launch_bounds__(128, GqOccupancy<LA, LB, LC, LD>::blocks) k_gq
         live = live || (stidx[ijg.x * MAXCOMP + ORD.ab[k] / NB] >= 0 && stidx[ijg.y * MAXCOMP + ORD.ab[k] % NB] >= 0);
       if (!live) continue;
     }
-    const int li = ch.y + lane;
-    const bool act = li < ch.z;
-    const int H = ql.bk_list[act ? li : ch.y];
-    const int h0 = ql.gr_start[H], hn = act ? ql.gr_n[H] : 0;
+    const int li = ch.first + lane;
+    const bool act = li < ch.end;
+    const int H = ql.bk_list[act ? li : ch.first];
+    const int h0 = ql.gr_start[H], hn = act ? min(ql.gr_n[H], ch.q1) : 0;
     const bool dens = ql.dtol > 0.0 || ql.mcut > 0.0;
     const int2 klh = __ldg(reinterpret_cast<const int2*>(&rec[h0].si));
     const double pmax = dens ? quartet_pmax(ql, ijg.x, ijg.y, klh.x, klh.y) : 0.0;
@@ -337,12 +337,12 @@ __global__ void __launch_bounds__(128, GqOccupancy<LA, LB, LC, LD>::blocks) k_gq
     double X[XN];
 #pragma unroll
     for (int i = 0; i < XN; ++i) X[i] = 0.0;
-    const double gmax = ql.gr_max[G];
+    const double gmax = pair_bound(rec, g0 + ch.p0);   // the largest of this piece (bounds descend)
     // Each lane walks its own ket group's pairs (outer loop, one gather of the ket
     // record per pair); the warp walks the bra group's pairs in step (inner loop:
     // every lane reads the same bra record, one L1 wavefront per load).  Both
     // lists are sorted by Schwarz bound, so the screens end the loops.
-    for (int qi = 0;; ++qi) {
+    for (int qi = ch.q0;; ++qi) {
       const bool lv = qi < hn;
       const int q = h0 + (lv ? qi : 0);
       const PairView kq = load_pair(rec, q);
@@ -368,7 +368,7 @@ __global__ void __launch_bounds__(128, GqOccupancy<LA, LB, LC, LD>::blocks) k_gq
 #pragma unroll
           for (int d = 0; d < ND; ++d) ccd[cc * ND + d] = wKL * sK[cc] * sL[d];
       }
-      for (int p = g0; p < g0 + gn; ++p) {
+      for (int p = g0 + ch.p0; p < g0 + ch.p1; ++p) {
         const PairView bp = load_pair(rec, p);
         const double sp = bp.bound;
         const bool pass = qok && sp * sq >= thr;

@@ -98,16 +98,16 @@ __global__ void __launch_bounds__(256) k_gq_wide(MolLaunch lq, OpTableDev tab, i
     if (lane == 0) tk = atomicAdd(lq.queue, 1);
     const int c = __shfl_sync(0xffffffffu, tk, 0) * lq.numprocs + lq.myid;
     if (c >= nchunks) break;
-    const int4 ch = lq.chunks[c];
-    const MolLaunch& ql = lq.insts ? lq.insts[ch.w] : lq;
+    const Chunk ch = lq.chunks[c];
+    const MolLaunch& ql = lq.insts ? lq.insts[ch.inst] : lq;
     const PairRec* __restrict__ rec = ql.rec;
     const double* __restrict__ scoef = ql.scoef;
     const double* __restrict__ boys = ql.boys;
     const double* __restrict__ D = ql.dt;
     const int nt = ql.nt;
-    const int G = ch.x;
-    const int g0 = ql.gr_start[G], gn = ql.gr_n[G];
-    const double gmax = ql.gr_max[G];
+    const int G = ch.G;
+    const int g0 = ql.gr_start[G];
+    const double gmax = pair_bound(rec, g0 + ch.p0);   // the largest of this piece (bounds descend)
     const int2 ij0 = __ldg(reinterpret_cast<const int2*>(&rec[g0].si));
     if (lane == 0) {
       bool ta, tb;
@@ -120,7 +120,7 @@ __global__ void __launch_bounds__(256) k_gq_wide(MolLaunch lq, OpTableDev tab, i
     const int nab = na * nb;
     const bool bra_top = meta[4] != 0 && tab.ops_p != nullptr;
     for (int t = lane; t < nab; t += 32) P[W::OAB + t] = dt_at(D, nt, tA[t / nb], tB[t % nb]);
-    for (int k = ch.y; k < ch.z; ++k) {
+    for (int k = ch.first; k < ch.end; ++k) {
       const int H = ql.bk_list[k];
       const int h0 = ql.gr_start[H], hn = ql.gr_n[H];
       const double hmax = ql.gr_max[H];
@@ -165,15 +165,15 @@ __global__ void __launch_bounds__(256) k_gq_wide(MolLaunch lq, OpTableDev tab, i
       for (int t = lane; t < nb * nc; t += 32) P[W::OBC + t] = dt_at(D, nt, tB[t / nc], tC[t % nc]);
       for (int t = lane; t < nb * nd; t += 32) P[W::OBD + t] = dt_at(D, nt, tB[t / nd], tD[t % nd]);
       bool any = false;   // warp-uniform
-      for (int p = g0; p < g0 + gn; ++p) {
+      for (int p = g0 + ch.p0; p < g0 + ch.p1; ++p) {
         const PairView bp = load_pair(rec, p);
         const double sp = bp.bound;
         if (sp * hmax < thr) break;
         const int I = bp.si, J = bp.sj;
         const double zb = bp.zeta;
-        const int qe = (G == H) ? p + 1 : h0 + hn;
+        const int qe = min((G == H) ? p + 1 : h0 + hn, h0 + min(hn, ch.q1));
         bool cab_ready = false;
-        for (int q = h0; q < qe; ++q) {
+        for (int q = h0 + ch.q0; q < qe; ++q) {
           const PairView kq = load_pair(rec, q);
           const double sq = kq.bound;
           if (sp * sq < thr) break;   // the reference's screen (warp-uniform)
