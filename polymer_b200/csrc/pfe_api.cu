@@ -220,6 +220,9 @@ static void reset_context(pfe_context* ctx) {
   ctx->d_gr_start = ctx->d_gr_n = ctx->d_bk_list = nullptr;
   ctx->d_gr_max = nullptr;
   ctx->d_prec = nullptr;
+  ctx->d_poff = ctx->d_ptgt = ctx->d_prown = ctx->d_pinv = ctx->d_pinv_row = nullptr;
+  ctx->d_prow = nullptr;
+  ctx->d_pd = ctx->d_pj = ctx->d_pk = nullptr;
   ctx->d_raw = nullptr;
   ctx->d_raw_steps = ctx->d_raw_cost = nullptr;
   ctx->d_raw_pair = nullptr;
@@ -354,6 +357,17 @@ static int setup_impl(pfe_context* ctx, const pfe_args* a, const HostShells& hs,
       blk[sh] = it->second;
     }
     ctx->nblk = (int)keys.size();
+    ctx->h_blk = blk;
+    ctx->h_blk_L.assign(ctx->nblk, 0);
+    ctx->h_blk_t.assign((size_t)ctx->nblk * MAXCOMP, -1);
+    for (const auto& kv : keys) {
+      ctx->h_blk_L[kv.second] = kv.first[0];
+      for (size_t c = 1; c < kv.first.size(); ++c) {
+        // a component's target: the contracted row, or the primitive itself when it carries a coefficient
+        const int v = kv.first[c];
+        ctx->h_blk_t[(size_t)kv.second * MAXCOMP + c - 1] = ctx->contracted ? v : tidx[v];
+      }
+    }
     if ((long long)ctx->nblk * ctx->nblk > (1LL << 30)) {
       set_error("too many shells for the block-pair index (more than 32768 distinct shells)");
       return PFE_EINVAL;

@@ -91,6 +91,10 @@ struct ClassLaunch {
   int wpb, per_warp;         // warps per block and doubles per warp (variant 1)
   size_t smem_big, smem_warp;
   float tuned_ms[4];         // autotuner timings per variant (0 = not run)
+  // straight-line variant: X of up to xcap chunks (a tile) at xbuf, and a flag per chunk
+  double* xbuf;
+  unsigned char* xlive;
+  int xcap;
   double* xg;                // block variant: per-block X scratch in global memory, or null
   int nslots_p, nslots_p2;   // slots of the pure-bra and bra-and-ket tables (0: none)
   // variant 3 (warp per primitive quartet, kept outputs only): per-warp shared
@@ -108,6 +112,19 @@ struct ClassLaunch {
 
 // The opaque handle of the C ABI.
 struct pfe_context {
+  // block panels of the digestion (molecules; pfe_mol.cu): the kept components of every
+  // contracted block are consecutive panel rows, and the matrices of a block pair are
+  // contiguous: element (p, q) at row_base[p] + q * row_n[p], where a block of n rows
+  // from row p0 has row_base[p] = p0 * np + (p - p0) and row_n[p] = n
+  std::vector<int> h_blk, h_blk_L, h_blk_t;   // shell -> block; block -> L, -> target per component (MAXCOMP)
+  int np = 0;
+  int* d_poff = nullptr;        // shell -> first panel row of its block
+  int* d_ptgt = nullptr;        // panel row -> target (-1: none)
+  long long* d_prow = nullptr;  // row_base
+  int* d_prown = nullptr;       // row_n
+  int* d_pinv = nullptr;        // target -> its panel rows: d_pinv[t] .. d_pinv[t + 1] of d_pinv_row
+  int* d_pinv_row = nullptr;
+  double *d_pd = nullptr, *d_pj = nullptr, *d_pk = nullptr;
   int device = 0;
   int num_sms = 148;
   cudaStream_t stream = nullptr;

@@ -469,6 +469,70 @@ __global__ void k_block_dmax(const double* __restrict__ D, int nt, const int* __
   if (v > 0.0) atomicMax(bmax + (size_t)b1 * nblk + b2, (unsigned long long)__double_as_longlong(v));
 }
 
+// ------------------------------------------------------------------ block panels
+
+// The panel tables of a molecule as the kernels around a build read them.
+struct PanelView {
+  const int* tgt;
+  const long long* row;
+  const int* rown;
+  const int* inv;
+  const int* inv_row;
+  int np;
+};
+
+// The density into the panels and J', K' to zero, one element per thread.
+__device__ __forceinline__ void panel_in(const PanelView& v, const double* __restrict__ dt, int nt, long long t,
+                                         double* __restrict__ pd, double* __restrict__ pj, double* __restrict__ pk) {
+  const int p = (int)(t % v.np), q = (int)(t / v.np);
+  const int i = v.tgt[p], j = v.tgt[q];
+  const long long o = v.row[p] + (long long)q * v.rown[p];
+  pd[o] = (i >= 0 && j >= 0) ? dt[i + (size_t)nt * j] : 0.0;
+  pj[o] = 0.0;
+  pk[o] = 0.0;
+}
+
+// M(i, j) + M(j, i) of a panel matrix summed over the panel rows of targets i and j
+// (several where shells of different blocks share a target).
+__device__ __forceinline__ double panel_sym(const PanelView& v, const double* __restrict__ m, int i, int j) {
+  double a = 0.0;
+  for (int x = v.inv[i]; x < v.inv[i + 1]; ++x)
+    for (int y = v.inv[j]; y < v.inv[j + 1]; ++y) {
+      const int p = v.inv_row[x], q = v.inv_row[y];
+      a += m[v.row[p] + (long long)q * v.rown[p]] + m[v.row[q] + (long long)p * v.rown[q]];
+    }
+  return a;
+}
+
+__global__ void k_panel_in(PanelView v, const double* __restrict__ dt, int nt, double* __restrict__ pd,
+                           double* __restrict__ pj, double* __restrict__ pk) {
+  const long long t = blockIdx.x * (long long)blockDim.x + threadIdx.x;
+  if (t < (long long)v.np * v.np) panel_in(v, dt, nt, t, pd, pj, pk);
+}
+
+// C_C = J' + J'^T and X_C = K' + K'^T from the target-space accumulators and the panels.
+__global__ void k_panel_out(PanelView v, const double* __restrict__ jt, const double* __restrict__ kt,
+                            const double* __restrict__ pj, const double* __restrict__ pk, int nt,
+                            double* __restrict__ cc, double* __restrict__ xc) {
+  const long long t = blockIdx.x * (long long)blockDim.x + threadIdx.x;
+  if (t >= (long long)nt * nt) return;
+  const int i = (int)(t % nt), j = (int)(t / nt);
+  const long long tt = i * (long long)nt + j;
+  cc[t] = jt[t] + jt[tt] + panel_sym(v, pj, i, j);
+  xc[t] = kt[t] + kt[tt] + panel_sym(v, pk, i, j);
+}
+
+// Primitive targets: half of the panels' symmetric sum into J' and K' (the
+// contraction symmetrises them again).
+__global__ void k_panel_fold(PanelView v, double* __restrict__ jt, double* __restrict__ kt,
+                             const double* __restrict__ pj, const double* __restrict__ pk, int nt) {
+  const long long t = blockIdx.x * (long long)blockDim.x + threadIdx.x;
+  if (t >= (long long)nt * nt) return;
+  const int i = (int)(t % nt), j = (int)(t / nt);
+  jt[t] += 0.5 * panel_sym(v, pj, i, j);
+  kt[t] += 0.5 * panel_sym(v, pk, i, j);
+}
+
 // ------------------------------------------------------------------ interpreted classes
 
 // Digestion of a contracted X(abcd) into the targets of one group quartet,
@@ -906,6 +970,92 @@ static unsigned int longest_piece(double steps) {
   return (unsigned int)std::min(4.0e9, std::max((double)kLeastSteps, share));
 }
 
+static PanelView panel_view(const pfe_context* c) {
+  return PanelView{c->d_ptgt, c->d_prow, c->d_prown, c->d_pinv, c->d_pinv_row, c->np};
+}
+
+// The block panels of a molecule whose shells of top L keep their lower components
+// where bit L of `bits` says so (a batch: where any of its molecules needs them).
+static int build_panels(pfe_context* ctx, int bits) {
+  const int nblk = ctx->nblk;
+  std::vector<int> first(nblk + 1, 0);
+  for (int b = 0; b < nblk; ++b) first[b + 1] = first[b] + kept_n(ctx->h_blk_L[b], bits);
+  const int np = ctx->np = first[nblk];
+  std::vector<int> tgt(np, -1), rown(np), poff(ctx->npshell), inv(ctx->nt + 1, 0), inv_row;
+  std::vector<long long> row(np);
+  for (int b = 0; b < nblk; ++b) {
+    const int L = ctx->h_blk_L[b], f = kept_first(L, bits);
+    for (int c = 0; c < ncum(L); ++c)
+      if (comp_rank(L, c) >= f) tgt[first[b] + comp_rank(L, c) - f] = ctx->h_blk_t[(size_t)b * MAXCOMP + c];
+    for (int p = first[b]; p < first[b + 1]; ++p) {
+      row[p] = (long long)first[b] * np + (p - first[b]);
+      rown[p] = first[b + 1] - first[b];
+    }
+  }
+  for (int s = 0; s < ctx->npshell; ++s) poff[s] = first[ctx->h_blk[s]];
+  for (int p = 0; p < np; ++p)
+    if (tgt[p] >= 0) ++inv[tgt[p] + 1];
+  for (int t = 0; t < ctx->nt; ++t) inv[t + 1] += inv[t];
+  inv_row.resize(inv[ctx->nt] + 1);
+  {
+    std::vector<int> at(inv.begin(), inv.end() - 1);
+    for (int p = 0; p < np; ++p)
+      if (tgt[p] >= 0) inv_row[at[tgt[p]]++] = p;
+  }
+  auto put = [&](auto** d, const auto& v) -> cudaError_t {
+    cudaError_t e = ctx->alloc((void**)d, sizeof(v[0]) * v.size());
+    return e != cudaSuccess ? e : cudaMemcpy(*d, v.data(), sizeof(v[0]) * v.size(), cudaMemcpyHostToDevice);
+  };
+  PFE_CUDA(put(&ctx->d_poff, poff));
+  PFE_CUDA(put(&ctx->d_ptgt, tgt));
+  PFE_CUDA(put(&ctx->d_prow, row));
+  PFE_CUDA(put(&ctx->d_prown, rown));
+  PFE_CUDA(put(&ctx->d_pinv, inv));
+  PFE_CUDA(put(&ctx->d_pinv_row, inv_row));
+  const size_t bytes = sizeof(double) * (size_t)np * np;
+  PFE_CUDA(ctx->alloc((void**)&ctx->d_pd, bytes));
+  PFE_CUDA(ctx->alloc((void**)&ctx->d_pj, bytes));
+  PFE_CUDA(ctx->alloc((void**)&ctx->d_pk, bytes));
+  return PFE_OK;
+}
+
+// Kept integrals of a class's group quartet: what one lane stores.
+static int kept_integrals(int cb, int ck, int bits) {
+  return kept_n(kCL[cb][0], bits) * kept_n(kCL[cb][1], bits) * kept_n(kCL[ck][0], bits) * kept_n(kCL[ck][1], bits);
+}
+
+// Memory for the stored integrals of the straight-line classes: one buffer that the
+// classes use one after another, of the largest class's size up to kTileBytes; larger
+// classes run in tiles of that size.  Measured on B200: a tile's passes last long
+// enough (milliseconds) that their tails do not show, and the buffer's traffic
+// (written and read once, at HBM rate) is a tenth of what the digestion inside every
+// pass cost.
+template <typename Owner>
+static int alloc_integrals(Owner* own, ClassLaunch* launches, int nlaunch, int bits) {
+  constexpr size_t kTileBytes = (size_t)1 << 30;
+  size_t most = 0, flags = 0;
+  for (int i = 0; i < nlaunch; ++i) {
+    ClassLaunch& cl = launches[i];
+    if (!cl.has_straight || cl.cb == 0) continue;
+    const size_t per = sizeof(double) * 32 * (size_t)kept_integrals(cl.cb, cl.ck, bits);
+    cl.xcap = (int)std::max<size_t>(1, std::min<size_t>(kTileBytes / per, (size_t)cl.nchunks_host));
+    most = std::max(most, per * cl.xcap);
+    flags = std::max(flags, (size_t)cl.xcap);
+  }
+  double* x = nullptr;
+  unsigned char* f = nullptr;
+  if (most > 0) {
+    PFE_CUDA(own->alloc((void**)&x, most));
+    PFE_CUDA(own->alloc((void**)&f, flags));
+    PFE_CUDA(cudaMemset(f, 0, flags));
+  }
+  for (int i = 0; i < nlaunch; ++i) {
+    launches[i].xbuf = x;
+    launches[i].xlive = f;
+  }
+  return PFE_OK;
+}
+
 template <typename Owner>
 static int finish_chunks(Owner* own, pfe_context* const* inst, int ninst, ClassLaunch* launches, int nlaunch,
                          cudaStream_t s) {
@@ -1281,6 +1431,8 @@ int molecular_setup(pfe_context* ctx, const pfe_args* a) {
   if (!ctx->in_batch) {
     pfe_context* const self = ctx;
     if ((rc = finish_chunks(ctx, &self, 1, ctx->launches, ctx->nlaunch, s)) != PFE_OK) return rc;
+    if ((rc = build_panels(ctx, lower_kept_bits(ctx))) != PFE_OK) return rc;
+    if ((rc = alloc_integrals(ctx, ctx->launches, ctx->nlaunch, lower_kept_bits(ctx))) != PFE_OK) return rc;
     free_raw(ctx);
   }
   ctx->free_now(d_count);
@@ -1322,6 +1474,12 @@ static MolLaunch make_launch(pfe_context* ctx, const double* d_dt) {
   ql.nt = ctx->nt;
   ql.myid = ctx->myid;
   ql.numprocs = ctx->numprocs;
+  ql.pd = ctx->d_pd;
+  ql.pj = ctx->d_pj;
+  ql.pk = ctx->d_pk;
+  ql.poff = ctx->d_poff;
+  ql.ptgt = ctx->d_ptgt;
+  ql.np = ctx->np;
   return ql;
 }
 
@@ -1333,8 +1491,19 @@ static void launch_class(pfe_context* ctx, const ClassLaunch& cl, MolLaunch ql, 
   cudaMemsetAsync(cl.queue, 0, sizeof(int) * 64, s);   // every launch (pass) of the class starts its queue at 0
   const int work = (cl.nchunks_host + ctx->numprocs - 1) / ctx->numprocs;
   if ((variant == 0 && cl.has_straight) || !cl.has_table) {
-    const int grid = std::min((work + 3) / 4, ctx->num_sms * cl.gmul);
-    straight_launcher(cl.cb, cl.ck, mixed, ql.insts != nullptr)(ql, std::max(grid, 1), s);
+    // (00|00) digests in its kernel; the other classes store X tile by tile
+    const bool stored = cl.cb > 0;
+    const int cap = stored ? cl.xcap : std::max(work, 1);
+    for (int t0 = 0; t0 < work; t0 += cap) {
+      if (t0 > 0) cudaMemsetAsync(cl.queue, 0, sizeof(int) * 64, s);
+      ql.t0 = t0;
+      ql.tn = std::min(cap, work - t0);
+      ql.xbuf = cl.xbuf;
+      ql.xlive = cl.xlive;
+      const int grid = std::min((ql.tn + 3) / 4, ctx->num_sms * cl.gmul);
+      straight_launcher(cl.cb, cl.ck, mixed, ql.insts != nullptr)(ql, std::max(grid, 1), s);
+      if (stored) launch_digest(cl.cb, cl.ck, ql, ctx->num_sms, s);
+    }
     return;
   }
   OpTableDev t{cl.ops,   cl.levels,   cl.out,     cl.nlevels,   cl.nout,   cl.nslots,     cl.ops_p,
@@ -1369,6 +1538,26 @@ static const double* target_density(pfe_context* ctx, const double* d_pp, cudaSt
   k_check_density<<<(unsigned)((np2 + 255) / 256), 256, 0, s>>>(d_pp, ctx->npgs, ctx->d_tidx, ctx->d_tcoef,
                                                                   ctx->d_pt, ctx->nt, ctx->d_flag);
   return ctx->d_pt;
+}
+
+static void launch_panel_in(pfe_context* ctx, const double* d_dt, cudaStream_t s) {
+  const long long n2 = (long long)ctx->np * ctx->np;
+  k_panel_in<<<(unsigned)((n2 + 255) / 256), 256, 0, s>>>(panel_view(ctx), d_dt, ctx->nt, ctx->d_pd, ctx->d_pj,
+                                                          ctx->d_pk);
+}
+
+// The outputs from the accumulators: contracted targets symmetrised straight into
+// C_C and X_C, primitive targets through the contraction.
+static int finish_build(pfe_context* ctx, double* d_cc, double* d_xc, cudaStream_t s) {
+  const unsigned grid = (unsigned)(((long long)ctx->nt * ctx->nt + 255) / 256);
+  if (ctx->contracted) {
+    k_panel_out<<<grid, 256, 0, s>>>(panel_view(ctx), ctx->d_jp, ctx->d_kp, ctx->d_pj, ctx->d_pk, ctx->nt, d_cc, d_xc);
+    PFE_CUDA(cudaGetLastError());
+    return PFE_OK;
+  }
+  k_panel_fold<<<grid, 256, 0, s>>>(panel_view(ctx), ctx->d_jp, ctx->d_kp, ctx->d_pj, ctx->d_pk, ctx->nt);
+  PFE_CUDA(cudaGetLastError());
+  return contract_outputs(ctx, ctx->d_jp, ctx->d_kp, d_cc, d_xc, /*symmetrize=*/true, 1, s);
 }
 
 static bool variant_ok(const ClassLaunch& cl, int v) {
@@ -1419,7 +1608,9 @@ static int tune_class(pfe_context* ctx, ClassLaunch& cl, const MolLaunch& ql, cu
 }
 
 int autotune(pfe_context* ctx, const double* d_pp, cudaStream_t s) {
-  const MolLaunch ql = make_launch(ctx, target_density(ctx, d_pp, s));
+  const double* d_dt = target_density(ctx, d_pp, s);
+  const MolLaunch ql = make_launch(ctx, d_dt);
+  launch_panel_in(ctx, d_dt, s);
   PFE_CUDA(cudaGetLastError());
   cudaEvent_t e0, e1;
   PFE_CUDA(cudaEventCreate(&e0));
@@ -1444,6 +1635,8 @@ static int prepare_build(pfe_context* ctx, const double* d_dt, cudaStream_t s, b
   PFE_CUDA(cudaMemsetAsync(ctx->d_jp, 0, target_bytes(ctx), s));
   PFE_CUDA(cudaMemsetAsync(ctx->d_kp, 0, target_bytes(ctx), s));
   PFE_CUDA(cudaMemsetAsync(ctx->d_n32, 0, sizeof(unsigned long long), s));
+  launch_panel_in(ctx, d_dt, s);
+  PFE_CUDA(cudaGetLastError());
   if (always_bmax || ctx->dtol > 0.0 || ctx->mcut > 0.0) {
     const long long nt2 = (long long)ctx->nt * ctx->nt;
     PFE_CUDA(cudaMemsetAsync(ctx->d_bmax, 0, sizeof(double) * (size_t)ctx->nblk * ctx->nblk, s));
@@ -1519,13 +1712,7 @@ static int run_build(pfe_context* ctx, const double* d_dt, double* d_cc, double*
       for (int v = 0; v < 4; ++v) ctx->ev_tuned[i][v] = cl.tuned_ms[v];
     }
   }
-  if (ctx->contracted) {
-    launch_symmetrize(ctx->d_jp, d_cc, ctx->ncgs, 1, s);
-    launch_symmetrize(ctx->d_kp, d_xc, ctx->ncgs, 1, s);
-    PFE_CUDA(cudaGetLastError());
-    return PFE_OK;
-  }
-  return contract_outputs(ctx, ctx->d_jp, ctx->d_kp, d_cc, d_xc, /*symmetrize=*/true, 1, s);
+  return finish_build(ctx, d_cc, d_xc, s);
 }
 
 int molecular_fock(pfe_context* ctx, const double* d_pp, double* d_cc, double* d_xc, cudaStream_t s) {
@@ -1633,15 +1820,23 @@ int batch_setup(pfe_batch* b) {
     const int rc = finish_chunks(b, b->inst.data(), (int)b->inst.size(), b->launches, b->nlaunch, st);
     if (rc != PFE_OK) return rc;
   }
-  for (pfe_context* c : b->inst) {   // the joined lists replace them
-    free_raw(c);
+  int bits = 0;
+  for (pfe_context* c : b->inst) bits |= lower_kept_bits(c);
+  for (pfe_context* c : b->inst) {
+    free_raw(c);   // the joined lists replace them
+    const int rc = build_panels(c, bits);
+    if (rc != PFE_OK) return rc;
   }
-  PFE_CUDA(b->alloc(&b->d_insts, sizeof(MolLaunch) * b->inst.size()));
+  {
+    const int rc = alloc_integrals(b, b->launches, b->nlaunch, bits);
+    if (rc != PFE_OK) return rc;
+  }
+  PFE_CUDA(b->alloc(&b->d_insts, (sizeof(MolLaunch) + sizeof(PanelView)) * b->inst.size()));
   PFE_CUDA(b->alloc((void**)&b->d_off, sizeof(long long) * b->off.size()));
   PFE_CUDA(cudaMemcpy(b->d_off, b->off.data(), sizeof(long long) * b->off.size(), cudaMemcpyHostToDevice));
   b->all_contracted = true;
   for (pfe_context* c : b->inst) b->all_contracted = b->all_contracted && c->contracted;
-  PFE_CUDA(cudaMallocHost(&b->h_insts, sizeof(MolLaunch) * b->inst.size()));
+  PFE_CUDA(cudaMallocHost(&b->h_insts, (sizeof(MolLaunch) + sizeof(PanelView)) * b->inst.size()));
   PFE_CUDA(cudaEventCreateWithFlags(&b->ev_insts, cudaEventDisableTiming));
   b->insts_for = nullptr;
   b->mixed = false;
@@ -1657,9 +1852,11 @@ int batch_refresh(pfe_batch* b, const double* d_pc) {
   if (b->ev_pending) PFE_CUDA(cudaEventSynchronize(b->ev_insts));
   b->ev_pending = false;
   MolLaunch* h = static_cast<MolLaunch*>(b->h_insts);
+  PanelView* pv = reinterpret_cast<PanelView*>(h + b->inst.size());   // after the records
   for (size_t k = 0; k < b->inst.size(); ++k) {
     pfe_context* c = b->inst[k];
     h[k] = make_launch(c, c->contracted ? d_pc + b->off[k] : c->d_pt);
+    pv[k] = panel_view(c);
     b->mixed = b->mixed || c->mcut > 0.0;
   }
   b->insts_for = d_pc;
@@ -1689,10 +1886,13 @@ static int batch_decontract(pfe_batch* b, const double* d_pc, cudaStream_t s) {
 // The per-instance work around a batched build as three launches over every
 // instance (blockIdx.y = instance, the threads of its blocks stride over its
 // matrices) instead of seven small ones per instance: zero J'/K', the block
-// maxima and the FP32 counter; the block maxima of |P_T|; after the class
+// maxima and the FP32 counter and fill the density panels; the block maxima of |P_T|; after the class
 // kernels, C_C = J' + J'^T and X_C = K' + K'^T at the packed offsets.
-__global__ void k_batch_zero(const MolLaunch* __restrict__ insts) {
+__global__ void k_batch_zero(const MolLaunch* __restrict__ insts, const PanelView* __restrict__ pv) {
   const MolLaunch& q = insts[blockIdx.y];
+  const long long np2 = (long long)q.np * q.np;
+  for (long long t = blockIdx.x * (long long)blockDim.x + threadIdx.x; t < np2; t += (long long)gridDim.x * blockDim.x)
+    panel_in(pv[blockIdx.y], q.dt, q.nt, t, const_cast<double*>(q.pd), q.pj, q.pk);
   const long long nt2 = (long long)q.nt * q.nt, nb2 = (long long)q.nblk * q.nblk;
   for (long long t = blockIdx.x * (long long)blockDim.x + threadIdx.x; t < nt2; t += (long long)gridDim.x * blockDim.x) {
     q.jt[t] = 0.0;
@@ -1717,7 +1917,8 @@ __global__ void k_batch_dmax(const MolLaunch* __restrict__ insts) {
   }
 }
 
-__global__ void k_batch_symmetrize(const MolLaunch* __restrict__ insts, const long long* __restrict__ off,
+__global__ void k_batch_symmetrize(const MolLaunch* __restrict__ insts, const PanelView* __restrict__ pv,
+                                   const long long* __restrict__ off,
                                    double* __restrict__ cc, double* __restrict__ xc) {
   const MolLaunch& q = insts[blockIdx.y];
   const int n = q.nt;
@@ -1727,8 +1928,8 @@ __global__ void k_batch_symmetrize(const MolLaunch* __restrict__ insts, const lo
   for (long long t = blockIdx.x * (long long)blockDim.x + threadIdx.x; t < nt2; t += (long long)gridDim.x * blockDim.x) {
     const int i = (int)(t % n), j = (int)(t / n);
     const long long tt = i * (long long)n + j;   // (j, i)
-    c[t] = q.jt[t] + q.jt[tt];
-    x[t] = q.kt[t] + q.kt[tt];
+    c[t] = q.jt[t] + q.jt[tt] + panel_sym(pv[blockIdx.y], q.pj, i, j);
+    x[t] = q.kt[t] + q.kt[tt] + panel_sym(pv[blockIdx.y], q.pk, i, j);
   }
 }
 
@@ -1752,7 +1953,8 @@ int batch_fock_pc(pfe_batch* b, const double* d_pc, double* d_cc, double* d_xc, 
   }
   // the records travel with every build: a captured graph uploads what the host
   // last wrote into the pinned copy
-  PFE_CUDA(cudaMemcpyAsync(b->d_insts, b->h_insts, sizeof(MolLaunch) * n, cudaMemcpyHostToDevice, s));
+  PFE_CUDA(cudaMemcpyAsync(b->d_insts, b->h_insts, (sizeof(MolLaunch) + sizeof(PanelView)) * n, cudaMemcpyHostToDevice,
+                           s));
   if (!capturing) {
     PFE_CUDA(cudaEventRecord(b->ev_insts, s));
     b->ev_pending = true;
@@ -1761,7 +1963,8 @@ int batch_fock_pc(pfe_batch* b, const double* d_pc, double* d_cc, double* d_xc, 
   // change between graph replays), one launch each over the whole batch
   const MolLaunch* di = static_cast<const MolLaunch*>(b->d_insts);
   const dim3 gb(8, (unsigned)n);
-  k_batch_zero<<<gb, 256, 0, s>>>(di);
+  const PanelView* dv = reinterpret_cast<const PanelView*>(di + n);
+  k_batch_zero<<<gb, 256, 0, s>>>(di, dv);
   k_batch_dmax<<<gb, 256, 0, s>>>(di);
   PFE_CUDA(cudaGetLastError());
   pfe_context* c0 = b->inst[0];
@@ -1774,17 +1977,11 @@ int batch_fock_pc(pfe_batch* b, const double* d_pc, double* d_cc, double* d_xc, 
     PFE_CUDA(cudaGetLastError());
   }
   if (b->all_contracted) {
-    k_batch_symmetrize<<<gb, 256, 0, s>>>(di, b->d_off, d_cc, d_xc);
+    k_batch_symmetrize<<<gb, 256, 0, s>>>(di, dv, b->d_off, d_cc, d_xc);
   } else {
     for (size_t k = 0; k < n; ++k) {
-      pfe_context* c = b->inst[k];
-      if (c->contracted) {
-        launch_symmetrize(c->d_jp, d_cc + b->off[k], c->ncgs, 1, s);
-        launch_symmetrize(c->d_kp, d_xc + b->off[k], c->ncgs, 1, s);
-      } else {
-        int rc = contract_outputs(c, c->d_jp, c->d_kp, d_cc + b->off[k], d_xc + b->off[k], true, 1, s);
-        if (rc != PFE_OK) return rc;
-      }
+      const int rc = finish_build(b->inst[k], d_cc + b->off[k], d_xc + b->off[k], s);
+      if (rc != PFE_OK) return rc;
     }
   }
   PFE_CUDA(cudaGetLastError());
@@ -1797,7 +1994,8 @@ int batch_autotune(pfe_batch* b, const double* d_pc, cudaStream_t s) {
   int rc = batch_decontract(b, d_pc, s);
   if (rc != PFE_OK) return rc;
   if (b->insts_for != d_pc && (rc = batch_refresh(b, d_pc)) != PFE_OK) return rc;
-  PFE_CUDA(cudaMemcpyAsync(b->d_insts, b->h_insts, sizeof(MolLaunch) * b->inst.size(), cudaMemcpyHostToDevice, s));
+  PFE_CUDA(cudaMemcpyAsync(b->d_insts, b->h_insts, (sizeof(MolLaunch) + sizeof(PanelView)) * b->inst.size(),
+                           cudaMemcpyHostToDevice, s));
   PFE_CUDA(cudaEventRecord(b->ev_insts, s));
   b->ev_pending = true;
   for (size_t k = 0; k < b->inst.size(); ++k) {

@@ -1,0 +1,221 @@
+// Digestion of the straight-line molecular classes: X(abcd) of every group quartet,
+// stored by the register passes (k_gq) as one 256-byte row per integral and chunk,
+// contracted with the density into J' and K' once.
+//
+// What bounds it: the L1's wavefronts.  A lane's targets lie at addresses of its own
+// (its ket's shells), so a scattered load or atomic of a warp costs 32 wavefronts;
+// digested inside every register pass that was 55 % of the C20H42 build ((21|11): 56
+// gathers and 56 atomics per lane in each of 9 passes).  Here
+//   * the density and the accumulators are block panels: the matrix of a shell pair is
+//     contiguous, so the warp copies the blocks of its 32 quartets cooperatively, lanes
+//     along the elements (one or two lines per block instead of one per element), into
+//     shared memory rows of 33 doubles, from where each lane reads its own column;
+//   * K' and J'(cd) leave the same way: columns to shared memory, then atomics with the
+//     lanes along the elements of a block;
+//   * the bra is the warp's, so J'(ab) is summed over the lanes first.
+// The multiply-adds (six per integral) run per lane from registers.
+// Measured, C20H42 6-31G** (B200): see the figures at launch_digest.
+
+#include <algorithm>
+
+#include "pfe_common.cuh"
+#include "pfe_context.cuh"
+#include "pfe_mol_kernels.cuh"
+
+namespace pfe {
+
+namespace {
+
+// Kept components of the class's shells: KEPT is the lower_kept bits of L = 1 and 2.
+template <int LA, int LB, int LC, int LD, int KEPT>
+struct DigestShape {
+  static constexpr int NA = kept_n(LA, KEPT), NB = kept_n(LB, KEPT), NC = kept_n(LC, KEPT), ND = kept_n(LD, KEPT);
+  static constexpr int R_AC = 0, R_AD = NA * NC, R_BC = R_AD + NA * ND, R_BD = R_BC + NB * NC, R_CD = R_BD + NB * ND;
+  static constexpr int ROWS = R_CD + NC * ND;
+  static constexpr int PER_WARP = ROWS * 33;   // doubles
+  static constexpr int WARPS = PER_WARP * 8 * 4 <= 100 * 1024 ? 4 : (PER_WARP * 8 * 2 <= 100 * 1024 ? 2 : 1);
+};
+
+// The warp's copy of 32 blocks of M doubles (block of lane l at m + shfl(off, l)) into
+// rows [0, M) of s, lane l's block in column l.
+template <int M>
+__device__ __forceinline__ void load_blocks(const double* __restrict__ m, long long off, double* __restrict__ s,
+                                            int lane) {
+  const int lo = (int)off, hi = (int)(off >> 32);
+#pragma unroll
+  for (int i = 0; i < M; ++i) {
+    const int f = i * 32 + lane, l = f / M, e = f - l * M;
+    const long long o = ((long long)__shfl_sync(0xffffffffu, hi, l) << 32) |
+                        (unsigned int)__shfl_sync(0xffffffffu, lo, l);
+    s[e * 33 + l] = __ldg(m + o + e);
+  }
+}
+
+// The reverse with atomics, for the first `cnt` lanes' blocks, scaled by w.
+template <int M>
+__device__ __forceinline__ void add_blocks(double* __restrict__ m, long long off, const double* __restrict__ s, int cnt,
+                                           double w, int lane) {
+  const int lo = (int)off, hi = (int)(off >> 32);
+#pragma unroll
+  for (int i = 0; i < M; ++i) {
+    const int f = i * 32 + lane, l = f / M, e = f - l * M;
+    const long long o = ((long long)__shfl_sync(0xffffffffu, hi, l) << 32) |
+                        (unsigned int)__shfl_sync(0xffffffffu, lo, l);
+    const double v = s[e * 33 + l];
+    if (l < cnt && v != 0.0) atomicAdd(m + o + e, w * v);
+  }
+}
+
+template <int LA, int LB, int LC, int LD, int KEPT>
+__global__ void __launch_bounds__(32 * DigestShape<LA, LB, LC, LD, KEPT>::WARPS) k_digest(MolLaunch lq) {
+  using S = DigestShape<LA, LB, LC, LD, KEPT>;
+  constexpr int NA = S::NA, NB = S::NB, NC = S::NC, ND = S::ND, NCD = NC * ND;
+  extern __shared__ double smem[];
+  const int lane = threadIdx.x & 31;
+  double* __restrict__ sm = smem + (size_t)(threadIdx.x >> 5) * S::PER_WARP;
+  double* __restrict__ col = sm + lane;   // this lane's column
+  const int nchunks = *lq.nchunks;
+  const int step = gridDim.x * S::WARPS;
+  for (int t = blockIdx.x * S::WARPS + (threadIdx.x >> 5); t < lq.tn; t += step) {
+    const int c = (lq.t0 + t) * lq.numprocs + lq.myid;
+    if (c >= nchunks) break;
+    if (!lq.xlive[t]) continue;
+    __syncwarp();                      // every lane has read the flag
+    if (lane == 0) lq.xlive[t] = 0;    // clean for the next tile or build
+    const Chunk ch = lq.chunks[c];
+    const PairRec* __restrict__ rec = lq.rec;
+    const int *bk_list = lq.bk_list, *gr_start = lq.gr_start, *poff = lq.poff, *ptgt = lq.ptgt;
+    const double* __restrict__ pd = lq.pd;
+    double *pj = lq.pj, *pk = lq.pk;
+    int np = lq.np;
+    if (lq.insts) {
+      const MolLaunch* q = lq.insts + ch.inst;
+      rec = q->rec; bk_list = q->bk_list; gr_start = q->gr_start; poff = q->poff; ptgt = q->ptgt;
+      pd = q->pd; pj = q->pj; pk = q->pk; np = q->np;
+    }
+    const int cnt = ch.end - ch.first;
+    const int H = bk_list[ch.first + (lane < cnt ? lane : 0)];
+    const int2 ij = __ldg(reinterpret_cast<const int2*>(&rec[gr_start[ch.G]].si));
+    const int2 kl = __ldg(reinterpret_cast<const int2*>(&rec[gr_start[H]].si));
+    const int pA = poff[ij.x], pB = poff[ij.y], pC = poff[kl.x], pD = poff[kl.y];
+    const long long oAB = (long long)pA * np + (long long)pB * NA;
+    const long long oAC = (long long)pA * np + (long long)pC * NA, oAD = (long long)pA * np + (long long)pD * NA;
+    const long long oBC = (long long)pB * np + (long long)pC * NB, oBD = (long long)pB * np + (long long)pD * NB;
+    const long long oCD = (long long)pC * np + (long long)pD * NC;
+    load_blocks<NA * NC>(pd, oAC, sm + S::R_AC * 33, lane);
+    load_blocks<NA * ND>(pd, oAD, sm + S::R_AD * 33, lane);
+    load_blocks<NB * NC>(pd, oBC, sm + S::R_BC * 33, lane);
+    load_blocks<NB * ND>(pd, oBD, sm + S::R_BD * 33, lane);
+    load_blocks<NC * ND>(pd, oCD, sm + S::R_CD * 33, lane);
+    __syncwarp();
+    const double* __restrict__ xb = lq.xbuf + (size_t)t * ((size_t)NA * NB * NCD * 32) + lane;
+    double kbc[NB * NC], kbd[NB * ND], jcd[NCD];
+#pragma unroll
+    for (int i = 0; i < NB * NC; ++i) kbc[i] = 0.0;
+#pragma unroll
+    for (int i = 0; i < NB * ND; ++i) kbd[i] = 0.0;
+#pragma unroll
+    for (int i = 0; i < NCD; ++i) jcd[i] = 0.0;
+#pragma unroll 1
+    for (int a = 0; a < NA; ++a) {
+      double dac[NC], dad[ND], kac[NC], kad[ND];
+#pragma unroll
+      for (int x = 0; x < NC; ++x) { dac[x] = col[(S::R_AC + x * NA + a) * 33]; kac[x] = 0.0; }
+#pragma unroll
+      for (int x = 0; x < ND; ++x) { dad[x] = col[(S::R_AD + x * NA + a) * 33]; kad[x] = 0.0; }
+      // components without a target have no stored integrals (warp-uniform)
+      if (ptgt[pA + a] >= 0) {
+#pragma unroll
+        for (int b = 0; b < NB; ++b) {
+          if (ptgt[pB + b] < 0) continue;
+          const double pab = __ldg(pd + oAB + b * NA + a);
+          double x[NCD];
+#pragma unroll
+          for (int cd = 0; cd < NCD; ++cd) x[cd] = __ldcs(xb + ((a * NB + b) * NCD + cd) * 32);
+          double jab = 0.0;
+#pragma unroll
+          for (int cc = 0; cc < NC; ++cc) {
+            const double dbc = col[(S::R_BC + cc * NB + b) * 33];
+#pragma unroll
+            for (int d = 0; d < ND; ++d) {
+              const double v = x[cc * ND + d];
+              jab = fma(col[(S::R_CD + d * NC + cc) * 33], v, jab);
+              jcd[cc * ND + d] = fma(pab, v, jcd[cc * ND + d]);
+              kad[d] = fma(dbc, v, kad[d]);
+              kac[cc] = fma(col[(S::R_BD + d * NB + b) * 33], v, kac[cc]);
+              kbd[b * ND + d] = fma(dac[cc], v, kbd[b * ND + d]);
+              kbc[b * NC + cc] = fma(dad[d], v, kbc[b * NC + cc]);
+            }
+          }
+          jab = warp_sum(jab);
+          if (lane == 0 && jab != 0.0) atomicAdd(pj + oAB + b * NA + a, 0.25 * jab);
+        }
+      }
+#pragma unroll
+      for (int x = 0; x < NC; ++x) col[(S::R_AC + x * NA + a) * 33] = kac[x];
+#pragma unroll
+      for (int x = 0; x < ND; ++x) col[(S::R_AD + x * NA + a) * 33] = kad[x];
+    }
+#pragma unroll
+    for (int b = 0; b < NB; ++b) {
+#pragma unroll
+      for (int x = 0; x < NC; ++x) col[(S::R_BC + x * NB + b) * 33] = kbc[b * NC + x];
+#pragma unroll
+      for (int x = 0; x < ND; ++x) col[(S::R_BD + x * NB + b) * 33] = kbd[b * ND + x];
+    }
+#pragma unroll
+    for (int cc = 0; cc < NC; ++cc)
+#pragma unroll
+      for (int d = 0; d < ND; ++d) col[(S::R_CD + d * NC + cc) * 33] = jcd[cc * ND + d];
+    __syncwarp();
+    add_blocks<NA * NC>(pk, oAC, sm + S::R_AC * 33, cnt, 0.125, lane);
+    add_blocks<NA * ND>(pk, oAD, sm + S::R_AD * 33, cnt, 0.125, lane);
+    add_blocks<NB * NC>(pk, oBC, sm + S::R_BC * 33, cnt, 0.125, lane);
+    add_blocks<NB * ND>(pk, oBD, sm + S::R_BD * 33, cnt, 0.125, lane);
+    add_blocks<NC * ND>(pj, oCD, sm + S::R_CD * 33, cnt, 0.25, lane);
+    __syncwarp();   // the rows are refilled for the next chunk
+  }
+}
+
+template <int LA, int LB, int LC, int LD, int KEPT>
+void run(const MolLaunch& ql, int num_sms, cudaStream_t s) {
+  using S = DigestShape<LA, LB, LC, LD, KEPT>;
+  constexpr int bytes = S::PER_WARP * S::WARPS * 8;
+  auto kern = k_digest<LA, LB, LC, LD, KEPT>;
+  cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
+  const int per_sm = std::max(1, std::min(2048 / (32 * S::WARPS), (220 * 1024) / (bytes + 1024)));
+  const int grid = std::min((ql.tn + S::WARPS - 1) / S::WARPS, num_sms * std::min(per_sm, 8));
+  kern<<<std::max(grid, 1), 32 * S::WARPS, bytes, s>>>(ql);
+}
+
+// the kept bits that matter to a class: those of the angular momenta it has
+template <int LA, int LB, int LC, int LD>
+void pick(const MolLaunch& ql, int num_sms, cudaStream_t s) {
+  constexpr bool p = LA == 1 || LB == 1 || LC == 1 || LD == 1, d = LA == 2 || LB == 2 || LC == 2 || LD == 2;
+  const int bits = ql.lower_kept_bits & ((p ? 2 : 0) | (d ? 4 : 0));
+  if (bits == 0) return run<LA, LB, LC, LD, 0>(ql, num_sms, s);
+  if constexpr (p) {
+    if (bits == 2) return run<LA, LB, LC, LD, 2>(ql, num_sms, s);
+  }
+  if constexpr (d) {
+    if (bits == 4) return run<LA, LB, LC, LD, 4>(ql, num_sms, s);
+  }
+  if constexpr (p && d) return run<LA, LB, LC, LD, 6>(ql, num_sms, s);
+}
+
+}  // namespace
+
+void launch_digest(int cb, int ck, const MolLaunch& ql, int num_sms, cudaStream_t s) {
+  switch (cb * 8 + ck) {
+#define D(CB, CK, A, B, C, E) case CB * 8 + CK: return pick<A, B, C, E>(ql, num_sms, s);
+    D(1, 0, 1, 0, 0, 0) D(1, 1, 1, 0, 1, 0)
+    D(2, 0, 1, 1, 0, 0) D(2, 1, 1, 1, 1, 0) D(2, 2, 1, 1, 1, 1)
+    D(3, 0, 2, 0, 0, 0) D(3, 1, 2, 0, 1, 0) D(3, 2, 2, 0, 1, 1) D(3, 3, 2, 0, 2, 0)
+    D(4, 0, 2, 1, 0, 0) D(4, 1, 2, 1, 1, 0) D(4, 2, 2, 1, 1, 1) D(4, 3, 2, 1, 2, 0) D(4, 4, 2, 1, 2, 1)
+    D(5, 0, 2, 2, 0, 0) D(5, 1, 2, 2, 1, 0) D(5, 2, 2, 2, 1, 1) D(5, 3, 2, 2, 2, 0)
+#undef D
+    default: return;
+  }
+}
+
+}  // namespace pfe

@@ -76,6 +76,19 @@ struct MolLaunch {
   int myid, numprocs;
   const MolLaunch* insts;   // batches: the launch record of every instance (Chunk::inst), else null
   int lower_kept_bits;      // bit L: some shell of top L has a coefficient on a lower component
+  // block panels (see Panels): the density and the J', K' accumulators of the
+  // digestion kernels, and the panel row where a shell's block begins
+  const double* pd;
+  double* pj;
+  double* pk;
+  const int* poff;
+  const int* ptgt;        // panel row -> target (-1: none)
+  int np;                 // panel rows
+  // one tile of a straight-line class: tickets [t0, t0 + tn) of this rank's chunks; X of
+  // ticket t0 + t at xbuf + t * (kept integrals) * 32, xlive[t] set when it holds any quartet
+  int t0, tn;
+  double* xbuf;
+  unsigned char* xlive;
 };
 
 // The launch record of a set-up molecular context for target-space density d_dt.
@@ -146,12 +159,29 @@ __device__ __forceinline__ double dt_at(const double* __restrict__ D, int nt, in
 // registers; the bra's primitive pairs are walked in step by the whole warp.
 // Classes with more integrals than registers hold X in NPASS launches, pass
 // PASS keeping the bra components ab in [AB0, AB1) (the recursion is repeated
-// per pass; the outputs a pass does not keep are dead code in it).
+// per pass; the outputs a pass does not keep are dead code in it).  X then goes to
+// memory and is digested once per group quartet by the class's digestion kernel
+// (pfe_mol_digest.cu).
 // Angular momentum of component i of a cumulative shell, in the reference's
 // component order (x power outer, z power inner: s, z, zz, y, yz, yy, x, xz, xy, xx).
 __host__ __device__ constexpr int comp_tot(int L, int i) {
   return L == 0 ? 0 : (L == 1 ? (i == 0 ? 0 : 1) : (i == 0 ? 0 : (i == 1 || i == 3 || i == 6) ? 1 : 2));
 }
+
+// Position of component i among its shell's components ordered by |i| (stable): the
+// order of the panel rows and of the stored integrals.
+__host__ __device__ constexpr int comp_rank(int L, int i) {
+  int r = 0;
+  for (int k = 0; k < ncum(L); ++k)
+    if (comp_tot(L, k) < comp_tot(L, i) || (comp_tot(L, k) == comp_tot(L, i) && k < i)) ++r;
+  return r;
+}
+
+// Components a shell of top L keeps: all of them where some shell of that L has a
+// coefficient below its top level (bit L of the lower_kept bits), else the top level,
+// which comes last in the order.
+__host__ __device__ constexpr int kept_first(int L, int bits) { return (L == 0 || ((bits >> L) & 1)) ? 0 : ncum(L - 1); }
+__host__ __device__ constexpr int kept_n(int L, int bits) { return ncum(L) - kept_first(L, bits); }
 
 // Bra component pairs ab = a*NB + b ordered by (|a|, |b|): the passes of a
 // class then keep the lower (for pure shells coefficient-free) components
@@ -275,8 +305,6 @@ __global__ void __launch_bounds__(128, GqOccupancy<LA, LB, LC, LD>::blocks) k_gq
   constexpr int XN = (AB1 - AB0) * NCD;
   static_assert(AB0 < NAB, "every pass keeps at least one bra component pair");
   // the pass keeps the pairs ab at positions [AB0, AB1) of ORD; X(k, cd) is pair ORD.ab[AB0 + k]
-  auto in_pass = [&](int a, int b) { const int k = ORD.pos[a * NB + b]; return k >= AB0 && k < AB1; };
-  auto xi = [&](int a, int b, int cc, int d) { return (ORD.pos[a * NB + b] - AB0) * NCD + cc * ND + d; };
   const int lane = threadIdx.x & 31;
   const int nchunks = *lq.nchunks;
   const double c2pi = 2.0 / sqrt(REF_PI);
@@ -297,8 +325,9 @@ __global__ void __launch_bounds__(128, GqOccupancy<LA, LB, LC, LD>::blocks) k_gq
   for (;;) {
     int t = 0;
     if (lane == 0) t = atomicAdd(lq.queue + PASS, 1);
-    const int c = __shfl_sync(0xffffffffu, t, 0) * lq.numprocs + lq.myid;
-    if (c >= nchunks) break;
+    t = __shfl_sync(0xffffffffu, t, 0);
+    const int c = (lq.t0 + t) * lq.numprocs + lq.myid;
+    if (t >= lq.tn || c >= nchunks) break;
     const Chunk ch = lq.chunks[c];
     // this chunk's instance: batches read its launch record from global memory
     const MolLaunch& ql = [&]() -> const MolLaunch& {
@@ -438,101 +467,49 @@ __global__ void __launch_bounds__(128, GqOccupancy<LA, LB, LC, LD>::blocks) k_gq
       for (int o = 16; o > 0; o >>= 1) n += __shfl_xor_sync(0xffffffffu, n, o);
       if (lane == 0 && n) atomicAdd(ql.n32, n);
     }
-    // digestion of this pass's part of X against the target-space density
     if (!__any_sync(0xffffffffu, any)) continue;   // nothing passed the screens in this chunk
-    const double* __restrict__ D = ql.dt;
-    const int I0 = ijg.x, J0 = ijg.y, K0 = klh.x, L0 = klh.y;
-    int ta[NA], tb[NB], tc[NC], td[ND];
-#pragma unroll
-    for (int x = 0; x < NA; ++x) ta[x] = stidx[I0 * MAXCOMP + x];
-#pragma unroll
-    for (int x = 0; x < NB; ++x) tb[x] = stidx[J0 * MAXCOMP + x];
-#pragma unroll
-    for (int x = 0; x < NC; ++x) tc[x] = stidx[K0 * MAXCOMP + x];
-#pragma unroll
-    for (int x = 0; x < ND; ++x) td[x] = stidx[L0 * MAXCOMP + x];
-    // J'(ab) += 1/4 sum_cd P(cd) X: the bra is the warp's, reduce over lanes first
-#pragma unroll
-    for (int k = AB0; k < AB1; ++k) {
-      double v = 0.0;
-#pragma unroll
-      for (int cc = 0; cc < NC; ++cc)
-#pragma unroll
-        for (int d = 0; d < ND; ++d) v = fma(dt_at(D, nt, tc[cc], td[d]), X[(k - AB0) * NCD + cc * ND + d], v);
-      v = warp_sum(v);
-      if (lane == 0) add_target(ql.jt, nt, ta[ORD.ab[k] / NB], tb[ORD.ab[k] % NB], 0.25 * v);
-    }
-    if (act && any) {
-      // J'(cd) += 1/4 sum_ab P(ab) X
-      double Pab[NAB];
-#pragma unroll
-      for (int k = AB0; k < AB1; ++k) Pab[ORD.ab[k]] = dt_at(D, nt, ta[ORD.ab[k] / NB], tb[ORD.ab[k] % NB]);
-#pragma unroll
-      for (int cd = 0; cd < NCD; ++cd) {
-        double v = 0.0;
-#pragma unroll
-        for (int k = AB0; k < AB1; ++k) v = fma(Pab[ORD.ab[k]], X[(k - AB0) * NCD + cd], v);
-        add_target(ql.jt, nt, tc[cd / ND], td[cd % ND], 0.25 * v);
+    if constexpr (LT == 0) {
+      // one integral per lane: digested here against the target-space density
+      const double* __restrict__ D = ql.dt;
+      const int ta = stidx[ijg.x * MAXCOMP], tb = stidx[ijg.y * MAXCOMP];
+      const int tc = stidx[klh.x * MAXCOMP], td = stidx[klh.y * MAXCOMP];
+      const double v = warp_sum(dt_at(D, nt, tc, td) * X[0]);   // the bra is the warp's
+      if (lane == 0) add_target(ql.jt, nt, ta, tb, 0.25 * v);
+      if (act && any) {
+        add_target(ql.jt, nt, tc, td, 0.25 * dt_at(D, nt, ta, tb) * X[0]);
+        add_target(ql.kt, nt, ta, td, 0.125 * dt_at(D, nt, tb, tc) * X[0]);
+        add_target(ql.kt, nt, ta, tc, 0.125 * dt_at(D, nt, tb, td) * X[0]);
+        add_target(ql.kt, nt, tb, td, 0.125 * dt_at(D, nt, ta, tc) * X[0]);
+        add_target(ql.kt, nt, tb, tc, 0.125 * dt_at(D, nt, ta, td) * X[0]);
       }
-      // K'(ad) += 1/8 P(bc) X ; K'(ac) += 1/8 P(bd) X   (in_pass folds at compile time)
+    } else {
+      // this pass's part of X to the digestion kernel: the kept components, one
+      // coalesced 256-byte row per integral
+      const int bits = lq.lower_kept_bits;
+      const int fa = kept_first(LA, bits), fb = kept_first(LB, bits), fc = kept_first(LC, bits),
+                fd = kept_first(LD, bits);
+      const int nb = NB - fb, nc = NC - fc, nd = ND - fd;
+      double* __restrict__ xb = lq.xbuf + (size_t)t * ((size_t)(NA - fa) * nb * nc * nd * 32) + lane;
 #pragma unroll
-      for (int a = 0; a < NA; ++a) {
-        bool a_in = false;
+      for (int k = AB0; k < AB1; ++k) {
+        const int ra = comp_rank(LA, ORD.ab[k] / NB) - fa, rb = comp_rank(LB, ORD.ab[k] % NB) - fb;
+        if (ra < 0 || rb < 0) continue;
 #pragma unroll
-        for (int b = 0; b < NB; ++b) a_in = a_in || in_pass(a, b);
-        if (!a_in) continue;
+        for (int cc = 0; cc < NC; ++cc)
 #pragma unroll
-        for (int d = 0; d < ND; ++d) {
-          double v = 0.0;
-#pragma unroll
-          for (int b = 0; b < NB; ++b)
-            if (in_pass(a, b))
-#pragma unroll
-              for (int cc = 0; cc < NC; ++cc) v = fma(dt_at(D, nt, tb[b], tc[cc]), X[xi(a, b, cc, d)], v);
-          add_target(ql.kt, nt, ta[a], td[d], 0.125 * v);
-        }
-#pragma unroll
-        for (int cc = 0; cc < NC; ++cc) {
-          double v = 0.0;
-#pragma unroll
-          for (int b = 0; b < NB; ++b)
-            if (in_pass(a, b))
-#pragma unroll
-              for (int d = 0; d < ND; ++d) v = fma(dt_at(D, nt, tb[b], td[d]), X[xi(a, b, cc, d)], v);
-          add_target(ql.kt, nt, ta[a], tc[cc], 0.125 * v);
-        }
+          for (int d = 0; d < ND; ++d) {
+            const int rc = comp_rank(LC, cc) - fc, rd = comp_rank(LD, d) - fd;
+            if (rc < 0 || rd < 0) continue;
+            xb[(((ra * nb + rb) * nc + rc) * nd + rd) * 32] = X[(k - AB0) * NCD + cc * ND + d];
+          }
       }
-      // K'(bd) += 1/8 P(ac) X ; K'(bc) += 1/8 P(ad) X
-#pragma unroll
-      for (int b = 0; b < NB; ++b) {
-        bool b_in = false;
-#pragma unroll
-        for (int a = 0; a < NA; ++a) b_in = b_in || in_pass(a, b);
-        if (!b_in) continue;
-#pragma unroll
-        for (int d = 0; d < ND; ++d) {
-          double v = 0.0;
-#pragma unroll
-          for (int a = 0; a < NA; ++a)
-            if (in_pass(a, b))
-#pragma unroll
-              for (int cc = 0; cc < NC; ++cc) v = fma(dt_at(D, nt, ta[a], tc[cc]), X[xi(a, b, cc, d)], v);
-          add_target(ql.kt, nt, tb[b], td[d], 0.125 * v);
-        }
-#pragma unroll
-        for (int cc = 0; cc < NC; ++cc) {
-          double v = 0.0;
-#pragma unroll
-          for (int a = 0; a < NA; ++a)
-            if (in_pass(a, b))
-#pragma unroll
-              for (int d = 0; d < ND; ++d) v = fma(dt_at(D, nt, ta[a], td[d]), X[xi(a, b, cc, d)], v);
-          add_target(ql.kt, nt, tb[b], tc[cc], 0.125 * v);
-        }
-      }
+      if (lane == 0) lq.xlive[t] = 1;
     }
   }
 }
+
+// Digestion of the stored X of a class's tile (pfe_mol_digest.cu), after its passes.
+void launch_digest(int cb, int ck, const MolLaunch& ql, int num_sms, cudaStream_t s);
 
 // ------------------------------------------------------------------ launch tables
 
