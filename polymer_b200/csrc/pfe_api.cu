@@ -498,9 +498,6 @@ int32_t pfe_context_create(int32_t device, pfe_context** out) {
   ctx->device = device;
   PFE_CUDA(cudaDeviceGetAttribute(&ctx->num_sms, cudaDevAttrMultiProcessorCount, device));
   PFE_CUDA(cudaStreamCreateWithFlags(&ctx->stream, cudaStreamNonBlocking));
-  PFE_CUDA(cudaStreamCreateWithFlags(&ctx->side, cudaStreamNonBlocking));
-  PFE_CUDA(cudaEventCreateWithFlags(&ctx->ev_fork, cudaEventDisableTiming));
-  PFE_CUDA(cudaEventCreateWithFlags(&ctx->ev_join, cudaEventDisableTiming));
   *out = ctx;   // the cuBLAS handle comes with the first call that needs it (ensure_blas)
   return PFE_OK;
 }
@@ -511,12 +508,14 @@ int32_t pfe_context_destroy(pfe_context* ctx) {
   cudaStreamSynchronize(ctx->stream);
   reset_context(ctx);
   if (ctx->blas) cublasDestroy(ctx->blas);
-  if (ctx->side) {
-    cudaStreamSynchronize(ctx->side);
-    cudaStreamDestroy(ctx->side);
+  for (int k = 0; k < pfe_context::kSide; ++k) {
+    if (ctx->side[k]) {
+      cudaStreamSynchronize(ctx->side[k]);
+      cudaStreamDestroy(ctx->side[k]);
+    }
+    if (ctx->ev_join[k]) cudaEventDestroy(ctx->ev_join[k]);
   }
   if (ctx->ev_fork) cudaEventDestroy(ctx->ev_fork);
-  if (ctx->ev_join) cudaEventDestroy(ctx->ev_join);
   if (ctx->stream) cudaStreamDestroy(ctx->stream);
   delete ctx;
   return PFE_OK;
@@ -732,7 +731,7 @@ int32_t pfe_batch_census(pfe_batch* b, pfe_census* out) {
   }
   int n = 0;
   for (int i = 0; i < b->nlaunch; ++i)
-    n += (b->launches[i].variant == 0 && b->launches[i].has_straight) ? b->launches[i].npass_live : 1;
+    n += (b->launches[i].variant == 0 && b->launches[i].has_straight) ? b->launches[i].launches_live : 1;
   tot.kernel_launches = n;
   *out = tot;
   return PFE_OK;
@@ -761,12 +760,11 @@ int32_t pfe_context_census(pfe_context* ctx, pfe_census* out) {
   }
   out->pairs = ctx->npairs;
   if (ctx->molecular) {
-    // class kernels (straight-line passes), the target-space density and its check,
-    // the two symmetrisations (primitive targets: the contraction is cuBLAS), the block
-    // maxima under density screening or mixed precision
+    // class kernels (pass groups and digestion), the target-space density and its check,
+    // the panels' beginning and end, the block maxima under density screening or mixed precision
     int n = 0;
     for (int i = 0; i < ctx->nlaunch; ++i)
-      n += (ctx->launches[i].variant == 0 && ctx->launches[i].has_straight) ? ctx->launches[i].npass_live : 1;
+      n += (ctx->launches[i].variant == 0 && ctx->launches[i].has_straight) ? ctx->launches[i].launches_live : 1;
     n += (ctx->contracted ? 2 : 0) + 2 + ((ctx->dtol > 0.0 || ctx->mcut > 0.0) ? 1 : 0);
     out->kernel_launches = n;
   } else {

@@ -104,7 +104,7 @@ struct ClassLaunch {
   size_t smem_wide;
   int* queue;                // device work queue: one chunk counter per launch (pass), zeroed before each
   int npass;                 // register passes of the straight-line variant
-  int npass_live;            // of which launched: the others keep no component with a coefficient
+  int launches_live;         // its kernel launches: pass groups with a component that has a coefficient, digestion
   int gmul = 32;             // straight-line variant: persistent grid of up to gmul blocks per SM
 };
 
@@ -128,10 +128,12 @@ struct pfe_context {
   int device = 0;
   int num_sms = 148;
   cudaStream_t stream = nullptr;
-  // the interpreter classes' launches run on `side`, beside the straight-line
-  // classes on the caller's stream (forked and joined with the two events)
-  cudaStream_t side = nullptr;
-  cudaEvent_t ev_fork = nullptr, ev_join = nullptr;
+  // class launches beside those on the caller's stream (launch_classes), forked
+  // and joined with the events; made at set-up (ensure_side)
+  static constexpr int kSide = 5;
+  cudaStream_t side[kSide] = {};
+  cudaEvent_t ev_fork = nullptr, ev_join[kSide] = {};
+  bool concurrent = false;   // every class has a buffer of its own for its stored integrals
   cublasHandle_t blas = nullptr;
   bool ready = false;
   uint64_t key = 0;
@@ -273,6 +275,7 @@ struct pfe_batch {
   int* d_queue = nullptr;           // the joined launches' work queues (64 counters each)
   long long* d_off = nullptr;       // off[] on the device (the batched symmetrisation)
   bool all_contracted = false;      // every instance digests in contracted space
+  bool concurrent = false;          // every class has a buffer of its own for its stored integrals
   void* d_insts = nullptr;          // the instances' launch records (MolLaunch) on the device
   void* h_insts = nullptr;          // ... and their pinned host copy, uploaded by every build (so a
                                     // captured graph re-reads it at each replay)
@@ -314,6 +317,7 @@ inline bool ensure_blas(pfe_context* ctx) {
   }
   return true;
 }
+int ensure_side(pfe_context* ctx);
 int batch_setup(pfe_batch* b);
 int batch_fock_pc(pfe_batch* b, const double* d_pc, double* d_cc, double* d_xc, cudaStream_t s);
 int batch_refresh(pfe_batch* b, const double* d_pc);

@@ -481,7 +481,7 @@ struct PanelView {
   int np;
 };
 
-// The density into the panels and J', K' to zero, one element per thread.
+// The density into the panels and the panels' J', K' to zero, one element per thread.
 __device__ __forceinline__ void panel_in(const PanelView& v, const double* __restrict__ dt, int nt, long long t,
                                          double* __restrict__ pd, double* __restrict__ pj, double* __restrict__ pk) {
   const int p = (int)(t % v.np), q = (int)(t / v.np);
@@ -504,10 +504,21 @@ __device__ __forceinline__ double panel_sym(const PanelView& v, const double* __
   return a;
 }
 
-__global__ void k_panel_in(PanelView v, const double* __restrict__ dt, int nt, double* __restrict__ pd,
-                           double* __restrict__ pj, double* __restrict__ pk) {
+constexpr int kQueueInts = 64 * 64;   // work-queue counters of a context or batch
+
+// The beginning of a build in one launch: the panels, the target-space J'/K', the
+// work-queue counters and the FP32 counter to zero, with density screening or mixed
+// precision (bmax non-null) the block maxima too.
+__global__ void k_begin(PanelView v, const double* __restrict__ dt, int nt, double* __restrict__ pd,
+                        double* __restrict__ pj, double* __restrict__ pk, double* __restrict__ jt,
+                        double* __restrict__ kt, int* __restrict__ queue, unsigned long long* __restrict__ n32,
+                        double* __restrict__ bmax, int nblk) {
   const long long t = blockIdx.x * (long long)blockDim.x + threadIdx.x;
   if (t < (long long)v.np * v.np) panel_in(v, dt, nt, t, pd, pj, pk);
+  if (t < (long long)nt * nt) jt[t] = kt[t] = 0.0;
+  if (t < kQueueInts) queue[t] = 0;
+  if (bmax && t < (long long)nblk * nblk) bmax[t] = 0.0;
+  if (t == 0) *n32 = 0ull;
 }
 
 // C_C = J' + J'^T and X_C = K' + K'^T from the target-space accumulators and the panels.
@@ -905,6 +916,14 @@ static int lower_kept_bits(const pfe_context* ctx) {
   return bits;
 }
 
+// Kernel launches of a class's straight-line variant: its pass groups that are live
+// with these lower_kept bits, and the digestion of the stored integrals.
+static int class_launches(const ClassLaunch& cl, int bits) {
+  if (!cl.has_straight) return 1;
+  return pass_groups_live(kCL[cl.cb][0], kCL[cl.cb][1], kCL[cl.ck][0], kCL[cl.ck][1], cl.npass, bits) +
+         (cl.cb > 0 ? 1 : 0);
+}
+
 static int size_wide(ClassLaunch& cl, const int kept_max[3], const bool lower_kept[3]) {
   cl.has_wide = false;
   const WideVariant wv = wide_variant(cl.cb, cl.ck);
@@ -1024,34 +1043,49 @@ static int kept_integrals(int cb, int ck, int bits) {
   return kept_n(kCL[cb][0], bits) * kept_n(kCL[cb][1], bits) * kept_n(kCL[ck][0], bits) * kept_n(kCL[ck][1], bits);
 }
 
-// Memory for the stored integrals of the straight-line classes: one buffer that the
-// classes use one after another, of the largest class's size up to kTileBytes; larger
-// classes run in tiles of that size.  Measured on B200: a tile's passes last long
-// enough (milliseconds) that their tails do not show, and the buffer's traffic
-// (written and read once, at HBM rate) is a tenth of what the digestion inside every
-// pass cost.
+// Memory for the stored integrals of the straight-line classes.  Where all classes fit
+// kTogetherBytes together, each has a buffer of its own and the classes run side by
+// side (launch_classes); otherwise they use one buffer after another, of the largest
+// class's size up to kTileBytes, and larger classes run in tiles of that size.
+// Measured on B200: a tile's passes last long enough (milliseconds) that their tails
+// do not show, and the buffer's traffic (written and read once, at HBM rate) is a tenth
+// of what the digestion inside every pass cost.
 template <typename Owner>
 static int alloc_integrals(Owner* own, ClassLaunch* launches, int nlaunch, int bits) {
-  constexpr size_t kTileBytes = (size_t)1 << 30;
-  size_t most = 0, flags = 0;
+  constexpr size_t kTileBytes = (size_t)1 << 30, kTogetherBytes = (size_t)1 << 30;
+  auto bytes_per = [&](const ClassLaunch& cl) {
+    return sizeof(double) * 32 * (size_t)kept_integrals(cl.cb, cl.ck, bits);
+  };
+  size_t most = 0, most_flags = 0, sum = 0, sum_flags = 0;
   for (int i = 0; i < nlaunch; ++i) {
     ClassLaunch& cl = launches[i];
+    cl.xcap = 0;
     if (!cl.has_straight || cl.cb == 0) continue;
-    const size_t per = sizeof(double) * 32 * (size_t)kept_integrals(cl.cb, cl.ck, bits);
-    cl.xcap = (int)std::max<size_t>(1, std::min<size_t>(kTileBytes / per, (size_t)cl.nchunks_host));
-    most = std::max(most, per * cl.xcap);
-    flags = std::max(flags, (size_t)cl.xcap);
+    cl.xcap = (int)std::max<size_t>(1, std::min<size_t>(kTileBytes / bytes_per(cl), (size_t)cl.nchunks_host));
+    most = std::max(most, bytes_per(cl) * cl.xcap);
+    most_flags = std::max(most_flags, (size_t)cl.xcap);
+    sum += bytes_per(cl) * (size_t)cl.nchunks_host;
+    sum_flags += (size_t)cl.nchunks_host;
   }
+  own->concurrent = sum <= kTogetherBytes;
   double* x = nullptr;
   unsigned char* f = nullptr;
   if (most > 0) {
-    PFE_CUDA(own->alloc((void**)&x, most));
+    const size_t flags = own->concurrent ? sum_flags : most_flags;
+    PFE_CUDA(own->alloc((void**)&x, own->concurrent ? sum : most));
     PFE_CUDA(own->alloc((void**)&f, flags));
     PFE_CUDA(cudaMemset(f, 0, flags));
   }
+  size_t xo = 0, fo = 0;
   for (int i = 0; i < nlaunch; ++i) {
-    launches[i].xbuf = x;
-    launches[i].xlive = f;
+    ClassLaunch& cl = launches[i];
+    if (cl.xcap == 0) continue;
+    cl.xbuf = x + xo;
+    cl.xlive = f + fo;
+    if (own->concurrent) {
+      xo += bytes_per(cl) / sizeof(double) * cl.xcap;
+      fo += cl.xcap;
+    }
   }
   return PFE_OK;
 }
@@ -1291,8 +1325,8 @@ int molecular_setup(pfe_context* ctx, const pfe_args* a) {
   // the chunks of every class pair cb >= ck in one list, a class pair after another
   ctx->nlaunch = 0;
   ctx->census_quartets = ctx->census_flops = ctx->census_ref = 0.0;
-  PFE_CUDA(ctx->alloc((void**)&ctx->d_queue, sizeof(int) * 64 * 64));
-  PFE_CUDA(cudaMemsetAsync(ctx->d_queue, 0, sizeof(int) * 64 * 64, s));
+  PFE_CUDA(ctx->alloc((void**)&ctx->d_queue, sizeof(int) * kQueueInts));
+  PFE_CUDA(cudaMemsetAsync(ctx->d_queue, 0, sizeof(int) * kQueueInts, s));
   PairRows rows{};
   unsigned int serial = 0;
   for (int cb = 0; cb < 6; ++cb)
@@ -1352,12 +1386,7 @@ int molecular_setup(pfe_context* ctx, const pfe_args* a) {
       cl.quartets = nq;
       cl.has_straight = straight_launcher(cb, ck) != nullptr;
       cl.npass = cl.has_straight ? straight_npass(cb, ck) : 0;
-      cl.npass_live = 0;   // register passes actually launched (the rest keep no coefficient)
-      for (int p = 0; p < cl.npass; ++p)
-        cl.npass_live += (cl.npass == 1 || pass_live(kCL[cb][0], kCL[cb][1], kCL[ck][0], kCL[ck][1], cl.npass, p,
-                                                     lower_kept_bits(ctx)))
-                             ? 1
-                             : 0;
+      cl.launches_live = class_launches(cl, lower_kept_bits(ctx));
       cl.has_table = false;
       cl.variant = 0;
       cl.xg = nullptr;
@@ -1432,6 +1461,7 @@ int molecular_setup(pfe_context* ctx, const pfe_args* a) {
     pfe_context* const self = ctx;
     if ((rc = finish_chunks(ctx, &self, 1, ctx->launches, ctx->nlaunch, s)) != PFE_OK) return rc;
     if ((rc = build_panels(ctx, lower_kept_bits(ctx))) != PFE_OK) return rc;
+    if ((rc = ensure_side(ctx)) != PFE_OK) return rc;
     if ((rc = alloc_integrals(ctx, ctx->launches, ctx->nlaunch, lower_kept_bits(ctx))) != PFE_OK) return rc;
     free_raw(ctx);
   }
@@ -1483,12 +1513,13 @@ static MolLaunch make_launch(pfe_context* ctx, const double* d_dt) {
   return ql;
 }
 
+// One class of a build on stream s; its work-queue counters are zero (the build's
+// beginning), those of later tiles are zeroed here.
 static void launch_class(pfe_context* ctx, const ClassLaunch& cl, MolLaunch ql, int variant, cudaStream_t s,
                          bool mixed) {
   ql.chunks = cl.chunks;
   ql.nchunks = cl.d_nchunks;
   ql.queue = cl.queue;
-  cudaMemsetAsync(cl.queue, 0, sizeof(int) * 64, s);   // every launch (pass) of the class starts its queue at 0
   const int work = (cl.nchunks_host + ctx->numprocs - 1) / ctx->numprocs;
   if ((variant == 0 && cl.has_straight) || !cl.has_table) {
     // (00|00) digests in its kernel; the other classes store X tile by tile
@@ -1525,8 +1556,6 @@ static void launch_class(pfe_context* ctx, const ClassLaunch& cl, MolLaunch ql, 
   }
 }
 
-static size_t target_bytes(const pfe_context* ctx) { return sizeof(double) * (size_t)ctx->nt * ctx->nt; }
-
 // Density in target space: P_P itself (primitive targets) or P_C read off P_P
 // and checked (contracted targets); returns the pointer the kernels read.
 static const double* target_density(pfe_context* ctx, const double* d_pp, cudaStream_t s) {
@@ -1540,10 +1569,23 @@ static const double* target_density(pfe_context* ctx, const double* d_pp, cudaSt
   return ctx->d_pt;
 }
 
-static void launch_panel_in(pfe_context* ctx, const double* d_dt, cudaStream_t s) {
-  const long long n2 = (long long)ctx->np * ctx->np;
-  k_panel_in<<<(unsigned)((n2 + 255) / 256), 256, 0, s>>>(panel_view(ctx), d_dt, ctx->nt, ctx->d_pd, ctx->d_pj,
-                                                          ctx->d_pk);
+// Zero every accumulator and work queue of a build and fill the density panels;
+// with density screening or mixed precision, the block maxima of the density.
+static int begin_build(pfe_context* ctx, const double* d_dt, cudaStream_t s, bool always_bmax = false) {
+  const bool screen = always_bmax || ctx->dtol > 0.0 || ctx->mcut > 0.0;
+  const long long nt2 = (long long)ctx->nt * ctx->nt;
+  const long long n = std::max<long long>(
+      {(long long)ctx->np * ctx->np, nt2, (long long)kQueueInts, screen ? (long long)ctx->nblk * ctx->nblk : 0});
+  k_begin<<<(unsigned)((n + 255) / 256), 256, 0, s>>>(panel_view(ctx), d_dt, ctx->nt, ctx->d_pd, ctx->d_pj, ctx->d_pk,
+                                                      ctx->d_jp, ctx->d_kp, ctx->d_queue, ctx->d_n32,
+                                                      screen ? ctx->d_bmax : nullptr, ctx->nblk);
+  PFE_CUDA(cudaGetLastError());
+  if (screen) {
+    k_block_dmax<<<(unsigned)((nt2 + 255) / 256), 256, 0, s>>>(d_dt, ctx->nt, ctx->d_tblk, ctx->nblk,
+                                                               (unsigned long long*)ctx->d_bmax);
+    PFE_CUDA(cudaGetLastError());
+  }
+  return PFE_OK;
 }
 
 // The outputs from the accumulators: contracted targets symmetrised straight into
@@ -1585,11 +1627,15 @@ static int tune_class(pfe_context* ctx, ClassLaunch& cl, const MolLaunch& ql, cu
     float tv = 1e30f;
     for (int gi = 0; gi < ng; ++gi) {
       if (v == 0) cl.gmul = kGmul[gi];
-      launch_class(ctx, cl, ql, v, s, mixed);
+      auto once = [&]() {
+        cudaMemsetAsync(cl.queue, 0, sizeof(int) * 64, s);
+        launch_class(ctx, cl, ql, v, s, mixed);
+      };
+      once();
       float t = 1e30f;
       for (int r = 0; r < 2; ++r) {
         PFE_CUDA(cudaEventRecord(e0, s));
-        launch_class(ctx, cl, ql, v, s, mixed);
+        once();
         PFE_CUDA(cudaEventRecord(e1, s));
         PFE_CUDA(cudaEventSynchronize(e1));
         float ms = 0.f;
@@ -1610,8 +1656,8 @@ static int tune_class(pfe_context* ctx, ClassLaunch& cl, const MolLaunch& ql, cu
 int autotune(pfe_context* ctx, const double* d_pp, cudaStream_t s) {
   const double* d_dt = target_density(ctx, d_pp, s);
   const MolLaunch ql = make_launch(ctx, d_dt);
-  launch_panel_in(ctx, d_dt, s);
-  PFE_CUDA(cudaGetLastError());
+  const int rc0 = begin_build(ctx, d_dt, s);
+  if (rc0 != PFE_OK) return rc0;
   cudaEvent_t e0, e1;
   PFE_CUDA(cudaEventCreate(&e0));
   PFE_CUDA(cudaEventCreate(&e1));
@@ -1622,70 +1668,75 @@ int autotune(pfe_context* ctx, const double* d_pp, cudaStream_t s) {
   }
   cudaEventDestroy(e0);
   cudaEventDestroy(e1);
-  PFE_CUDA(cudaMemsetAsync(ctx->d_jp, 0, target_bytes(ctx), s));
-  PFE_CUDA(cudaMemsetAsync(ctx->d_kp, 0, target_bytes(ctx), s));
   PFE_CUDA(cudaStreamSynchronize(s));
   ctx->tuned = true;
   return PFE_OK;
 }
 
-// Zero the target-space J'/K' and the FP32 counter; block maxima of the density
-// when screening or mixed precision is on.
-static int prepare_build(pfe_context* ctx, const double* d_dt, cudaStream_t s, bool always_bmax = false) {
-  PFE_CUDA(cudaMemsetAsync(ctx->d_jp, 0, target_bytes(ctx), s));
-  PFE_CUDA(cudaMemsetAsync(ctx->d_kp, 0, target_bytes(ctx), s));
-  PFE_CUDA(cudaMemsetAsync(ctx->d_n32, 0, sizeof(unsigned long long), s));
-  launch_panel_in(ctx, d_dt, s);
-  PFE_CUDA(cudaGetLastError());
-  if (always_bmax || ctx->dtol > 0.0 || ctx->mcut > 0.0) {
-    const long long nt2 = (long long)ctx->nt * ctx->nt;
-    PFE_CUDA(cudaMemsetAsync(ctx->d_bmax, 0, sizeof(double) * (size_t)ctx->nblk * ctx->nblk, s));
-    k_block_dmax<<<(unsigned)((nt2 + 255) / 256), 256, 0, s>>>(d_dt, ctx->nt, ctx->d_tblk, ctx->nblk,
-                                                               (unsigned long long*)ctx->d_bmax);
-    PFE_CUDA(cudaGetLastError());
+int ensure_side(pfe_context* ctx) {
+  if (!ctx->ev_fork) PFE_CUDA(cudaEventCreateWithFlags(&ctx->ev_fork, cudaEventDisableTiming));
+  for (int k = 0; k < pfe_context::kSide; ++k) {
+    if (!ctx->side[k]) PFE_CUDA(cudaStreamCreateWithFlags(&ctx->side[k], cudaStreamNonBlocking));
+    if (!ctx->ev_join[k]) PFE_CUDA(cudaEventCreateWithFlags(&ctx->ev_join[k], cudaEventDisableTiming));
   }
   return PFE_OK;
 }
 
-// The class launches of one molecule's build: the interpreter classes (wide,
-// warp and block variants: few resident warps, bound by shared memory or
-// barriers) on the context's side stream, forked from s, and the straight-line
-// classes on s, so that the two kinds share the SMs; s then waits for the side
-// stream.  J' and K' take atomic adds only, so the order of the classes does not
-// matter.  Measured: C20H42 34.0 -> 32.0 ms.  Batches keep one stream (the
-// 32-cluster water batch was 2 % slower split: its interpreter classes are a
-// small share, and they slowed the straight-line ones beside them).  Serial on
-// s when `serial` (per-class timing).
+// The class launches of a build, forked from the caller's stream s onto side streams
+// and joined back (J' and K' take atomic adds only, so the order of the classes does
+// not matter).
+//   * Small builds (`together`: every class has its own buffer of stored integrals)
+//     spread the classes over all streams, the costliest first, each to the stream
+//     with the least work so far: their launches hold fewer warps than the GPU, and
+//     what a build lasts is the sum of their latencies.
+//   * Large builds run the straight-line classes one after another on s, and of a
+//     single molecule the interpreter classes (few resident warps, bound by shared
+//     memory or barriers) beside them on one side stream: C20H42 34.0 -> 32.0 ms; the
+//     32-cluster water batch was 2 % slower split that way.
+// Serial on s when `serial` (per-class timing).
 static int launch_classes(pfe_context* cx, const ClassLaunch* launches, int nlaunch, const MolLaunch& ql,
-                          cudaStream_t s, bool mixed, bool serial) {
-  bool any_side = false;
-  for (int i = 0; i < nlaunch && !serial; ++i)
-    any_side = any_side || !((launches[i].variant == 0 && launches[i].has_straight) || !launches[i].has_table);
-  const bool split = any_side && cx->side != nullptr;
-  if (split) {
-    PFE_CUDA(cudaEventRecord(cx->ev_fork, s));
-    PFE_CUDA(cudaStreamWaitEvent(cx->side, cx->ev_fork, 0));
-    for (int i = 0; i < nlaunch; ++i) {
-      const ClassLaunch& cl = launches[i];
-      if (!((cl.variant == 0 && cl.has_straight) || !cl.has_table)) launch_class(cx, cl, ql, cl.variant, cx->side, mixed);
+                          cudaStream_t s, bool mixed, bool together, bool serial) {
+  cudaStream_t on[64];
+  int order[64];
+  double load[pfe_context::kSide + 1] = {0.0};
+  bool used[pfe_context::kSide + 1] = {false};
+  auto work = [&](int i) { return launches[i].quartets * class_flops(launches[i].cb, launches[i].ck); };
+  for (int i = 0; i < nlaunch; ++i) order[i] = i;
+  const bool fork = !serial && cx->ev_fork != nullptr;
+  if (fork && together) std::sort(order, order + nlaunch, [&](int a, int b) { return work(a) > work(b); });
+  for (int j = 0; j < nlaunch; ++j) {
+    const ClassLaunch& cl = launches[order[j]];
+    int k = 0;
+    if (fork && together) {
+      for (int x = 1; x <= pfe_context::kSide; ++x)
+        if (load[x] < load[k]) k = x;
+      load[k] += work(order[j]);
+    } else if (fork && !ql.insts && !((cl.variant == 0 && cl.has_straight) || !cl.has_table)) {
+      k = 1;
     }
-    PFE_CUDA(cudaGetLastError());
+    used[k] = true;
+    on[order[j]] = k == 0 ? s : cx->side[k - 1];
   }
-  for (int i = 0; i < nlaunch; ++i) {
-    const ClassLaunch& cl = launches[i];
-    const bool straight = (cl.variant == 0 && cl.has_straight) || !cl.has_table;
-    if (!split || straight) launch_class(cx, cl, ql, cl.variant, s, mixed);
+  bool any = false;
+  for (int k = 1; k <= pfe_context::kSide; ++k) any = any || used[k];
+  if (any) PFE_CUDA(cudaEventRecord(cx->ev_fork, s));
+  for (int k = 1; k <= pfe_context::kSide; ++k)
+    if (used[k]) PFE_CUDA(cudaStreamWaitEvent(cx->side[k - 1], cx->ev_fork, 0));
+  for (int j = 0; j < nlaunch; ++j) {
+    const ClassLaunch& cl = launches[order[j]];
+    launch_class(cx, cl, ql, cl.variant, on[order[j]], mixed);
   }
   PFE_CUDA(cudaGetLastError());
-  if (split) {
-    PFE_CUDA(cudaEventRecord(cx->ev_join, cx->side));
-    PFE_CUDA(cudaStreamWaitEvent(s, cx->ev_join, 0));
-  }
+  for (int k = 1; k <= pfe_context::kSide; ++k)
+    if (used[k]) {
+      PFE_CUDA(cudaEventRecord(cx->ev_join[k - 1], cx->side[k - 1]));
+      PFE_CUDA(cudaStreamWaitEvent(s, cx->ev_join[k - 1], 0));
+    }
   return PFE_OK;
 }
 
 static int run_build(pfe_context* ctx, const double* d_dt, double* d_cc, double* d_xc, cudaStream_t s) {
-  const int rc = prepare_build(ctx, d_dt, s);
+  const int rc = begin_build(ctx, d_dt, s);
   if (rc != PFE_OK) return rc;
   const MolLaunch ql = make_launch(ctx, d_dt);
   if (ctx->profile) {
@@ -1695,7 +1746,7 @@ static int run_build(pfe_context* ctx, const double* d_dt, double* d_cc, double*
     PFE_CUDA(cudaEventRecord(ctx->ev[0], s));
   }
   if (!ctx->profile) {
-    const int rc2 = launch_classes(ctx, ctx->launches, ctx->nlaunch, ql, s, ctx->mcut > 0.0, false);
+    const int rc2 = launch_classes(ctx, ctx->launches, ctx->nlaunch, ql, s, ctx->mcut > 0.0, ctx->concurrent, false);
     if (rc2 != PFE_OK) return rc2;
   }
   for (int i = 0; i < ctx->nlaunch && ctx->profile; ++i) {
@@ -1776,7 +1827,7 @@ namespace pfe {
 // tagged with its instance.
 int batch_setup(pfe_batch* b) {
   b->nlaunch = 0;
-  PFE_CUDA(b->alloc((void**)&b->d_queue, sizeof(int) * 64 * 64));
+  PFE_CUDA(b->alloc((void**)&b->d_queue, sizeof(int) * kQueueInts));
   cudaStream_t st = nullptr;
   PFE_CUDA(cudaStreamCreateWithFlags(&st, cudaStreamNonBlocking));
   struct StreamGuard {
@@ -1798,10 +1849,7 @@ int batch_setup(pfe_batch* b) {
       {  // launched passes over the whole batch: a pass is skipped only if no instance needs it
         int bits = 0;
         for (pfe_context* c : b->inst) bits |= lower_kept_bits(c);
-        cl.npass_live = 0;
-        for (int p = 0; p < cl.npass; ++p)
-          cl.npass_live +=
-              (cl.npass == 1 || pass_live(kCL[cb][0], kCL[cb][1], kCL[ck][0], kCL[ck][1], cl.npass, p, bits)) ? 1 : 0;
+        cl.launches_live = class_launches(cl, bits);
       }
       if (cl.has_wide) {   // the wide variant's working set must cover every instance
         int km[3] = {1, 1, 1};
@@ -1828,7 +1876,8 @@ int batch_setup(pfe_batch* b) {
     if (rc != PFE_OK) return rc;
   }
   {
-    const int rc = alloc_integrals(b, b->launches, b->nlaunch, bits);
+    int rc = alloc_integrals(b, b->launches, b->nlaunch, bits);
+    if (rc == PFE_OK) rc = ensure_side(b->inst[0]);
     if (rc != PFE_OK) return rc;
   }
   PFE_CUDA(b->alloc(&b->d_insts, (sizeof(MolLaunch) + sizeof(PanelView)) * b->inst.size()));
@@ -1888,8 +1937,11 @@ static int batch_decontract(pfe_batch* b, const double* d_pc, cudaStream_t s) {
 // matrices) instead of seven small ones per instance: zero J'/K', the block
 // maxima and the FP32 counter and fill the density panels; the block maxima of |P_T|; after the class
 // kernels, C_C = J' + J'^T and X_C = K' + K'^T at the packed offsets.
-__global__ void k_batch_zero(const MolLaunch* __restrict__ insts, const PanelView* __restrict__ pv) {
+__global__ void k_batch_zero(const MolLaunch* __restrict__ insts, const PanelView* __restrict__ pv,
+                             int* __restrict__ queue) {
   const MolLaunch& q = insts[blockIdx.y];
+  if (blockIdx.y == 0)
+    for (int t = blockIdx.x * blockDim.x + threadIdx.x; t < kQueueInts; t += gridDim.x * blockDim.x) queue[t] = 0;
   const long long np2 = (long long)q.np * q.np;
   for (long long t = blockIdx.x * (long long)blockDim.x + threadIdx.x; t < np2; t += (long long)gridDim.x * blockDim.x)
     panel_in(pv[blockIdx.y], q.dt, q.nt, t, const_cast<double*>(q.pd), q.pj, q.pk);
@@ -1964,17 +2016,16 @@ int batch_fock_pc(pfe_batch* b, const double* d_pc, double* d_cc, double* d_xc, 
   const MolLaunch* di = static_cast<const MolLaunch*>(b->d_insts);
   const dim3 gb(8, (unsigned)n);
   const PanelView* dv = reinterpret_cast<const PanelView*>(di + n);
-  k_batch_zero<<<gb, 256, 0, s>>>(di, dv);
+  k_batch_zero<<<gb, 256, 0, s>>>(di, dv, b->d_queue);
   k_batch_dmax<<<gb, 256, 0, s>>>(di);
   PFE_CUDA(cudaGetLastError());
   pfe_context* c0 = b->inst[0];
   MolLaunch lq = make_launch(c0, c0->d_pt);
   lq.insts = di;
   for (pfe_context* c : b->inst) lq.lower_kept_bits |= lower_kept_bits(c);   // a pass is skipped only if dead everywhere
-  for (int i = 0; i < b->nlaunch; ++i) {
-    const ClassLaunch& cl = b->launches[i];
-    launch_class(c0, cl, lq, cl.variant, s, b->mixed);
-    PFE_CUDA(cudaGetLastError());
+  {
+    const int rc = launch_classes(c0, b->launches, b->nlaunch, lq, s, b->mixed, b->concurrent, false);
+    if (rc != PFE_OK) return rc;
   }
   if (b->all_contracted) {
     k_batch_symmetrize<<<gb, 256, 0, s>>>(di, dv, b->d_off, d_cc, d_xc);
@@ -2000,7 +2051,7 @@ int batch_autotune(pfe_batch* b, const double* d_pc, cudaStream_t s) {
   b->ev_pending = true;
   for (size_t k = 0; k < b->inst.size(); ++k) {
     pfe_context* c = b->inst[k];
-    if ((rc = prepare_build(c, c->contracted ? d_pc + b->off[k] : c->d_pt, s, true)) != PFE_OK) return rc;
+    if ((rc = begin_build(c, c->contracted ? d_pc + b->off[k] : c->d_pt, s, true)) != PFE_OK) return rc;
   }
   pfe_context* c0 = b->inst[0];
   MolLaunch lq = make_launch(c0, c0->d_pt);

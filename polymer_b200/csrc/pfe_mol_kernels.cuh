@@ -268,15 +268,6 @@ struct GqOccupancy {
 #endif
 };
 
-template <int LT>
-struct GqSmemBoys {
-#ifdef PFE_GQ_SMEM_BOYS
-  static constexpr bool use = BoysSmem<LT>::use;
-#else
-  static constexpr bool use = false;
-#endif
-};
-
 // Classes of total angular momentum up to maxl evaluate the Boys function without
 // the table (boys_direct): their lanes' per-quartet table-row gathers were half of
 // their L1 wavefronts.  Measured on the 32-cluster water batch: (10|00) 55.8 ->
@@ -293,7 +284,7 @@ struct GqBoysDirect {
 };
 
 template <int LA, int LB, int LC, int LD, int NPASS, int PASS, bool MIXED, bool BATCH>
-__global__ void __launch_bounds__(128, GqOccupancy<LA, LB, LC, LD>::blocks) k_gq(MolLaunch lq) {
+__device__ __forceinline__ void gq_pass(const MolLaunch& lq) {
   constexpr int NA = ncum(LA), NB = ncum(LB), NC = ncum(LC), ND = ncum(LD);
   constexpr int NI = NA * NB * NC * ND;
   constexpr int NAB = NA * NB;
@@ -308,17 +299,6 @@ __global__ void __launch_bounds__(128, GqOccupancy<LA, LB, LC, LD>::blocks) k_gq
   const int lane = threadIdx.x & 31;
   const int nchunks = *lq.nchunks;
   const double c2pi = 2.0 / sqrt(REF_PI);
-  // with PFE_GQ_SMEM_BOYS, classes of total angular momentum up to 4 read their
-  // Boys rows from a copy of the table's first rows in shared memory (the launch
-  // passes its size); off by default: measured on C20H42 it cost 10-16 % on the
-  // low classes (fewer resident blocks, the per-block copy), the L1-cached
-  // gathers of the global table are as fast
-  constexpr bool SBOYS = GqSmemBoys<LT>::use;
-  extern __shared__ double s_boys[];
-  if constexpr (SBOYS) {
-    boys_stage<LT>(lq.boys, s_boys);
-    __syncthreads();
-  }
   // the warp takes the next chunk of this rank's share (every numprocs-th,
   // starting at myid) from the pass's work queue: chunks are sorted costliest
   // first, so the launch ends with the cheap ones
@@ -420,7 +400,6 @@ __global__ void __launch_bounds__(128, GqOccupancy<LA, LB, LC, LD>::blocks) k_gq
         n32 += f32 ? 1u : 0u;
         double F[LT + 1];
         if constexpr (LT <= GqBoysDirect::maxl) boys_direct<LT>(T, f32 ? 1.0 : pref, F);
-        else if constexpr (SBOYS) boys_tab_smem<LT>(T, f32 ? 1.0 : pref, s_boys, F);
         else boys_tab<LT>(T, f32 ? 1.0 : pref, boys, F);
         double out[NI];
         if constexpr (LT == 0) {
@@ -513,43 +492,64 @@ void launch_digest(int cb, int ck, const MolLaunch& ql, int num_sms, cudaStream_
 
 // ------------------------------------------------------------------ launch tables
 
+// Register passes per kernel: the live ones of a group run side by side in one launch
+// (blockIdx.y), so that their tails overlap and a small molecule's build is not
+// launch-bound.
+constexpr int kPassGroup = 8;
+
+template <int LA, int LB, int LC, int LD, int NPASS, int P0, int PN, bool MIXED, bool BATCH>
+__device__ __forceinline__ void gq_select(const MolLaunch& lq, int p) {
+  if constexpr (PN == 1) {
+    gq_pass<LA, LB, LC, LD, NPASS, P0, MIXED, BATCH>(lq);
+  } else {
+    if (p == P0) gq_pass<LA, LB, LC, LD, NPASS, P0, MIXED, BATCH>(lq);
+    else gq_select<LA, LB, LC, LD, NPASS, P0 + 1, PN - 1, MIXED, BATCH>(lq, p);
+  }
+}
+
+// Passes P0 .. P0 + PN - 1; blockIdx.y is the position among the live ones (bits of live).
+template <int LA, int LB, int LC, int LD, int NPASS, int P0, int PN, bool MIXED, bool BATCH>
+__global__ void __launch_bounds__(128, GqOccupancy<LA, LB, LC, LD>::blocks)
+    k_gq(const __grid_constant__ MolLaunch lq, unsigned int live) {
+  unsigned int m = live;
+  for (int y = blockIdx.y; y > 0; --y) m &= m - 1;
+  gq_select<LA, LB, LC, LD, NPASS, P0, PN, MIXED, BATCH>(lq, P0 + __ffs(m) - 1);
+}
+
 using LaunchFn = void (*)(const MolLaunch&, int grid, cudaStream_t);
 
-template <int LA, int LB, int LC, int LD, int NPASS, int PASS, bool MIXED, bool BATCH>
-struct Passes {
-  static void run(const MolLaunch& ql, int grid, cudaStream_t s) {
-    if (NPASS > 1 && !pass_live(LA, LB, LC, LD, NPASS, PASS, ql.lower_kept_bits)) {
-      if constexpr (PASS + 1 < NPASS) Passes<LA, LB, LC, LD, NPASS, PASS + 1, MIXED, BATCH>::run(ql, grid, s);
-      return;
+template <int LA, int LB, int LC, int LD, int NPASS, int P0, bool MIXED, bool BATCH>
+void launch_groups(const MolLaunch& ql, int grid, cudaStream_t s) {
+  constexpr int PN = NPASS - P0 < kPassGroup ? NPASS - P0 : kPassGroup;
+  unsigned int live = 0;
+  int n = 0;
+  for (int p = 0; p < PN; ++p)
+    if (NPASS == 1 || pass_live(LA, LB, LC, LD, NPASS, P0 + p, ql.lower_kept_bits)) {
+      live |= 1u << p;
+      ++n;
     }
-    constexpr int LT = LA + LB + LC + LD;
-    auto kern = k_gq<LA, LB, LC, LD, NPASS, PASS, MIXED, BATCH>;
-    if constexpr (GqSmemBoys<LT>::use) {
-      // the staged Boys rows: allow them once, and launch no more blocks than can be
-      // resident (each block copies the rows once; the work queue spreads the chunks)
-      static int resident = 0;
-      if (resident == 0) {
-        cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)BoysSmem<LT>::BYTES);
-        int per_sm = 0, dev = 0, nsm = 0;
-        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, 128, BoysSmem<LT>::BYTES);
-        cudaGetDevice(&dev);
-        cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev);
-        resident = std::max(1, per_sm) * std::max(1, nsm);
-      }
-      kern<<<std::min(grid, resident), 128, BoysSmem<LT>::BYTES, s>>>(ql);
-    } else {
-      kern<<<grid, 128, 0, s>>>(ql);
-    }
-    if constexpr (PASS + 1 < NPASS) Passes<LA, LB, LC, LD, NPASS, PASS + 1, MIXED, BATCH>::run(ql, grid, s);
-  }
-};
+  if (n > 0) k_gq<LA, LB, LC, LD, NPASS, P0, PN, MIXED, BATCH><<<dim3(grid, n), 128, 0, s>>>(ql, live);
+  if constexpr (P0 + PN < NPASS) launch_groups<LA, LB, LC, LD, NPASS, P0 + PN, MIXED, BATCH>(ql, grid, s);
+}
 
 template <int LA, int LB, int LC, int LD, int NPASS, bool MIXED, bool BATCH = false>
 void launch_q(const MolLaunch& ql, int grid, cudaStream_t s) {
-  Passes<LA, LB, LC, LD, NPASS, 0, MIXED, BATCH>::run(ql, grid, s);
+  launch_groups<LA, LB, LC, LD, NPASS, 0, MIXED, BATCH>(ql, grid, s);
 }
 
-// Launches per straight-line class (its passes); must match the table below.
+// Kernels launch_q launches for a class (groups with a live pass).
+inline int pass_groups_live(int LA, int LB, int LC, int LD, int npass, int lower_kept_bits) {
+  int n = 0;
+  for (int p0 = 0; p0 < npass; p0 += kPassGroup) {
+    bool any = false;
+    for (int p = p0; p < npass && p < p0 + kPassGroup; ++p)
+      any = any || npass == 1 || pass_live(LA, LB, LC, LD, npass, p, lower_kept_bits);
+    n += any ? 1 : 0;
+  }
+  return n;
+}
+
+// Register passes per straight-line class; must match the table below.
 static inline int straight_npass(int cb, int ck) {
   static const int np[6][6] = {{1, 0, 0, 0, 0, 0}, {1, 1, 0, 0, 0, 0}, {1, 2, 8, 0, 0, 0},
                                {2, 2, 5, 3, 0, 0}, {1, 4, 14, 10, 40, 0}, {3, 10, 50, 25, 0, 0}};
