@@ -104,6 +104,7 @@ struct ClassLaunch {
   size_t smem_wide;
   int* queue;                // device work queue: one chunk counter per launch (pass), zeroed before each
   int npass;                 // register passes of the straight-line variant
+  unsigned long long live;   // of which some component has a coefficient (live_passes)
   int launches_live;         // its kernel launches: pass groups with a component that has a coefficient, digestion
   int gmul = 32;             // straight-line variant: persistent grid of up to gmul blocks per SM
 };
@@ -130,7 +131,7 @@ struct pfe_context {
   cudaStream_t stream = nullptr;
   // class launches beside those on the caller's stream (launch_classes), forked
   // and joined with the events; made at set-up (ensure_side)
-  static constexpr int kSide = 5;
+  static constexpr int kSide = 7;
   cudaStream_t side[kSide] = {};
   cudaEvent_t ev_fork = nullptr, ev_join[kSide] = {};
   bool concurrent = false;   // every class has a buffer of its own for its stored integrals

@@ -916,12 +916,14 @@ static int lower_kept_bits(const pfe_context* ctx) {
   return bits;
 }
 
-// Kernel launches of a class's straight-line variant: its pass groups that are live
-// with these lower_kept bits, and the digestion of the stored integrals.
-static int class_launches(const ClassLaunch& cl, int bits) {
-  if (!cl.has_straight) return 1;
-  return pass_groups_live(kCL[cl.cb][0], kCL[cl.cb][1], kCL[cl.ck][0], kCL[cl.ck][1], cl.npass, bits) +
-         (cl.cb > 0 ? 1 : 0);
+// The live register passes of a class for these lower_kept bits, and its kernel
+// launches: the pass groups that have one and the digestion of the stored integrals.
+static void set_passes(ClassLaunch& cl, int bits) {
+  cl.launches_live = 1;
+  cl.live = 0;
+  if (!cl.has_straight) return;
+  cl.live = live_passes(kCL[cl.cb][0], kCL[cl.cb][1], kCL[cl.ck][0], kCL[cl.ck][1], cl.npass, bits);
+  cl.launches_live = pass_groups(cl.npass, cl.live) + (cl.cb > 0 ? 1 : 0);
 }
 
 static int size_wide(ClassLaunch& cl, const int kept_max[3], const bool lower_kept[3]) {
@@ -979,14 +981,14 @@ static GroupView group_view(const pfe_context* ctx) {
 // thousands where both groups are products of long contractions), so in a small
 // molecule, whose classes have fewer chunks than the GPU has warps, a launch lasts
 // as long as its longest lane.  The aim is a quarter of what each of the resident warps gets
-// on average, but no less than kLeastSteps: a piece pays its own set-up and
-// digestion (about two microseconds).  Ranks of one build must cut alike, so the
-// rule reads the work alone, not the device.
-static unsigned int longest_piece(double steps) {
+// on average, but no less than 12 steps, whose time is that of a piece's own set-up and
+// digestion; in the interpreter classes, where one quartet takes tens of microseconds,
+// two.  Ranks of one build must cut alike, so the rule reads the work alone, not the
+// device.
+static unsigned int longest_piece(double steps, bool serial) {
   constexpr double kWarps = 148.0 * 8.0;   // resident warps of the 255-register kernels on a B200
-  constexpr unsigned int kLeastSteps = 24;
   const double share = steps / (4.0 * kWarps);
-  return (unsigned int)std::min(4.0e9, std::max((double)kLeastSteps, share));
+  return (unsigned int)std::min(4.0e9, std::max(serial ? 2.0 : 12.0, share));
 }
 
 static PanelView panel_view(const pfe_context* c) {
@@ -1103,7 +1105,7 @@ static int finish_chunks(Owner* own, pfe_context* const* inst, int ninst, ClassL
   if (nraw >= (1LL << 31)) { set_error("too many chunks"); return PFE_EINVAL; }
   for (int cb = 0; cb < 6; ++cb)
     for (int ck = 0; ck <= cb; ++ck) {
-      pm.most[pair_code(cb, ck)] = longest_piece(steps[pair_code(cb, ck)]);
+      pm.most[pair_code(cb, ck)] = longest_piece(steps[pair_code(cb, ck)], !straight_launcher(cb, ck));
       if (!straight_launcher(cb, ck)) pm.serial |= 1u << pair_code(cb, ck);
     }
   PairStat stat[kClassPairs] = {};
@@ -1386,7 +1388,7 @@ int molecular_setup(pfe_context* ctx, const pfe_args* a) {
       cl.quartets = nq;
       cl.has_straight = straight_launcher(cb, ck) != nullptr;
       cl.npass = cl.has_straight ? straight_npass(cb, ck) : 0;
-      cl.launches_live = class_launches(cl, lower_kept_bits(ctx));
+      set_passes(cl, lower_kept_bits(ctx));
       cl.has_table = false;
       cl.variant = 0;
       cl.xg = nullptr;
@@ -1520,6 +1522,7 @@ static void launch_class(pfe_context* ctx, const ClassLaunch& cl, MolLaunch ql, 
   ql.chunks = cl.chunks;
   ql.nchunks = cl.d_nchunks;
   ql.queue = cl.queue;
+  ql.live = cl.live;
   const int work = (cl.nchunks_host + ctx->numprocs - 1) / ctx->numprocs;
   if ((variant == 0 && cl.has_straight) || !cl.has_table) {
     // (00|00) digests in its kernel; the other classes store X tile by tile
@@ -1700,18 +1703,24 @@ static int launch_classes(pfe_context* cx, const ClassLaunch* launches, int nlau
   int order[64];
   double load[pfe_context::kSide + 1] = {0.0};
   bool used[pfe_context::kSide + 1] = {false};
-  auto work = [&](int i) { return launches[i].quartets * class_flops(launches[i].cb, launches[i].ck); };
+  auto straight = [&](int i) { return (launches[i].variant == 0 && launches[i].has_straight) || !launches[i].has_table; };
+  // the interpreters run at about a fifth of the straight-line classes' rate
+  auto work = [&](int i) {
+    return launches[i].quartets * class_flops(launches[i].cb, launches[i].ck) * (straight(i) ? 1.0 : 5.0);
+  };
   for (int i = 0; i < nlaunch; ++i) order[i] = i;
   const bool fork = !serial && cx->ev_fork != nullptr;
-  if (fork && together) std::sort(order, order + nlaunch, [&](int a, int b) { return work(a) > work(b); });
+  if (fork && together)   // the interpreter classes first: their longest pieces take longest
+    std::sort(order, order + nlaunch, [&](int a, int b) {
+      return straight(a) != straight(b) ? !straight(a) : work(a) > work(b);
+    });
   for (int j = 0; j < nlaunch; ++j) {
-    const ClassLaunch& cl = launches[order[j]];
     int k = 0;
     if (fork && together) {
       for (int x = 1; x <= pfe_context::kSide; ++x)
         if (load[x] < load[k]) k = x;
       load[k] += work(order[j]);
-    } else if (fork && !ql.insts && !((cl.variant == 0 && cl.has_straight) || !cl.has_table)) {
+    } else if (fork && !ql.insts && !straight(order[j])) {
       k = 1;
     }
     used[k] = true;
@@ -1849,7 +1858,7 @@ int batch_setup(pfe_batch* b) {
       {  // launched passes over the whole batch: a pass is skipped only if no instance needs it
         int bits = 0;
         for (pfe_context* c : b->inst) bits |= lower_kept_bits(c);
-        cl.launches_live = class_launches(cl, bits);
+        set_passes(cl, bits);
       }
       if (cl.has_wide) {   // the wide variant's working set must cover every instance
         int km[3] = {1, 1, 1};

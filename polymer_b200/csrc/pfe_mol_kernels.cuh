@@ -87,6 +87,7 @@ struct MolLaunch {
   // one tile of a straight-line class: tickets [t0, t0 + tn) of this rank's chunks; X of
   // ticket t0 + t at xbuf + t * (kept integrals) * 32, xlive[t] set when it holds any quartet
   int t0, tn;
+  unsigned long long live;   // register passes launched (live_passes)
   double* xbuf;
   unsigned char* xlive;
 };
@@ -237,23 +238,26 @@ __host__ __device__ constexpr void pass_range(int LA, int LB, int LC, int LD, in
   ab1 = lsplit ? (pass == 0 ? nlow : NAB) : ((ab0 + abp < NAB) ? ab0 + abp : NAB);
 }
 
-// Whether register pass `pass` keeps a bra component pair that can carry a
-// coefficient: a component below its shell's top level has none unless bit L of
-// lower_kept_bits is set (the kernel skips such chunks anyway; a pass that keeps
-// none of them is not launched at all).
-inline bool pass_live(int LA, int LB, int LC, int LD, int npass, int pass, int lower_kept_bits) {
+// The register passes of a class that keep a bra component pair that can carry a
+// coefficient (bit p of the mask): a component below its shell's top level has none
+// unless bit L of lower_kept_bits is set (the kernel skips such chunks anyway; a pass
+// that keeps none of them is not launched at all).
+inline unsigned long long live_passes(int LA, int LB, int LC, int LD, int npass, int lower_kept_bits) {
   int ab[MAXCOMP * MAXCOMP] = {}, pos[MAXCOMP * MAXCOMP] = {};
   ab_order_fill(LA, LB, ab, pos);
-  int ab0 = 0, ab1 = 0;
-  pass_range(LA, LB, LC, LD, npass, pass, ab0, ab1);
   const int NB = ncum(LB);
-  for (int k = ab0; k < ab1; ++k) {
-    const int a = ab[k] / NB, b = ab[k] % NB;
-    const bool ka = comp_tot(LA, a) == LA || ((lower_kept_bits >> LA) & 1);
-    const bool kb = comp_tot(LB, b) == LB || ((lower_kept_bits >> LB) & 1);
-    if (ka && kb) return true;
+  unsigned long long live = 0;
+  for (int p = 0; p < npass; ++p) {
+    int ab0 = 0, ab1 = 0;
+    pass_range(LA, LB, LC, LD, npass, p, ab0, ab1);
+    for (int k = ab0; k < ab1; ++k) {
+      const int a = ab[k] / NB, b = ab[k] % NB;
+      const bool ka = comp_tot(LA, a) == LA || ((lower_kept_bits >> LA) & 1);
+      const bool kb = comp_tot(LB, b) == LB || ((lower_kept_bits >> LB) & 1);
+      if (ka && kb) live |= 1ull << p;
+    }
   }
-  return false;
+  return npass == 1 ? 1ull : live;
 }
 
 // resident blocks of 128 threads the register allocation aims at: 4 (at most
@@ -519,33 +523,23 @@ __global__ void __launch_bounds__(128, GqOccupancy<LA, LB, LC, LD>::blocks)
 using LaunchFn = void (*)(const MolLaunch&, int grid, cudaStream_t);
 
 template <int LA, int LB, int LC, int LD, int NPASS, int P0, bool MIXED, bool BATCH>
-void launch_groups(const MolLaunch& ql, int grid, cudaStream_t s) {
+void launch_groups(const MolLaunch& ql, unsigned long long live, int grid, cudaStream_t s) {
   constexpr int PN = NPASS - P0 < kPassGroup ? NPASS - P0 : kPassGroup;
-  unsigned int live = 0;
-  int n = 0;
-  for (int p = 0; p < PN; ++p)
-    if (NPASS == 1 || pass_live(LA, LB, LC, LD, NPASS, P0 + p, ql.lower_kept_bits)) {
-      live |= 1u << p;
-      ++n;
-    }
-  if (n > 0) k_gq<LA, LB, LC, LD, NPASS, P0, PN, MIXED, BATCH><<<dim3(grid, n), 128, 0, s>>>(ql, live);
-  if constexpr (P0 + PN < NPASS) launch_groups<LA, LB, LC, LD, NPASS, P0 + PN, MIXED, BATCH>(ql, grid, s);
+  const unsigned int m = (unsigned int)(live >> P0) & ((1u << PN) - 1);
+  if (m) k_gq<LA, LB, LC, LD, NPASS, P0, PN, MIXED, BATCH><<<dim3(grid, __builtin_popcount(m)), 128, 0, s>>>(ql, m);
+  if constexpr (P0 + PN < NPASS) launch_groups<LA, LB, LC, LD, NPASS, P0 + PN, MIXED, BATCH>(ql, live, grid, s);
 }
 
 template <int LA, int LB, int LC, int LD, int NPASS, bool MIXED, bool BATCH = false>
 void launch_q(const MolLaunch& ql, int grid, cudaStream_t s) {
-  launch_groups<LA, LB, LC, LD, NPASS, 0, MIXED, BATCH>(ql, grid, s);
+  static_assert(NPASS <= 64, "a bit per pass");
+  launch_groups<LA, LB, LC, LD, NPASS, 0, MIXED, BATCH>(ql, ql.live, grid, s);
 }
 
 // Kernels launch_q launches for a class (groups with a live pass).
-inline int pass_groups_live(int LA, int LB, int LC, int LD, int npass, int lower_kept_bits) {
+inline int pass_groups(int npass, unsigned long long live) {
   int n = 0;
-  for (int p0 = 0; p0 < npass; p0 += kPassGroup) {
-    bool any = false;
-    for (int p = p0; p < npass && p < p0 + kPassGroup; ++p)
-      any = any || npass == 1 || pass_live(LA, LB, LC, LD, npass, p, lower_kept_bits);
-    n += any ? 1 : 0;
-  }
+  for (int p0 = 0; p0 < npass; p0 += kPassGroup) n += ((live >> p0) & ((1ull << kPassGroup) - 1)) ? 1 : 0;
   return n;
 }
 
