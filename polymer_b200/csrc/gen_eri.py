@@ -167,7 +167,7 @@ class Gen:
 OPS_THRESHOLD = 1600  # classes with more integrals have no straight-line function (op tables only)
 
 
-def gen_optable(LA, LB, LC, LD, pure_bra=False, pure_ket=False, compact=True):
+def gen_optable(LA, LB, LC, LD, pure_bra=False, pure_ket=False, compact=True, top_d=False):
     """Level-scheduled op table of one class for the block-cooperative interpreter.
 
     Slot 0 holds zero, slots 1..L+1 the Boys values F[m]; the recursion nodes
@@ -246,6 +246,11 @@ def gen_optable(LA, LB, LC, LD, pure_bra=False, pure_ket=False, compact=True):
         order.append(key)
         return key
 
+    def top(L, c):
+        # top_d: d shells keep their top-level components, s and p shells every one
+        # (the sp and pure d shells of 6-31G**, where no shell kind is pure throughout)
+        return not top_d or L < 2 or tot(c) == L
+
     def kept(a, b):
         # pure_bra: only the top-level components of the bra shells, for bra shells
         # whose lower components carry no coefficient (the d shells of 6-31G** and
@@ -256,7 +261,8 @@ def gen_optable(LA, LB, LC, LD, pure_bra=False, pure_ket=False, compact=True):
         # pure_ket: the same on the ket shells
         return not pure_ket or ((LC == 0 or tot(c) == LC) and (LD == 0 or tot(d) == LD))
 
-    outs = [hk(a, b, c, d) if kept(a, b) and kept_ket(c, d) else None
+    outs = [hk(a, b, c, d) if kept(a, b) and kept_ket(c, d) and top(LA, a) and top(LB, b) and top(LC, c) and top(LD, d)
+            else None
             for a in comps(LA) for b in comps(LB) for c in comps(LC) for d in comps(LD)]
     level = {}
     for k in order:   # 'order' is a valid topological order (post-order)
@@ -317,9 +323,10 @@ def pure_ket_gains(LA, LB, LC, LD):
             len(gen_optable(LA, LB, LC, LD, True, False)[0]))
 
 
-def emit_optable(LA, LB, LC, LD, pure_bra=False, pure_ket=False, name=None):
-    ops, lev, outs, nslots = gen_optable(LA, LB, LC, LD, pure_bra, pure_ket)
-    name = name or 'op_%d%d%d%d%s' % (LA, LB, LC, LD, '_pure2' if pure_ket else ('_pure' if pure_bra else ''))
+def emit_optable(LA, LB, LC, LD, pure_bra=False, pure_ket=False, name=None, top_d=False):
+    ops, lev, outs, nslots = gen_optable(LA, LB, LC, LD, pure_bra, pure_ket, top_d=top_d)
+    suffix = '_topd' if top_d else ('_pure2' if pure_ket else ('_pure' if pure_bra else ''))
+    name = name or 'op_%d%d%d%d%s' % (LA, LB, LC, LD, suffix)
     lines = ['// (%d%d|%d%d): %d ops in %d levels, %d slots' % (LA, LB, LC, LD, len(ops), len(lev) - 1, nslots)]
     flat = [v for op in ops for v in op] or [0] * 7
     lines.append('static const unsigned short %s_ops[%d] = {%s};' % (name, len(flat), ','.join(map(str, flat))))
@@ -458,6 +465,8 @@ def main():
             big.append(emit_optable(LA, LB, LC, LD))   # every class can run interpreted
             if LA >= 1:
                 big.append(emit_optable(LA, LB, LC, LD, pure_bra=True))
+            if LA == 2:
+                big.append(emit_optable(LA, LB, LC, LD, top_d=True))
             if LA >= 1 and LC >= 1 and pure_ket_gains(LA, LB, LC, LD):
                 big.append(emit_optable(LA, LB, LC, LD, pure_bra=True, pure_ket=True))
             if n > OPS_THRESHOLD:

@@ -339,6 +339,7 @@ struct OpTableDev;
 const struct OpTableHost* host_optable(int cb, int ck);
 const struct OpTableHost* host_optable_pure(int cb, int ck);
 const struct OpTableHost* host_optable_pure2(int cb, int ck);
+const struct OpTableHost* host_optable_topd(int cb, int ck);
 int upload_optable(pfe_context* ctx, const struct OpTableHost* h, OpTableDev* d);
 double class_flops(int cb, int ck);
 int lattice_setup(pfe_context* ctx, const pfe_args* a);

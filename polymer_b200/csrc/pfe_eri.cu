@@ -132,6 +132,28 @@ const OpTableHost* host_optable_pure2(int cb, int ck) {
   }
 }
 
+// The class's table with the top-level components of d shells only, all of s and p shells.
+const OpTableHost* host_optable_topd(int cb, int ck) {
+  switch (cb * 8 + ck) {
+    case 3 * 8 + 0: return &op_2000_topd;
+    case 3 * 8 + 1: return &op_2010_topd;
+    case 3 * 8 + 2: return &op_2011_topd;
+    case 3 * 8 + 3: return &op_2020_topd;
+    case 4 * 8 + 0: return &op_2100_topd;
+    case 4 * 8 + 1: return &op_2110_topd;
+    case 4 * 8 + 2: return &op_2111_topd;
+    case 4 * 8 + 3: return &op_2120_topd;
+    case 4 * 8 + 4: return &op_2121_topd;
+    case 5 * 8 + 0: return &op_2200_topd;
+    case 5 * 8 + 1: return &op_2210_topd;
+    case 5 * 8 + 2: return &op_2211_topd;
+    case 5 * 8 + 3: return &op_2220_topd;
+    case 5 * 8 + 4: return &op_2221_topd;
+    case 5 * 8 + 5: return &op_2222_topd;
+    default: return nullptr;
+  }
+}
+
 // The op tables are immutable: each is uploaded once per device and shared by
 // every context on it (a batch holds hundreds of contexts).  The copies live as
 // long as the process.

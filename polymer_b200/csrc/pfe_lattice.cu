@@ -42,6 +42,9 @@ struct LatticeLaunch {
   int* d_nchunks;
   int4* chunks;          // (bra pair, first ket, end ket, ticket)
   OpTableDev tab;        // of the evaluated class (max(cb,ck) | min(cb,ck))
+  OpTableDev tab_top;    // its table with the d shells' top level only
+  LatWideFn wide;        // kernel of that table, or null
+  int nx;                // kept integrals of its largest quartet
   int per_warp, wpb;
   size_t smem;
   double quartets;
@@ -62,6 +65,7 @@ struct LatticeState {
   LatticeLaunch launches[36];
   int nlaunch = 0;
   int* d_queue = nullptr;      // kLatQueueSlots chunk counters per launch (straight-line kernels, per pass)
+  int* d_ghost = nullptr;      // whether the last densities had a non-zero ghost element
   bool interpret_only = false; // every class on the op-table interpreter (tests)
   double quartets = 0.0, flops = 0.0;
 };
@@ -223,6 +227,7 @@ __global__ void __launch_bounds__(256) k_lattice(LatticeRun R, OpTableDev tab, i
   __shared__ OpGeom s_geo[8];
   __shared__ OpGeomF s_geof[8];
   __shared__ int s_prm[8][N1 + N2 + M1 + M2];
+  if (R.ghost && *R.ghost == 0) return;   // k_lat_wide does the class
   const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5, wpb = blockDim.x >> 5;
   double* v = smem + (size_t)wid * per_warp;
   double* DJ = v + tab.nslots;      // D(k,l), [c][d] over ket canonical comps
@@ -725,6 +730,15 @@ int lattice_setup(pfe_context* ctx, const pfe_args* a) {
       const OpTableHost* h = host_optable(e1, e2);
       if ((rc = upload_optable(ctx, h, &ll.tab)) != PFE_OK) return rc;
       static const int Lc[6][2] = {{0, 0}, {1, 0}, {1, 1}, {2, 0}, {2, 1}, {2, 2}};
+      ll.wide = nullptr;
+      if (const OpTableHost* ht = (ctx->lower_kept[2] || total >= (1 << 25)) ? nullptr : host_optable_topd(e1, e2)) {
+        ll.wide = lattice_wide_launcher(e1, e2, cb < ck);
+        if (ll.wide && (rc = upload_optable(ctx, ht, &ll.tab_top)) != PFE_OK) return rc;
+        ll.nx = 1;
+        for (int k = 0; k < 2; ++k)
+          ll.nx *= std::max(ctx->kept_max[Lc[e1][k]], 1) * std::max(ctx->kept_max[Lc[e2][k]], 1);
+        if (!L->d_ghost) PFE_CUDA(ctx->alloc((void**)&L->d_ghost, sizeof(int)));
+      }
       const int nbra = ncum(Lc[cb][0]) * ncum(Lc[cb][1]);
       const int nket = ncum(Lc[ck][0]) * ncum(Lc[ck][1]);
       const int maxc = std::max(ncum(Lc[ck][0]), ncum(Lc[ck][1]));
@@ -774,6 +788,22 @@ int lattice_fock(pfe_context* ctx, const double* d_pp, const double* d_pph, doub
   R.n32 = ctx->d_n32;
   PFE_CUDA(cudaMemsetAsync(ctx->d_n32, 0, sizeof(unsigned long long), s));
   PFE_CUDA(cudaMemsetAsync(L->d_queue, 0, sizeof(int) * 64 * kLatQueueSlots, s));
+  R.tidx = ctx->d_tidx;
+  // classes with pure d shells on their own kernels (FP64 in every cell), unless some
+  // ghost has a density; decided on the device
+  bool wide = false;
+  for (int i = 0; i < L->nlaunch; ++i) wide = wide || L->launches[i].wide != nullptr;
+  wide = wide && !L->interpret_only && !R.far32;
+  if (wide) {
+    PFE_CUDA(cudaMemsetAsync(L->d_ghost, 0, sizeof(int), s));
+    lattice_ghost_check(d_pp, (long long)pp, ctx->npgs, ctx->d_tidx, L->d_ghost, ctx->num_sms, s);
+    if (R.pph)
+      lattice_ghost_check(d_pph,
+                          (long long)ctx->npgs * ctx->npgs * (2 * ctx->cel2[0] + 1) *
+                              (2 * (ctx->cel2[0] + ctx->cel1[0]) + 1),
+                          ctx->npgs, ctx->d_tidx, L->d_ghost, ctx->num_sms, s);
+    PFE_CUDA(cudaGetLastError());
+  }
   for (int i = 0; i < L->nlaunch; ++i) {
     const LatticeLaunch& ll = L->launches[i];
     R.chunks = ll.chunks;
@@ -785,7 +815,14 @@ int lattice_fock(pfe_context* ctx, const double* d_pp, const double* d_pph, doub
       const int grid = std::min((ll.ncells_chunks + 3) / 4, ctx->num_sms * 16);
       f(R, std::max(grid, 1), s);
     } else {
-      int grid = std::min((ll.ncells_chunks + ll.wpb - 1) / ll.wpb, ctx->num_sms * 8);
+      R.ghost = nullptr;
+      if (wide && ll.wide) {
+        R.ghost = L->d_ghost;
+        const int rc = ll.wide(R, ll.tab_top, ll.nx, ll.ncells_chunks, ctx->num_sms, s);
+        if (rc != PFE_OK) return rc;
+      }
+      // (a block per SM where the launch is only the fallback of the above)
+      const int grid = std::min((ll.ncells_chunks + ll.wpb - 1) / ll.wpb, ctx->num_sms * (R.ghost ? 1 : 8));
       lat_variant(e1, e2, ll.cb < ll.ck).fn(R, ll.tab, std::max(grid, 1), ll.wpb, ll.per_warp, ll.smem, s);
     }
     PFE_CUDA(cudaGetLastError());

@@ -38,6 +38,10 @@ struct LatticeRun {
   int far32;
   unsigned long long* n32;
   int* queue;          // chunk counter of the straight-line kernels, zero at launch
+  const int* tidx;     // primitive -> contracted function (-1: a ghost)
+  // set where P_P or P_P_HELIX has a non-zero element of a ghost; null where the
+  // interpreter runs a class in any case
+  const int* ghost;
 };
 
 // The straight-line kernel of evaluated class (e1|e2) (e1 >= e2, swap: the
@@ -47,6 +51,13 @@ struct LatticeRun {
 constexpr int kLatQueueSlots = 4;
 using LatSlFn = void (*)(const LatticeRun&, int grid, cudaStream_t);
 LatSlFn lattice_sl_launcher(int e1, int e2, bool sw);
+// The warp-per-quartet kernel of a class with d shells for bases whose d shells are all
+// pure (pfe_lattice_wide.cu), on the class's top-level-d table; nx: kept integrals.
+struct OpTableDev;
+using LatWideFn = int (*)(const LatticeRun&, const OpTableDev&, int nx, int nchunks, int num_sms, cudaStream_t);
+LatWideFn lattice_wide_launcher(int e1, int e2, bool sw);
+void lattice_ghost_check(const double* p, long long n, int npgs, const int* tidx, int* flag, int num_sms,
+                         cudaStream_t s);
 // launches (register passes) of a straight-line class, 0 where the class has none
 int lattice_sl_passes(int e1, int e2);
 
