@@ -293,15 +293,8 @@ static int setup_impl(pfe_context* ctx, const pfe_args* a, const HostShells& hs,
     PFE_CUDA(cudaMemcpyAsync(ctx->d_sss, sss.data(), sizeof(double) * sss.size(), cudaMemcpyHostToDevice, s));
     PFE_CUDA(cudaStreamSynchronize(s));
   }
-  // Boys table, row-major [T][m]
-  {
-    std::vector<double> tab((size_t)NIG_T * NIG_M);
-    for (int t = 0; t < NIG_T; ++t)
-      for (int m = 0; m < NIG_M; ++m) tab[(size_t)t * NIG_M + m] = a->igamma[t + (size_t)NIG_T * m];
-    PFE_CUDA(ctx->alloc((void**)&ctx->d_boys, sizeof(double) * tab.size()));
-    PFE_CUDA(cudaMemcpyAsync(ctx->d_boys, tab.data(), sizeof(double) * tab.size(), cudaMemcpyHostToDevice, s));
-    PFE_CUDA(cudaStreamSynchronize(s));
-  }
+  if ((rc = acquire_boys(ctx->device, a->igamma, s, &ctx->boys)) != PFE_OK) return rc;
+  ctx->d_boys = ctx->boys->rows;
   // MAXC and CC
   {
     std::vector<double> maxc(a->npgs, 0.0);

@@ -107,50 +107,45 @@ __device__ __forceinline__ void boys_tab(double T, double pref, const double* __
   boys_eval<L>(T, pref, gv, F);
 }
 
-// Coefficients 1/(k! (2L+2k+1)), k = 0..17, of the Maclaurin series
-// F_L(T) = sum_k (-T)^k / (k! (2L+2k+1)); at T <= 1 the omitted terms are below 1e-17.
-template <int L>
-struct BoysSeries {
-  double c[18];
-  constexpr BoysSeries() : c() {
-    double f = 1.0;   // k!
-    for (int k = 0; k < 18; ++k) {
-      if (k > 0) f *= (double)k;
-      c[k] = 1.0 / (f * (double)(2 * L + 2 * k + 1));
-    }
-  }
-};
+// The table of boys_down: for every top order L = 0 .. kDownMax and every grid point
+// T0 = t/20 eight doubles (64 bytes, so a row is two sectors of one line):
+// F_{L+k}(T0)/k! for k = 0..6, and e^-T0.
+constexpr int kDownMax = 8;
+constexpr int kDownCols = 8;
+__host__ __device__ constexpr size_t down_row(int L, int t) { return ((size_t)L * NIG_T + t) * kDownCols; }
 
-// F_m(T)*pref for m = 0..L (L <= 2) without reading the table, for kernels whose
-// per-lane table-row gathers are what their L1 spends its wavefronts on:
-//  * T >= 1: F_0 = F1(0) erf(sqrt T)/sqrt T (F1(0) = sqrt(PI)/2, the constant of the
-//    asymptotic form) and upward recursion F_{m+1} = ((2m+1) F_m - e^-T)/(2T), whose
-//    error grows by at most (2m+1)/(2T) <= 3/2 per step here;
-//  * T < 1: the series above for F_L and downward recursion
-//    F_{m-1} = (2T F_m + e^-T)/(2m-1), which is stable.
-// The reference tabulates and Taylor-expands every order (boys_eval); the two agree to
-// the table's own accuracy (about 1e-14 relative), far inside the build's tolerance.
+// F_m(T)*pref for m = 0..L (L <= kDownMax): below TF(L) the top order alone from the
+// reference's 6-term series about the nearest grid point, e^-T from its tabulated value and
+// the series of e^(T0-T) (|T0-T| <= 0.025: 8 terms leave 4e-18), and the lower orders by
+// downward recursion F_m = (2T F_{m+1} + e^-T)/(2m+1), which is stable; above TF(L) the
+// asymptotic form of boys_eval.  Against boys_tab, which expands every order: four 16-byte
+// gathers per lane from rows of one line instead of up to eight from rows 224 bytes apart
+// (the part of the table that a class reads shrinks from 190 to 55 KB at L = 3, inside the
+// L1), and 15 + 2L multiply-adds instead of 7(L + 1).  The two agree to rounding.
 template <int L>
-__device__ __forceinline__ void boys_direct(double T, double pref, double* __restrict__ F) {
-  static_assert(L <= 2, "boys_direct: orders 0..2");
-  if (T >= 1.0) {
-    const double r = rsqrt(T);
-    F[0] = pref * PFE_F1_0 * erf(T * r) * r;
-    if (L >= 1) {
-      const double e = pref * exp(-T), h = 0.5 * r * r;
+__device__ __forceinline__ void boys_down(double T, double pref, const double* __restrict__ down,
+                                          double* __restrict__ F) {
+  static_assert(L <= kDownMax, "boys_down: orders 0..8");
+  if (T < c_TF[L]) {
+    const int ts = (int)floor(T * 20.0 + 0.5);   // NINT for T >= 0; <= 20 TF(L) < NIG_T
+    const double h = 0.05 * (double)ts - T;
+    const double2* r = reinterpret_cast<const double2*>(down + down_row(L, ts));
+    const double2 a = __ldg(r), b = __ldg(r + 1), c = __ldg(r + 2), d = __ldg(r + 3);
+    const double f = fma(fma(fma(fma(fma(fma(d.x, h, c.y), h, c.x), h, b.y), h, b.x), h, a.y), h, a.x);
+    const double x = fma(fma(fma(fma(fma(fma(fma(1.0 / 5040.0, h, 1.0 / 720.0), h, 1.0 / 120.0), h, 1.0 / 24.0), h,
+                                     1.0 / 6.0), h, 0.5), h, 1.0), h, 1.0);
+    const double e = pref * d.y * x, t2 = T + T;
+    F[L] = pref * f;
 #pragma unroll
-      for (int m = 0; m < L; ++m) F[m + 1] = ((double)(2 * m + 1) * F[m] - e) * h;
-    }
+    for (int m = L - 1; m >= 0; --m) F[m] = fma(t2, F[m + 1], e) * (1.0 / (double)(2 * m + 1));
   } else {
-    constexpr BoysSeries<L> S{};
-    double v = S.c[17];
+    const double it = 1.0 / T;
+    double v = pref * PFE_F1_0 * rsqrt(T);
+    F[0] = v;
 #pragma unroll
-    for (int k = 16; k >= 0; --k) v = fma(v, -T, S.c[k]);
-    F[L] = pref * v;
-    if (L >= 1) {
-      const double e = pref * exp(-T);
-#pragma unroll
-      for (int m = L; m > 0; --m) F[m - 1] = (2.0 * T * F[m] + e) * (1.0 / (double)(2 * m - 1));
+    for (int m = 1; m <= L; ++m) {
+      v *= it * (0.5 * (double)(2 * m - 1));
+      F[m] = v;
     }
   }
 }

@@ -7,6 +7,7 @@
 #include <cuda_runtime.h>
 
 #include <cstdint>
+#include <memory>
 #include <vector>
 
 #include "pfe_common.cuh"
@@ -26,6 +27,20 @@ inline cudaError_t injected_alloc_failure() {
   return cudaSuccess;
 }
 
+
+// The Boys tables of one IGAMMA on one device, shared by every context set up with the
+// same values (a batch holds hundreds) and freed with the last of them.
+struct BoysTables {
+  int device = 0;
+  std::vector<double> igamma;   // as given, column-major
+  double* rows = nullptr;       // [T][m]
+  double* down = nullptr;       // the table of boys_down
+  ~BoysTables() {
+    cudaFree(rows);
+    cudaFree(down);
+  }
+};
+int acquire_boys(int device, const double* igamma, cudaStream_t s, std::shared_ptr<BoysTables>* out);
 
 // Primitive-shell table, struct of arrays (n shells).
 struct DevShells {
@@ -151,7 +166,8 @@ struct pfe_context {
   // device data
   pfe::DevShells shells{};
   double* d_sss = nullptr;   // S_P(head I, head J, cell) for shell heads, [cell][J][I]
-  double* d_boys = nullptr;
+  std::shared_ptr<pfe::BoysTables> boys;
+  double* d_boys = nullptr;  // boys->rows
   double* d_maxc = nullptr;  // max_i |CC(i, p)| per primitive
   double* d_cc = nullptr;    // CC (ncgs x npgs, column-major)
   double* d_c2h = nullptr;

@@ -154,6 +154,62 @@ const OpTableHost* host_optable_topd(int cb, int ck) {
   }
 }
 
+// IGAMMA column-major [m][T] -> rows [T][m] and the rows of boys_down.
+__global__ void k_boys_tables(const double* __restrict__ ig, double* __restrict__ rows, double* __restrict__ down) {
+  const int t = blockIdx.x * blockDim.x + threadIdx.x;
+  if (t >= NIG_T) return;
+  for (int m = 0; m < NIG_M; ++m) rows[(size_t)t * NIG_M + m] = ig[t + (size_t)NIG_T * m];
+  const double e = exp(-0.05 * (double)t);
+  for (int L = 0; L <= kDownMax; ++L) {
+    double* r = down + down_row(L, t);
+    double f = 1.0;
+    for (int k = 0; k < kDownCols - 1; ++k) {
+      if (k > 0) f *= (double)k;
+      r[k] = ig[t + (size_t)NIG_T * (L + k)] / f;
+    }
+    r[kDownCols - 1] = e;
+  }
+}
+
+static std::mutex g_boys_mu;
+static std::vector<std::weak_ptr<BoysTables>> g_boys;
+
+int acquire_boys(int device, const double* igamma, cudaStream_t s, std::shared_ptr<BoysTables>* out) {
+  constexpr size_t n = (size_t)NIG_T * NIG_M;
+  std::lock_guard<std::mutex> lock(g_boys_mu);
+  for (size_t i = 0; i < g_boys.size();) {
+    std::shared_ptr<BoysTables> b = g_boys[i].lock();
+    if (!b) {
+      g_boys.erase(g_boys.begin() + i);
+      continue;
+    }
+    if (b->device == device && memcmp(b->igamma.data(), igamma, sizeof(double) * n) == 0) {
+      *out = b;
+      return PFE_OK;
+    }
+    ++i;
+  }
+  auto b = std::make_shared<BoysTables>();
+  b->device = device;
+  b->igamma.assign(igamma, igamma + n);
+  double* raw = nullptr;
+  struct Guard {
+    double*& p;
+    ~Guard() { cudaFree(p); }
+  } guard{raw};
+  if (cudaError_t f = injected_alloc_failure()) PFE_CUDA(f);
+  PFE_CUDA(cudaMalloc((void**)&raw, sizeof(double) * n));
+  PFE_CUDA(cudaMalloc((void**)&b->rows, sizeof(double) * n));
+  PFE_CUDA(cudaMalloc((void**)&b->down, sizeof(double) * down_row(kDownMax + 1, 0)));
+  PFE_CUDA(cudaMemcpyAsync(raw, b->igamma.data(), sizeof(double) * n, cudaMemcpyHostToDevice, s));
+  k_boys_tables<<<(NIG_T + 127) / 128, 128, 0, s>>>(raw, b->rows, b->down);
+  PFE_CUDA(cudaGetLastError());
+  PFE_CUDA(cudaStreamSynchronize(s));
+  g_boys.push_back(b);
+  *out = b;
+  return PFE_OK;
+}
+
 // The op tables are immutable: each is uploaded once per device and shared by
 // every context on it (a batch holds hundreds of contexts).  The copies live as
 // long as the process.

@@ -776,6 +776,7 @@ int lattice_fock(pfe_context* ctx, const double* d_pp, const double* d_pph, doub
   R.swp = L->swp;
   R.prim = ctx->shells.prim;
   R.boys = ctx->d_boys;
+  R.down = ctx->boys->down;
   R.pp = d_pp;
   R.pph = ctx->helix != 0.0 ? d_pph : nullptr;
   R.cp = ctx->d_jp;

@@ -22,7 +22,8 @@ struct LatticeRun {
   PairArrays pairs;
   const unsigned char* swp;
   const int* prim;
-  const double* boys;
+  const double* boys;  // table rows (boys_tab)
+  const double* down;  // the table of boys_down
   const double* pp;    // P_P (npgs,npgs,cells1)
   const double* pph;   // P_P_HELIX or null
   double* cp;          // C_P (npgs,npgs,cells1)

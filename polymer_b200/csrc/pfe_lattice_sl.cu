@@ -190,7 +190,7 @@ __global__ void __launch_bounds__(128) k_lat_sl(LatticeRun R) {
       const double dx = Pb[0] - Q[0], dy = Pb[1] - Q[1], dz = Pb[2] - Q[2];
       const double T = rho * (dx * dx + dy * dy + dz * dz);
       double F[LT + 1];
-      boys_tab<LT>(T, f32 ? 1.0 : pref, R.boys, F);
+      boys_down<LT>(T, f32 ? 1.0 : pref, R.down, F);
       double out[NI];
       if constexpr (LT == 0) {
         out[0] = F[0];

@@ -135,7 +135,7 @@ __global__ void __launch_bounds__(128) k_lat_wide(LatticeRun R, OpTableDev tab, 
       const double T = rho * ((Pb[0] - Q[0]) * (Pb[0] - Q[0]) + (Pb[1] - Q[1]) * (Pb[1] - Q[1]) +
                               (Pb[2] - Q[2]) * (Pb[2] - Q[2]));
       double F[LT + 1];
-      boys_tab<LT>(T, pref, R.boys, F);
+      boys_down<LT>(T, pref, R.down, F);
       __syncwarp();   // the previous cell's digestion has read the slots and blocks
 #pragma unroll
       for (int m = 0; m <= LT; ++m)

@@ -1488,6 +1488,7 @@ static MolLaunch make_launch(pfe_context* ctx, const double* d_dt) {
   ql.stidx = ctx->d_stidx;
   ql.scoef = ctx->d_scoef;
   ql.boys = ctx->d_boys;
+  ql.down = ctx->boys->down;
   ql.dt = d_dt;
   ql.jt = ctx->d_jp;
   ql.kt = ctx->d_kp;

@@ -53,7 +53,8 @@ struct MolLaunch {
   const int* prim;        // shell components -> primitive
   const int* stidx;       // shell x component -> target row (-1: none)
   const double* scoef;    // shell x component -> coefficient
-  const double* boys;
+  const double* boys;     // table rows (boys_tab)
+  const double* down;     // the table of boys_down
   const double* dt;       // density in target space (nt x nt, column-major)
   double* jt;             // J' targets (nt x nt)
   double* kt;             // K' targets
@@ -260,31 +261,17 @@ inline unsigned long long live_passes(int LA, int LB, int LC, int LD, int npass,
   return npass == 1 ? 1ull : live;
 }
 
-// resident blocks of 128 threads the register allocation aims at: 4 (at most
-// 128 registers) for the classes whose working set fits, else the compiler's choice
+// Resident blocks of 128 threads the register allocation aims at.  The kernels wait on
+// loads more than on the FP64 pipe, so a block more is worth some spilling as long as the
+// recursion's temporaries are few: measured per class on C20H42 and the water batch,
+// (11|10) 2.89 -> 2.45 ms, (20|10) 1.03 -> 0.87, (11|11) 2.11 -> 1.93 and (21|00) 0.48 -> 0.44
+// at three blocks (168 registers) against two; four cost (11|10) and (21|10) 15 %.  Above a
+// total of 4 the 255 registers of two blocks are better ((21|11), (21|20), (22|11): 5-10 %).
+// (10|00) gains 5 % at five blocks, (10|10) and (11|00) lose 10-20 % there.
 template <int LA, int LB, int LC, int LD>
 struct GqOccupancy {
-  static constexpr int NI = ncum(LA) * ncum(LB) * ncum(LC) * ncum(LD);
-#ifdef PFE_GQ_MINB
-  static constexpr int blocks = (NI <= 16 && LA + LB + LC + LD <= 2) ? 4 : PFE_GQ_MINB;
-#else
-  static constexpr int blocks = (NI <= 16 && LA + LB + LC + LD <= 2) ? 4 : 1;
-#endif
-};
-
-// Classes of total angular momentum up to maxl evaluate the Boys function without
-// the table (boys_direct): their lanes' per-quartet table-row gathers were half of
-// their L1 wavefronts.  Measured on the 32-cluster water batch: (10|00) 55.8 ->
-// 53.0 ms (long-scoreboard stalls halved, instructions +60 % for erf and exp), the
-// batched build 295.8 -> 287.5 ms; C20H42 unchanged.  The lattice kernels keep the
-// table (their classes ran 12 % slower on it: they already spend the FP64 pipe on
-// the screw rotations of every image cell).
-struct GqBoysDirect {
-#ifdef PFE_BOYS_DIRECT_MAXL
-  static constexpr int maxl = PFE_BOYS_DIRECT_MAXL;
-#else
-  static constexpr int maxl = 2;
-#endif
+  static constexpr int NI = ncum(LA) * ncum(LB) * ncum(LC) * ncum(LD), LT = LA + LB + LC + LD;
+  static constexpr int blocks = LT <= 1 ? 5 : ((NI <= 16 && LT == 2) ? 4 : (LT <= 4 ? 3 : 1));
 };
 
 template <int LA, int LB, int LC, int LD, int NPASS, int PASS, bool MIXED, bool BATCH>
@@ -321,7 +308,7 @@ __device__ __forceinline__ void gq_pass(const MolLaunch& lq) {
     // the tables the loops read, held in registers (ql may live in global memory)
     const PairRec* __restrict__ rec = ql.rec;
     const double* __restrict__ scoef = ql.scoef;
-    const double* __restrict__ boys = ql.boys;
+    const double* __restrict__ down = ql.down;
     const int* __restrict__ stidx = ql.stidx;
     const double mcut = ql.mcut;
     const int nt = ql.nt;
@@ -403,8 +390,7 @@ __device__ __forceinline__ void gq_pass(const MolLaunch& lq) {
         if constexpr (MIXED && LT > 0) f32 = __all_sync(__activemask(), sp * sq * pmax < mcut);
         n32 += f32 ? 1u : 0u;
         double F[LT + 1];
-        if constexpr (LT <= GqBoysDirect::maxl) boys_direct<LT>(T, f32 ? 1.0 : pref, F);
-        else boys_tab<LT>(T, f32 ? 1.0 : pref, boys, F);
+        boys_down<LT>(T, f32 ? 1.0 : pref, down, F);
         double out[NI];
         if constexpr (LT == 0) {
           out[0] = F[0];

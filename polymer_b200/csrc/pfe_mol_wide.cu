@@ -102,7 +102,7 @@ __global__ void __launch_bounds__(256) k_gq_wide(MolLaunch lq, OpTableDev tab, i
     const MolLaunch& ql = lq.insts ? lq.insts[ch.inst] : lq;
     const PairRec* __restrict__ rec = ql.rec;
     const double* __restrict__ scoef = ql.scoef;
-    const double* __restrict__ boys = ql.boys;
+    const double* __restrict__ down = ql.down;
     const double* __restrict__ D = ql.dt;
     const int nt = ql.nt;
     const int G = ch.G;
@@ -184,7 +184,7 @@ __global__ void __launch_bounds__(256) k_gq_wide(MolLaunch lq, OpTableDev tab, i
           const double T = rho * (dx * dx + dy * dy + dz * dz);
           const double pref = c2pi * bp.S * kq.S * sqrt(rho);
           double F[LT + 1];
-          boys_tab<LT>(T, pref, boys, F);
+          boys_down<LT>(T, pref, down, F);
           const double w = ((I != J) ? 2.0 : 1.0) * ((K != L) ? 2.0 : 1.0) * ((p != q) ? 2.0 : 1.0);
           __syncwarp();   // the previous quartet's ops and X update are done with v, geo, cab, ccd
           if (!cab_ready) {
