@@ -1,6 +1,7 @@
 // Device-side state of one Fock-build context (struct pfe_context of the C ABI).
 #pragma once
 
+#include <algorithm>
 #include <atomic>
 
 #include <cublas_v2.h>
@@ -41,6 +42,85 @@ struct BoysTables {
   }
 };
 int acquire_boys(int device, const double* igamma, cudaStream_t s, std::shared_ptr<BoysTables>* out);
+
+// Device memory of a context or batch.  Requests of up to kSmall bytes are cut from
+// blocks that are kept from one set-up to the next (a set-up makes over a hundred, and
+// cudaMalloc and cudaFree were most of a small molecule's: 1.1 of 2.6 ms); larger ones,
+// and small ones beyond kBlocks blocks, are allocations of their own, but for one buffer
+// of up to kKept bytes (`kept`) that also stays.  All of it is freed with the owner.  A block's memory may still be read by a build in flight when the
+// next set-up begins, so release_all waits for the device, as cudaFree does.
+struct DeviceMemory {
+  static constexpr size_t kSmall = 256 << 10, kBlock = 2 << 20;
+  static constexpr int kBlocks = 8;
+  std::vector<void*> owned;    // allocations of their own
+  std::vector<char*> blocks;
+  size_t block = 0, offset = 0;   // the next small request: blocks[block] + offset
+  static constexpr size_t kKept = 64 << 20;
+  void* kept = nullptr;
+  size_t kept_bytes = 0;
+  DeviceMemory() = default;
+  DeviceMemory(const DeviceMemory&) = delete;
+  DeviceMemory& operator=(const DeviceMemory&) = delete;
+  ~DeviceMemory() {
+    for (char* b : blocks) cudaFree(b);
+    cudaFree(kept);
+  }
+
+  cudaError_t alloc(void** p, size_t bytes) {
+    if (cudaError_t f = injected_alloc_failure()) return f;
+    const size_t n = (std::max<size_t>(bytes, 1) + 255) & ~size_t(255);
+    if (n <= kSmall) {
+      if (block < blocks.size() && offset + n > kBlock) {
+        ++block;
+        offset = 0;
+      }
+      if (block == blocks.size() && blocks.size() < (size_t)kBlocks) {
+        char* b = nullptr;
+        const cudaError_t e = cudaMalloc((void**)&b, kBlock);
+        if (e != cudaSuccess) return e;
+        blocks.push_back(b);
+      }
+      if (block < blocks.size()) {
+        *p = blocks[block] + offset;
+        offset += n;
+        return cudaSuccess;
+      }
+    }
+    const cudaError_t e = cudaMalloc(p, n);
+    if (e == cudaSuccess) owned.push_back(*p);
+    return e;
+  }
+  // The one buffer that outlasts set-ups: as large as the largest asked for, up to kKept.
+  cudaError_t alloc_kept(void** p, size_t bytes) {
+    if (bytes > kKept) return alloc(p, bytes);
+    if (cudaError_t f = injected_alloc_failure()) return f;
+    if (bytes > kept_bytes) {
+      cudaFree(kept);
+      kept = nullptr;
+      kept_bytes = 0;
+      const cudaError_t e = cudaMalloc(&kept, bytes);
+      if (e != cudaSuccess) return e;
+      kept_bytes = bytes;
+    }
+    *p = kept;
+    return cudaSuccess;
+  }
+  // (memory cut from a block stays taken until release_all)
+  void free_now(void* p) {
+    for (size_t i = 0; p && i < owned.size(); ++i)
+      if (owned[i] == p) {
+        owned.erase(owned.begin() + i);
+        cudaFree(p);
+        return;
+      }
+  }
+  void release_all() {
+    if (block > 0 || offset > 0 || kept) cudaDeviceSynchronize();
+    for (void* p : owned) cudaFree(p);
+    owned.clear();
+    block = offset = 0;
+  }
+};
 
 // Primitive-shell table, struct of arrays (n shells).
 struct DevShells {
@@ -127,7 +207,7 @@ struct ClassLaunch {
 }  // namespace pfe
 
 // The opaque handle of the C ABI.
-struct pfe_context {
+struct pfe_context : pfe::DeviceMemory {
   // block panels of the digestion (molecules; pfe_mol.cu): the kept components of every
   // contracted block are consecutive panel rows, and the matrices of a block pair are
   // contiguous: element (p, q) at row_base[p] + q * row_n[p], where a block of n rows
@@ -249,32 +329,15 @@ struct pfe_context {
   int ev_gmul[64] = {0};
   int nprof = 0;
 
-  std::vector<void*> owned;    // freed on reset/destroy
   std::vector<void*> pending;  // scratch freed at the end of setup
 
-  cudaError_t alloc(void** p, size_t bytes) {
-    if (cudaError_t f = pfe::injected_alloc_failure()) return f;
-    cudaError_t e = cudaMalloc(p, bytes ? bytes : 16);
-    if (e == cudaSuccess) owned.push_back(*p);
-    return e;
-  }
-  void free_now(void* p) {
-    if (!p) return;
-    for (size_t i = 0; i < owned.size(); ++i)
-      if (owned[i] == p) {
-        owned.erase(owned.begin() + i);
-        break;
-      }
-    cudaFree(p);
-  }
   void free_later(void* p) { pending.push_back(p); }
   void free_pending() {
     for (void* p : pending) free_now(p);
     pending.clear();
   }
   void release_all() {
-    for (void* p : owned) cudaFree(p);
-    owned.clear();
+    pfe::DeviceMemory::release_all();
     pending.clear();
   }
 };
@@ -283,7 +346,7 @@ struct pfe_context {
 // every instance has its own context (set-up, pairs, chunks); the batch joins
 // their chunk lists per quartet class, each chunk tagged with its instance, so
 // one launch per class (and pass) covers every instance.
-struct pfe_batch {
+struct pfe_batch : pfe::DeviceMemory {
   int device = 0;
   std::vector<pfe_context*> inst;
   std::vector<long long> off;       // packed offsets (doubles) of the ncgs x ncgs matrices, n+1
@@ -301,16 +364,8 @@ struct pfe_batch {
   const double* insts_for = nullptr;  // density the records point at (null: rewrite them)
   bool mixed = false;               // FP32-capable kernels (sticky once any instance asked for them)
   bool ready = false;               // set by a pfe_batch_setup that succeeded
-  std::vector<void*> owned;
-  cudaError_t alloc(void** p, size_t bytes) {
-    if (cudaError_t f = pfe::injected_alloc_failure()) return f;
-    cudaError_t e = cudaMalloc(p, bytes ? bytes : 16);
-    if (e == cudaSuccess) owned.push_back(*p);
-    return e;
-  }
   void release_all() {
-    for (void* p : owned) cudaFree(p);
-    owned.clear();
+    pfe::DeviceMemory::release_all();
     if (h_insts) cudaFreeHost(h_insts);
     h_insts = nullptr;
     if (ev_insts) cudaEventDestroy(ev_insts);

@@ -377,53 +377,53 @@ __global__ void k_piece_count(const Chunk* __restrict__ chunks, const unsigned c
   npiece[c] = pc.k * pc.m * pc.l;
 }
 
-// The pieces of every chunk at its offset (one warp per chunk), tagged with the
-// instance, and the key of each: its class pair, then its screened quartets
-// descending (the work queues hand out the costliest first); pieces without a
-// quartet get the last key and are dropped.
+// The pieces of a molecule's chunks (one warp per piece, found by its offset), tagged
+// with the instance, and the key of each: its class pair, then its screened quartets
+// descending (the work queues hand out the costliest first); pieces without a quartet
+// get the last key and are dropped.
 __global__ void k_piece_fill(const Chunk* __restrict__ chunks, const unsigned char* __restrict__ pair,
                              const unsigned int* __restrict__ steps, const unsigned int* __restrict__ cost, int nchunks,
                              GroupView v, const __grid_constant__ PairMost pm, int inst, const int* __restrict__ off,
                              Chunk* __restrict__ out, unsigned long long* __restrict__ key,
                              PairStat* __restrict__ stat) {
-  const int c = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
   const int lane = threadIdx.x & 31;
-  if (c >= nchunks) return;
+  const int o = off[0] + blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
+  if (o >= off[nchunks]) return;
+  int lo = 0, hi = nchunks - 1;   // the last chunk that begins at or before o
+  while (lo < hi) {
+    const int mid = (lo + hi + 1) >> 1;
+    if (off[mid] <= o) lo = mid; else hi = mid - 1;
+  }
+  const int c = lo, i = o - off[c];
   const Chunk ch = chunks[c];
   const int code = pair[c];
   const PieceCut pc = cut_chunk(ch, steps[c], pm.most[code], (pm.serial >> code) & 1, v);
-  int hmax = 1;
-  if (pc.l > 1)
-    for (int i = ch.first; i < ch.end; ++i) hmax = max(hmax, v.gr_n[v.bk_list[i]]);
+  const int ik = i / (pc.m * pc.l), im = i / pc.l % pc.m, il = i % pc.l;
   const int nk = ch.end - ch.first, np = ch.p1 - ch.p0;
-  int o = off[c];
-  unsigned int live = 0;
-  for (int ik = 0; ik < pc.k; ++ik)
-    for (int im = 0; im < pc.m; ++im)
-      for (int il = 0; il < pc.l; ++il, ++o) {
-        Chunk q = ch;
-        q.inst = inst;
-        q.first = ch.first + (int)((long long)nk * ik / pc.k);
-        q.end = ch.first + (int)((long long)nk * (ik + 1) / pc.k);
-        q.p0 = ch.p0 + (int)((long long)np * im / pc.m);
-        q.p1 = ch.p0 + (int)((long long)np * (im + 1) / pc.m);
-        if (pc.l > 1) {
-          q.q0 = (int)((long long)hmax * il / pc.l);
-          q.q1 = (int)((long long)hmax * (il + 1) / pc.l);
-        }
-        const int li = q.first + lane;
-        unsigned long long n = cost[c];
-        if (pc.k * pc.m * pc.l > 1) n = li < q.end ? piece_quartets(v, q.G, v.bk_list[li], q.p0, q.p1, q.q0, q.q1) : 0ull;
-        if (pc.k * pc.m * pc.l > 1)
-          for (int d = 16; d > 0; d >>= 1) n += __shfl_xor_sync(0xffffffffu, n, d);
-        if (lane == 0) {
-          out[o] = q;
-          key[o] = n ? ((unsigned long long)code << 32) | (0xffffffffull - min(n, 0xffffffffull))
-                     : (unsigned long long)kClassPairs << 32;
-        }
-        live += n ? 1u : 0u;
-      }
-  if (lane == 0 && live) atomicAdd(&stat[code].live, live);
+  Chunk q = ch;
+  q.inst = inst;
+  q.first = ch.first + (int)((long long)nk * ik / pc.k);
+  q.end = ch.first + (int)((long long)nk * (ik + 1) / pc.k);
+  q.p0 = ch.p0 + (int)((long long)np * im / pc.m);
+  q.p1 = ch.p0 + (int)((long long)np * (im + 1) / pc.m);
+  if (pc.l > 1) {
+    int hmax = 1;
+    for (int x = ch.first; x < ch.end; ++x) hmax = max(hmax, v.gr_n[v.bk_list[x]]);
+    q.q0 = (int)((long long)hmax * il / pc.l);
+    q.q1 = (int)((long long)hmax * (il + 1) / pc.l);
+  }
+  unsigned long long n = cost[c];
+  if (pc.k * pc.m * pc.l > 1) {
+    const int li = q.first + lane;
+    n = li < q.end ? piece_quartets(v, q.G, v.bk_list[li], q.p0, q.p1, q.q0, q.q1) : 0ull;
+    for (int d = 16; d > 0; d >>= 1) n += __shfl_xor_sync(0xffffffffu, n, d);
+  }
+  if (lane == 0) {
+    out[o] = q;
+    key[o] = n ? ((unsigned long long)code << 32) | (0xffffffffull - min(n, 0xffffffffull))
+               : (unsigned long long)kClassPairs << 32;
+    if (n) atomicAdd(&stat[code].live, 1u);
+  }
 }
 
 __global__ void k_piece_gather(const Chunk* __restrict__ in, const int* __restrict__ perm, int n,
@@ -1074,7 +1074,7 @@ static int alloc_integrals(Owner* own, ClassLaunch* launches, int nlaunch, int b
   unsigned char* f = nullptr;
   if (most > 0) {
     const size_t flags = own->concurrent ? sum_flags : most_flags;
-    PFE_CUDA(own->alloc((void**)&x, own->concurrent ? sum : most));
+    PFE_CUDA(own->alloc_kept((void**)&x, own->concurrent ? sum : most));
     PFE_CUDA(own->alloc((void**)&f, flags));
     PFE_CUDA(cudaMemset(f, 0, flags));
   }
@@ -1112,12 +1112,12 @@ static int finish_chunks(Owner* own, pfe_context* const* inst, int ninst, ClassL
   Chunk* sorted = nullptr;
   if (nraw > 0) {
     struct Scratch {   // freed on every way out
+      Owner* own;
       std::vector<void*> p;
-      ~Scratch() { for (void* q : p) cudaFree(q); }
-    } scratch;
+      ~Scratch() { for (void* q : p) own->free_now(q); }
+    } scratch{own, {}};
     auto tmp = [&](auto** p, size_t bytes) -> cudaError_t {
-      if (cudaError_t f = injected_alloc_failure()) return f;
-      const cudaError_t e = cudaMalloc((void**)p, bytes ? bytes : 16);
+      const cudaError_t e = own->alloc((void**)p, bytes);
       if (e == cudaSuccess) scratch.p.push_back((void*)*p);
       return e;
     };
@@ -1142,9 +1142,14 @@ static int finish_chunks(Owner* own, pfe_context* const* inst, int ninst, ClassL
     cub::DeviceScan::ExclusiveSum(nullptr, tb, npiece, off, (int)nraw + 1, s);
     PFE_CUDA(tmp(&cub_tmp, tb + 16));
     PFE_CUDA(cub::DeviceScan::ExclusiveSum(cub_tmp, tb, npiece, off, (int)nraw + 1, s));
-    int total = 0;
-    PFE_CUDA(cudaMemcpyAsync(&total, off + nraw, sizeof(int), cudaMemcpyDeviceToHost, s));
+    std::vector<int> first(ninst + 1, 0);   // where each instance's pieces begin
+    o = 0;
+    for (int k = 0; k < ninst; ++k) {
+      o += inst[k]->nraw;
+      PFE_CUDA(cudaMemcpyAsync(&first[k + 1], off + o, sizeof(int), cudaMemcpyDeviceToHost, s));
+    }
     PFE_CUDA(cudaStreamSynchronize(s));
+    const int total = first[ninst];
     Chunk* pieces = nullptr;
     unsigned long long *key = nullptr, *key2 = nullptr;
     int *iota = nullptr, *perm = nullptr;
@@ -1158,7 +1163,9 @@ static int finish_chunks(Owner* own, pfe_context* const* inst, int ninst, ClassL
     for (int k = 0; k < ninst; ++k) {
       const pfe_context* c = inst[k];
       if (c->nraw == 0) continue;
-      k_piece_fill<<<(c->nraw + 3) / 4, 128, 0, s>>>(c->d_raw, c->d_raw_pair, c->d_raw_steps, c->d_raw_cost, c->nraw,
+      // this instance's pieces: off[o] .. off[o + nraw] of the joined list
+      const int n = first[k + 1] - first[k];
+      if (n > 0) k_piece_fill<<<(n + 3) / 4, 128, 0, s>>>(c->d_raw, c->d_raw_pair, c->d_raw_steps, c->d_raw_cost, c->nraw,
                                                      group_view(c), pm, k, off + o, pieces, key, d_stat);
       o += c->nraw;
     }
