@@ -17,7 +17,7 @@ LIB = os.path.join(OUT, 'libpolymer_fock.so')
 # the largest units first: the pool starts them before the small ones
 SOURCES = ['pfe_mol_big2.cu', 'pfe_mol_big6.cu', 'pfe_mol_big4.cu', 'pfe_mol_big8.cu', 'pfe_mol_big3.cu',
            'pfe_mol_big7.cu', 'pfe_mol_big1.cu', 'pfe_mol_big5.cu', 'pfe_mol.cu', 'pfe_mol_batch.cu',
-           'pfe_mol_mixed.cu', 'pfe_mol_batch_mixed.cu', 'pfe_mol_wide.cu', 'pfe_mol_digest.cu', 'pfe_api.cu', 'pfe_eri.cu', 'pfe_lattice.cu', 'pfe_lattice_sl.cu', 'pfe_lattice_wide.cu',
+           'pfe_mol_mixed.cu', 'pfe_mol_batch_mixed.cu', 'pfe_mol_wide.cu', 'pfe_mol_digest.cu', 'pfe_api.cu', 'pfe_eri.cu', 'pfe_lattice.cu', 'pfe_lattice_sl.cu', 'pfe_lattice_sl2.cu', 'pfe_lattice_sl3.cu', 'pfe_lattice_wide.cu',
            'pfe_grad.cu', 'pfe_onee.cu',
            'pfe_mlp.cu', 'pfe_scf.cu']
 NVCC = os.environ.get('NVCC', 'nvcc')

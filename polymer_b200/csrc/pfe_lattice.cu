@@ -858,7 +858,7 @@ int lattice_class_launches(pfe_context* ctx) {
   for (int i = 0; i < L->nlaunch; ++i) {
     const LatticeLaunch& ll = L->launches[i];
     const int e1 = std::max(ll.cb, ll.ck), e2 = std::min(ll.cb, ll.ck);
-    n += L->interpret_only ? 1 : std::max(1, lattice_sl_passes(e1, e2));
+    n += L->interpret_only ? 1 : std::max(1, lattice_sl_passes(e1, e2, ll.cb < ll.ck));
   }
   return n;
 }

@@ -49,7 +49,7 @@ struct LatticeRun {
 // chunk's bra class is e2) on `grid` blocks of 128 threads, or null where the
 // class has more than 64 integrals (it keeps the op-table interpreter).
 // work-queue counters per lattice class launch (one per register pass)
-constexpr int kLatQueueSlots = 4;
+constexpr int kLatQueueSlots = 8;
 using LatSlFn = void (*)(const LatticeRun&, int grid, cudaStream_t);
 LatSlFn lattice_sl_launcher(int e1, int e2, bool sw);
 // The warp-per-quartet kernel of a class with d shells for bases whose d shells are all
@@ -60,6 +60,9 @@ LatWideFn lattice_wide_launcher(int e1, int e2, bool sw);
 void lattice_ghost_check(const double* p, long long n, int npgs, const int* tidx, int* flag, int num_sms,
                          cudaStream_t s);
 // launches (register passes) of a straight-line class, 0 where the class has none
-int lattice_sl_passes(int e1, int e2);
+int lattice_sl_passes(int e1, int e2, bool sw);
+// the launchers of classes with d shells in register passes (pfe_lattice_sl2.cu, pfe_lattice_sl3.cu)
+LatSlFn lattice_sl_launcher_d(int e1, int e2, bool sw);
+LatSlFn lattice_sl_launcher_2110(bool sw);
 
 }  // namespace pfe

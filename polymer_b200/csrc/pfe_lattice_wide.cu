@@ -251,9 +251,6 @@ void lattice_ghost_check(const double* p, long long n, int npgs, const int* tidx
 LatWideFn lattice_wide_launcher(int e1, int e2, bool sw) {
 #define L2(A, B, C, D) (sw ? &launch_wide<A, B, C, D, true> : &launch_wide<A, B, C, D, false>)
   switch (e1 * 8 + e2) {
-    case 26: return L2(2, 0, 1, 1);
-    case 27: return L2(2, 0, 2, 0);
-    case 33: return L2(2, 1, 1, 0);
     case 34: return L2(2, 1, 1, 1);
     case 35: return L2(2, 1, 2, 0);
     case 36: return L2(2, 1, 2, 1);
