@@ -10,12 +10,15 @@
 
 #include <cmath>
 #include <cstdio>
+#include <cstring>
+#include <memory>
 #include <mutex>
 #include <string>
 #include <type_traits>
 #include <vector>
 
 #include "pfe_common.cuh"
+#include "pfe_context.cuh"
 
 namespace pfe {
 
@@ -318,14 +321,6 @@ static void launch_nuclear(const OneeDev& d, const int* list, const int* start, 
   run(k_nuclear<0, 0, false>, 0, 0);
 }
 
-template <typename T>
-static int upload(std::vector<void*>& owned, const T* h, size_t n, T** d) {
-  PFE_CUDA(cudaMalloc((void**)d, sizeof(T) * (n ? n : 1)));
-  owned.push_back(*d);
-  PFE_CUDA(cudaMemcpy(*d, h, sizeof(T) * n, cudaMemcpyHostToDevice));
-  return PFE_OK;
-}
-
 // Host-side checks shared by the one-electron entry points, made before any
 // device work: the kernels index S_P/T_P/N_P by P_SHELL of every component a
 // shell reaches (i1+i2+i3 <= P_SHELL_ANG) and by the shell head P_SHELL(s,0,0,0),
@@ -365,19 +360,33 @@ static int onee_validate(const pfe_onee_args* a, bool need_atoms) {
   return PFE_OK;
 }
 
+// Device scratch of the allocating entry points, per device: the inputs, packed, and the
+// results.  Up to kScratchKept bytes stay from call to call (the thirteen allocations and
+// copies of a call were most of its time); larger calls allocate and free their own.
+struct OneeScratch {
+  std::mutex mu;   // held for the whole call
+  char* p = nullptr;
+  size_t n = 0;
+  std::vector<char> host;              // the packed inputs
+  std::shared_ptr<BoysTables> boys;    // of the last IGAMMA
+};
+static OneeScratch g_onee[64];
+constexpr size_t kScratchKept = (size_t)64 << 20;
+
+static size_t round256(size_t b) { return (b + 255) & ~size_t(255); }
+
 static int onee_run(const pfe_onee_args* a, double* s_p, double* t_p, double* n_p) {
   if (const int v = onee_validate(a, true)) return v;
-  std::vector<void*> owned;
-  OneeDev d{};
-  int rc = PFE_OK;
+  int dev = 0;
+  PFE_CUDA(cudaGetDevice(&dev));
+  if (dev < 0 || dev >= 64) { set_error("device index out of range"); return PFE_EINVAL; }
+  OneeScratch& sc = g_onee[dev];
+  std::lock_guard<std::mutex> lock(sc.mu);
+  int rc = acquire_boys(dev, a->igamma, nullptr, &sc.boys);
+  if (rc != PFE_OK) return rc;
   const size_t psz = (size_t)a->npshell * NPOW * NPOW * NPOW;
   const int n1 = (2 * a->cel1[0] + 1) * (2 * a->cel1[1] + 1) * (2 * a->cel1[2] + 1);
-  const size_t out_n = (size_t)a->npgs * a->npgs * n1;
-  double *ds = nullptr, *dt = nullptr, *dn = nullptr;
-  std::vector<double> tab((size_t)NIG_T * NIG_M);
-  for (int t = 0; t < NIG_T; ++t)
-    for (int m = 0; m < NIG_M; ++m) tab[(size_t)t * NIG_M + m] = a->igamma[t + (size_t)NIG_T * m];
-  int* dps = nullptr; int* dang = nullptr; int* diat = nullptr; int* dlist = nullptr;
+  const size_t out_bytes = sizeof(double) * (size_t)a->npgs * a->npgs * n1;
   std::vector<int> list;   // the shells ordered by L
   int start[4] = {0, 0, 0, 0};
   for (int L = 0; L <= LMAX_SUPPORTED; ++L) {
@@ -385,57 +394,72 @@ static int onee_run(const pfe_onee_args* a, double* s_p, double* t_p, double* n_
       if (a->p_shell_ang[sh] == L) list.push_back(sh);
     start[L + 1] = (int)list.size();
   }
-  double *dx = nullptr, *dy = nullptr, *dz = nullptr, *dzt = nullptr, *dax = nullptr, *day = nullptr, *daz = nullptr, *dboys = nullptr;
-  if ((rc = upload(owned, a->p_shell, psz, &dps)) || (rc = upload(owned, a->p_shell_ang, (size_t)a->npshell, &dang)) ||
-      (rc = upload(owned, a->pgsx, (size_t)a->npgs, &dx)) || (rc = upload(owned, a->pgsy, (size_t)a->npgs, &dy)) ||
-      (rc = upload(owned, a->pgsz, (size_t)a->npgs, &dz)) || (rc = upload(owned, a->zt, (size_t)a->npgs, &dzt)) ||
-      (rc = upload(owned, a->iatom, (size_t)a->natom, &diat)) || (rc = upload(owned, a->atomx, (size_t)a->natom, &dax)) ||
-      (rc = upload(owned, a->atomy, (size_t)a->natom, &day)) || (rc = upload(owned, a->atomz, (size_t)a->natom, &daz)) ||
-      (rc = upload(owned, tab.data(), tab.size(), &dboys)) || (rc = upload(owned, list.data(), list.size(), &dlist)))
-    goto done;
+  // the inputs, packed, and their places
+  struct Part {
+    const void* h;
+    size_t bytes, at;
+  };
+  const size_t pg = sizeof(double) * a->npgs, at = sizeof(double) * a->natom;
+  Part part[] = {{a->p_shell, sizeof(int) * psz, 0}, {a->p_shell_ang, sizeof(int) * a->npshell, 0},
+                 {a->pgsx, pg, 0}, {a->pgsy, pg, 0}, {a->pgsz, pg, 0}, {a->zt, pg, 0},
+                 {a->iatom, sizeof(int) * a->natom, 0}, {a->atomx, at, 0}, {a->atomy, at, 0}, {a->atomz, at, 0},
+                 {list.data(), sizeof(int) * list.size(), 0}};
+  size_t in_bytes = 0;
+  for (Part& p : part) {
+    p.at = in_bytes;
+    in_bytes += round256(p.bytes);
+  }
+  const int nout = n_p ? 1 : 2;
+  const size_t need = in_bytes + nout * round256(out_bytes);
+  char* own = nullptr;   // freed on every way out
+  struct Guard {
+    char*& p;
+    ~Guard() { cudaFree(p); }
+  } guard{own};
+  char* base = nullptr;
+  if (need > kScratchKept) {
+    PFE_CUDA(cudaMalloc((void**)&own, need));
+    base = own;
+  } else {
+    if (need > sc.n) {
+      cudaFree(sc.p);
+      sc.p = nullptr;
+      sc.n = 0;
+      PFE_CUDA(cudaMalloc((void**)&sc.p, need));
+      sc.n = need;
+    }
+    base = sc.p;
+  }
+  sc.host.resize(in_bytes);
+  for (const Part& p : part) memcpy(sc.host.data() + p.at, p.h, p.bytes);
+  PFE_CUDA(cudaMemcpy(base, sc.host.data(), in_bytes, cudaMemcpyHostToDevice));
+  auto i32 = [&](int k) { return reinterpret_cast<const int*>(base + part[k].at); };
+  auto f64 = [&](int k) { return reinterpret_cast<const double*>(base + part[k].at); };
+  OneeDev d{};
   d.npgs = a->npgs; d.npshell = a->npshell; d.natom = a->natom;
-  d.p_shell = dps; d.ang = dang; d.x = dx; d.y = dy; d.z = dz; d.zt = dzt;
-  d.iatom = diat; d.ax = dax; d.ay = day; d.az = daz; d.boys = dboys;
+  d.p_shell = i32(0); d.ang = i32(1); d.x = f64(2); d.y = f64(3); d.z = f64(4); d.zt = f64(5);
+  d.iatom = i32(6); d.ax = f64(7); d.ay = f64(8); d.az = f64(9); d.boys = sc.boys->rows;
   for (int k = 0; k < 3; ++k) { d.cel1[k] = a->cel1[k]; d.cel2[k] = a->cel2[k]; d.period[k] = a->period[k]; }
   d.helix = a->helix;
-  {
+  double* out0 = reinterpret_cast<double*>(base + in_bytes);
+  double* out1 = reinterpret_cast<double*>(base + in_bytes + round256(out_bytes));
+  // elements of primitives that no shell component reaches stay zero
+  PFE_CUDA(cudaMemsetAsync(out0, 0, nout * round256(out_bytes), nullptr));
+  if (n_p) {
+    launch_nuclear(d, i32(10), start, n1, out0);
+  } else {
     const long long total = (long long)a->npshell * a->npshell * n1;
-    const unsigned grid = (unsigned)((total + 127) / 128);
-    if (s_p || t_p) {
-      if (cudaMalloc(&ds, sizeof(double) * out_n) != cudaSuccess || cudaMalloc(&dt, sizeof(double) * out_n) != cudaSuccess) {
-        set_error("cudaMalloc failed");
-        rc = PFE_ENOMEM;
-        goto done;
-      }
-      owned.push_back(ds);
-      owned.push_back(dt);
-      cudaMemset(ds, 0, sizeof(double) * out_n);
-      cudaMemset(dt, 0, sizeof(double) * out_n);
-      k_overlap_kinetic<<<grid, 128>>>(d, ds, dt);
-      if (cudaGetLastError() != cudaSuccess || cudaDeviceSynchronize() != cudaSuccess) {
-        set_error("k_overlap_kinetic failed");
-        rc = PFE_ECUDA;
-        goto done;
-      }
-      if (s_p) cudaMemcpy(s_p, ds, sizeof(double) * out_n, cudaMemcpyDeviceToHost);
-      if (t_p) cudaMemcpy(t_p, dt, sizeof(double) * out_n, cudaMemcpyDeviceToHost);
-    }
-    if (n_p) {
-      if (cudaMalloc(&dn, sizeof(double) * out_n) != cudaSuccess) { set_error("cudaMalloc failed"); rc = PFE_ENOMEM; goto done; }
-      owned.push_back(dn);
-      cudaMemset(dn, 0, sizeof(double) * out_n);
-      launch_nuclear(d, dlist, start, n1, dn);
-      if (cudaGetLastError() != cudaSuccess || cudaDeviceSynchronize() != cudaSuccess) {
-        set_error("k_nuclear failed");
-        rc = PFE_ECUDA;
-        goto done;
-      }
-      cudaMemcpy(n_p, dn, sizeof(double) * out_n, cudaMemcpyDeviceToHost);
-    }
+    k_overlap_kinetic<<<(unsigned)((total + 127) / 128), 128>>>(d, out0, out1);
   }
-done:
-  for (void* p : owned) cudaFree(p);
-  return rc;
+  PFE_CUDA(cudaGetLastError());
+  if (n_p) {
+    PFE_CUDA(cudaMemcpy(n_p, out0, out_bytes, cudaMemcpyDeviceToHost));
+  } else {
+    if (s_p) PFE_CUDA(cudaMemcpy(s_p, out0, out_bytes, cudaMemcpyDeviceToHost));
+    if (t_p) PFE_CUDA(cudaMemcpy(t_p, out1, out_bytes, cudaMemcpyDeviceToHost));
+    if (!s_p && !t_p) PFE_CUDA(cudaDeviceSynchronize());
+  }
+  return PFE_OK;
 }
 
 // ---------------------------------------------------------------- fixed-scratch variant
@@ -454,8 +478,6 @@ static __device__ __align__(256) unsigned char g_noalloc_scratch[kNoAllocScratch
 
 static std::mutex g_noalloc_mu;          // held for the whole call: calls share the one buffer
 static void* g_noalloc_ptr[64] = {nullptr};
-
-static size_t round256(size_t b) { return (b + 255) & ~size_t(255); }
 
 // Device address of the scratch on the current device.  The first call on a
 // device does the set-up (loads the module there, looks up the symbol).
