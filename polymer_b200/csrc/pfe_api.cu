@@ -223,6 +223,8 @@ static void reset_context(pfe_context* ctx) {
   ctx->d_poff = ctx->d_ptgt = ctx->d_prown = ctx->d_pinv = ctx->d_pinv_row = nullptr;
   ctx->d_prow = nullptr;
   ctx->d_pd = ctx->d_pj = ctx->d_pk = nullptr;
+  ctx->d_tile = nullptr;
+  ctx->d_tile_at = nullptr;
   ctx->d_raw = nullptr;
   ctx->d_raw_steps = ctx->d_raw_cost = nullptr;
   ctx->d_raw_pair = nullptr;

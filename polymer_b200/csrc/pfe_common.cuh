@@ -114,6 +114,24 @@ constexpr int kDownMax = 8;
 constexpr int kDownCols = 8;
 __host__ __device__ constexpr size_t down_row(int L, int t) { return ((size_t)L * NIG_T + t) * kDownCols; }
 
+// The rows of boys_down that top order L reads (T below TF(L)), as four arrays of 16-byte
+// pieces in shared memory: a gather there costs the conflicts of eight lanes over eight
+// bank groups (about 11 wavefronts), in global memory a wavefront per lane.
+constexpr int kTF[3] = {33, 37, 41};   // TF(0:2)
+template <int L>
+struct DownSmem {
+  static constexpr bool use = L <= 2;
+  static constexpr int ROWS = use ? 20 * kTF[L < 3 ? L : 0] + 1 : 0;
+  static constexpr size_t BYTES = sizeof(double) * kDownCols * (size_t)ROWS;
+};
+
+template <int L>
+__device__ __forceinline__ void down_stage(const double* __restrict__ down, double2* __restrict__ s) {
+  constexpr int N = DownSmem<L>::ROWS;
+  const double2* g = reinterpret_cast<const double2*>(down + down_row(L, 0));
+  for (int i = threadIdx.x; i < 4 * N; i += blockDim.x) s[(i & 3) * N + (i >> 2)] = __ldg(g + i);
+}
+
 // F_m(T)*pref for m = 0..L (L <= kDownMax): below TF(L) the top order alone from the
 // reference's 6-term series about the nearest grid point, e^-T from its tabulated value and
 // the series of e^(T0-T) (|T0-T| <= 0.025: 8 terms leave 4e-18), and the lower orders by
@@ -122,15 +140,22 @@ __host__ __device__ constexpr size_t down_row(int L, int t) { return ((size_t)L 
 // gathers per lane from rows of one line instead of up to eight from rows 224 bytes apart
 // (the part of the table that a class reads shrinks from 190 to 55 KB at L = 3, inside the
 // L1), and 15 + 2L multiply-adds instead of 7(L + 1).  The two agree to rounding.
-template <int L>
+// SMEM: `staged` holds the rows (down_stage), else they are read from `down`.
+template <int L, bool SMEM = false>
 __device__ __forceinline__ void boys_down(double T, double pref, const double* __restrict__ down,
-                                          double* __restrict__ F) {
+                                          double* __restrict__ F, const double2* staged = nullptr) {
   static_assert(L <= kDownMax, "boys_down: orders 0..8");
   if (T < c_TF[L]) {
     const int ts = (int)floor(T * 20.0 + 0.5);   // NINT for T >= 0; <= 20 TF(L) < NIG_T
     const double h = 0.05 * (double)ts - T;
-    const double2* r = reinterpret_cast<const double2*>(down + down_row(L, ts));
-    const double2 a = __ldg(r), b = __ldg(r + 1), c = __ldg(r + 2), d = __ldg(r + 3);
+    double2 a, b, c, d;
+    if constexpr (SMEM) {
+      constexpr int N = DownSmem<L>::ROWS;
+      a = staged[ts]; b = staged[N + ts]; c = staged[2 * N + ts]; d = staged[3 * N + ts];
+    } else {
+      const double2* r = reinterpret_cast<const double2*>(down + down_row(L, ts));
+      a = __ldg(r); b = __ldg(r + 1); c = __ldg(r + 2); d = __ldg(r + 3);
+    }
     const double f = fma(fma(fma(fma(fma(fma(d.x, h, c.y), h, c.x), h, b.y), h, b.x), h, a.y), h, a.x);
     const double x = fma(fma(fma(fma(fma(fma(fma(1.0 / 5040.0, h, 1.0 / 720.0), h, 1.0 / 120.0), h, 1.0 / 24.0), h,
                                      1.0 / 6.0), h, 0.5), h, 1.0), h, 1.0);

@@ -280,6 +280,8 @@ struct pfe_context : pfe::DeviceMemory {
   int* d_gr_n = nullptr;
   double* d_gr_max = nullptr;
   int* d_bk_list = nullptr;  // group ids ordered by (class, size bucket, group)
+  double2* d_tile = nullptr; // their pair records by tile of 32 list entries (load_tile)
+  int* d_tile_at = nullptr;  // list position of a tile's first group -> base of the tile
   // density-dependent screening of molecular builds (no counterpart in the reference, which
   // screens by the Schwarz bounds alone): skip quartets with bound * max|P| < dtol, and run
   // the recursion in FP32 where bound * max|P| < mcut; max|P| per pair of contracted blocks

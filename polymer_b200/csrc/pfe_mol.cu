@@ -217,6 +217,38 @@ __device__ __forceinline__ int reach_end(const double* __restrict__ gr_max, cons
   return e;
 }
 
+// The longest group of every tile (warp per tile), its length.
+__global__ void k_tile_len(const int* __restrict__ bk_list, const int* __restrict__ gr_n,
+                           const int2* __restrict__ tiles, int ntiles, int* __restrict__ len) {
+  const int t = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
+  const int lane = threadIdx.x & 31;
+  if (t >= ntiles) return;
+  const int2 tl = tiles[t];   // first list entry, entries
+  int n = lane < tl.y ? gr_n[bk_list[tl.x + lane]] : 0;
+  for (int o = 16; o > 0; o >>= 1) n = max(n, __shfl_xor_sync(0xffffffffu, n, o));
+  if (lane == 0) len[t] = n;
+}
+
+// The tiles' records, interleaved by lane; lanes past their group's end hold zeros.
+__global__ void k_tile_fill(const int* __restrict__ bk_list, const int* __restrict__ gr_start,
+                            const int* __restrict__ gr_n, const PairRec* __restrict__ rec,
+                            const int2* __restrict__ tiles, int ntiles, const int* __restrict__ base,
+                            double2* __restrict__ tile, int* __restrict__ tile_at) {
+  const int t = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
+  const int lane = threadIdx.x & 31;
+  if (t >= ntiles) return;
+  const int2 tl = tiles[t];
+  const int H = bk_list[tl.x + (lane < tl.y ? lane : 0)];
+  const int n = lane < tl.y ? gr_n[H] : 0, r0 = gr_start[H];
+  const int b = base[t], len = base[t + 1] - b;
+  if (lane == 0) tile_at[tl.x] = b;
+  for (int qi = 0; qi < len; ++qi) {
+    const double2* r = reinterpret_cast<const double2*>(rec + r0 + (qi < n ? qi : 0));
+    for (int k = 0; k < kTileRec; ++k)
+      tile[((size_t)(b + qi) * kTileRec + k) * 32 + lane] = qi < n ? r[k] : make_double2(0.0, 0.0);
+  }
+}
+
 // The class pairs of one set-up: rows are the (class pair, bra group) combinations,
 // those of pair i at [row0[i], row0[i + 1]).
 struct PairRows {
@@ -1331,6 +1363,33 @@ int molecular_setup(pfe_context* ctx, const pfe_args* a) {
     if (seg[c].s1[b] == 0) seg[c].s0[b] = i;
     seg[c].s1[b] = i + 1;
   }
+  {  // the ket records by tile: a tile is 32 consecutive list entries of one bucket
+    std::vector<int2> tiles;
+    for (int c = 0; c < 6; ++c)
+      for (int b = 0; b < NBUCKET; ++b)
+        for (int k = seg[c].s0[b]; k < seg[c].s1[b]; k += 32)
+          tiles.push_back(make_int2(k, std::min(32, seg[c].s1[b] - k)));
+    const int nt = (int)tiles.size();
+    int2* d_tiles = nullptr;
+    int *len = nullptr, *base = nullptr;
+    PFE_CUDA(ctx->alloc((void**)&d_tiles, sizeof(int2) * nt));
+    PFE_CUDA(ctx->alloc((void**)&len, sizeof(int) * (nt + 1)));
+    PFE_CUDA(ctx->alloc((void**)&base, sizeof(int) * (nt + 1)));
+    PFE_CUDA(ctx->alloc((void**)&ctx->d_tile_at, sizeof(int) * ng));
+    PFE_CUDA(cudaMemcpyAsync(d_tiles, tiles.data(), sizeof(int2) * nt, cudaMemcpyHostToDevice, s));
+    PFE_CUDA(cudaMemsetAsync(len + nt, 0, sizeof(int), s));
+    k_tile_len<<<(nt + 3) / 4, 128, 0, s>>>(ctx->d_bk_list, ctx->d_gr_n, d_tiles, nt, len);
+    PFE_CUDA(cudaGetLastError());
+    if ((rc = exclusive_sum(ctx, len, base, nt + 1, s)) != PFE_OK) return rc;
+    int total = 0;
+    PFE_CUDA(cudaMemcpyAsync(&total, base + nt, sizeof(int), cudaMemcpyDeviceToHost, s));
+    PFE_CUDA(cudaStreamSynchronize(s));
+    PFE_CUDA(ctx->alloc((void**)&ctx->d_tile, sizeof(double2) * kTileRec * 32 * (size_t)total));
+    k_tile_fill<<<(nt + 3) / 4, 128, 0, s>>>(ctx->d_bk_list, ctx->d_gr_start, ctx->d_gr_n, (const PairRec*)ctx->d_prec,
+                                             d_tiles, nt, base, ctx->d_tile, ctx->d_tile_at);
+    PFE_CUDA(cudaGetLastError());
+    for (void* p : {(void*)d_tiles, (void*)len, (void*)base}) ctx->free_now(p);
+  }
   // the chunks of every class pair cb >= ck in one list, a class pair after another
   ctx->nlaunch = 0;
   ctx->census_quartets = ctx->census_flops = ctx->census_ref = 0.0;
@@ -1503,6 +1562,9 @@ static MolLaunch make_launch(pfe_context* ctx, const double* d_dt) {
   ql.gr_n = ctx->d_gr_n;
   ql.gr_max = ctx->d_gr_max;
   ql.bk_list = ctx->d_bk_list;
+  ql.tile = ctx->d_tile;
+  ql.tile_at = ctx->d_tile_at;
+  ql.num_sms = ctx->num_sms;
   ql.blk = ctx->d_blk;
   ql.tblk = ctx->d_tblk;
   ql.bmax = ctx->d_bmax;

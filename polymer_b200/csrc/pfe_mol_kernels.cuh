@@ -4,6 +4,8 @@
 // straight-line group-quartet kernel with its pass launchers.
 #pragma once
 
+#include <algorithm>
+
 #include "pfe_common.cuh"
 #include "pfe_context.cuh"
 #include "generated/eri_classes.cuh"
@@ -29,10 +31,9 @@ struct PairView {
 
 // the record of pair t with its Schwarz bound (the quartet loops load the whole
 // record before screening on the bound: one load latency per pair, not two)
-__device__ __forceinline__ PairView load_pair(const PairRec* __restrict__ rec, int t) {
-  const double2* r = reinterpret_cast<const double2*>(rec + t);
-  const double2 a = __ldg(r), b = __ldg(r + 1), c = __ldg(r + 2), d = __ldg(r + 3), e = __ldg(r + 4),
-                f = __ldg(r + 5), g = __ldg(r + 6);
+__device__ __forceinline__ PairView pair_view(const double2* __restrict__ r, int stride) {
+  const double2 a = __ldg(r), b = __ldg(r + stride), c = __ldg(r + 2 * stride), d = __ldg(r + 3 * stride),
+                e = __ldg(r + 4 * stride), f = __ldg(r + 5 * stride), g = __ldg(r + 6 * stride);
   PairView v;
   v.P[0] = a.x; v.P[1] = a.y; v.P[2] = b.x;
   v.PA[0] = b.y; v.PA[1] = c.x; v.PA[2] = c.y;
@@ -41,6 +42,19 @@ __device__ __forceinline__ PairView load_pair(const PairRec* __restrict__ rec, i
   v.si = __double2loint(g.x); v.sj = __double2hiint(g.x);
   v.oz = g.y;
   return v;
+}
+
+__device__ __forceinline__ PairView load_pair(const PairRec* __restrict__ rec, int t) {
+  return pair_view(reinterpret_cast<const double2*>(rec + t), 1);
+}
+
+// Ket records by tile: the records of 32 consecutive ket groups of a bucket, interleaved
+// by lane, so that a warp whose lanes each read their own group's pair qi touches 28
+// lines instead of 224.  Piece k of pair qi of lane l of a tile lies at
+// ((base + qi) * kTileRec + k) * 32 + l.
+constexpr int kTileRec = 7;   // 16-byte pieces of a record
+__device__ __forceinline__ PairView load_tile(const double2* __restrict__ tile, int at, int lane) {
+  return pair_view(tile + (size_t)at * (kTileRec * 32) + lane, 32);
 }
 
 __device__ __forceinline__ double pair_bound(const PairRec* __restrict__ rec, int t) {
@@ -62,6 +76,8 @@ struct MolLaunch {
   const int* gr_n;        // group -> number of pairs
   const double* gr_max;   // group -> largest bound
   const int* bk_list;     // ket groups by (class, bucket, group)
+  const double2* tile;    // their records by tile (load_tile)
+  const int* tile_at;     // list position of a tile's first group -> base of the tile
   const int* blk;         // shell -> contracted block
   const int* tblk;        // target -> contracted block (-1: none)
   const double* bmax;     // block-pair maxima of |P_T| (density screening / mixed precision)
@@ -85,6 +101,7 @@ struct MolLaunch {
   const int* poff;
   const int* ptgt;        // panel row -> target (-1: none)
   int np;                 // panel rows
+  int num_sms;
   // one tile of a straight-line class: tickets [t0, t0 + tn) of this rank's chunks; X of
   // ticket t0 + t at xbuf + t * (kept integrals) * 32, xlive[t] set when it holds any quartet
   int t0, tn;
@@ -267,15 +284,19 @@ inline unsigned long long live_passes(int LA, int LB, int LC, int LD, int npass,
 // (11|10) 2.89 -> 2.45 ms, (20|10) 1.03 -> 0.87, (11|11) 2.11 -> 1.93 and (21|00) 0.48 -> 0.44
 // at three blocks (168 registers) against two; four cost (11|10) and (21|10) 15 %.  Above a
 // total of 4 the 255 registers of two blocks are better ((21|11), (21|20), (22|11): 5-10 %).
-// (10|00) gains 5 % at five blocks, (10|10) and (11|00) lose 10-20 % there.
+// (10|00) gains 5 % at five blocks, (10|10) and (11|00) lose 10-20 % there.  The classes up
+// to a total of 2 hold the same warps in two blocks, each with its copy of the Boys rows in
+// shared memory, on a grid of resident blocks.
 template <int LA, int LB, int LC, int LD>
 struct GqOccupancy {
-  static constexpr int NI = ncum(LA) * ncum(LB) * ncum(LC) * ncum(LD), LT = LA + LB + LC + LD;
-  static constexpr int blocks = LT <= 1 ? 5 : ((NI <= 16 && LT == 2) ? 4 : (LT <= 4 ? 3 : 1));
+  static constexpr int LT = LA + LB + LC + LD;
+  static constexpr bool staged = DownSmem<LT>::use;
+  static constexpr int threads = staged ? (LT <= 1 ? 320 : 256) : 128;
+  static constexpr int blocks = staged ? 2 : (LT <= 4 ? 3 : 1);
 };
 
 template <int LA, int LB, int LC, int LD, int NPASS, int PASS, bool MIXED, bool BATCH>
-__device__ __forceinline__ void gq_pass(const MolLaunch& lq) {
+__device__ __forceinline__ void gq_pass(const MolLaunch& lq, const double2* s_boys) {
   constexpr int NA = ncum(LA), NB = ncum(LB), NC = ncum(LC), ND = ncum(LD);
   constexpr int NI = NA * NB * NC * ND;
   constexpr int NAB = NA * NB;
@@ -342,10 +363,13 @@ __device__ __forceinline__ void gq_pass(const MolLaunch& lq) {
     // record per pair); the warp walks the bra group's pairs in step (inner loop:
     // every lane reads the same bra record, one L1 wavefront per load).  Both
     // lists are sorted by Schwarz bound, so the screens end the loops.
+    const double2* __restrict__ tile = ql.tile;
+    const int tile0 = ql.tile_at[ch.first];
     for (int qi = ch.q0;; ++qi) {
       const bool lv = qi < hn;
-      const int q = h0 + (lv ? qi : 0);
-      const PairView kq = load_pair(rec, q);
+      if (!__any_sync(0xffffffffu, lv)) break;   // past the tile's longest group
+      const int q = h0 + qi;
+      const PairView kq = load_tile(tile, tile0 + qi, lane);
       const double sq = lv ? kq.bound : 0.0;
       const bool qok = lv && sq * gmax >= thr;
       if (!__any_sync(0xffffffffu, qok)) break;
@@ -390,7 +414,7 @@ __device__ __forceinline__ void gq_pass(const MolLaunch& lq) {
         if constexpr (MIXED && LT > 0) f32 = __all_sync(__activemask(), sp * sq * pmax < mcut);
         n32 += f32 ? 1u : 0u;
         double F[LT + 1];
-        boys_down<LT>(T, f32 ? 1.0 : pref, down, F);
+        boys_down<LT, DownSmem<LT>::use>(T, f32 ? 1.0 : pref, down, F, s_boys);
         double out[NI];
         if constexpr (LT == 0) {
           out[0] = F[0];
@@ -488,22 +512,27 @@ void launch_digest(int cb, int ck, const MolLaunch& ql, int num_sms, cudaStream_
 constexpr int kPassGroup = 8;
 
 template <int LA, int LB, int LC, int LD, int NPASS, int P0, int PN, bool MIXED, bool BATCH>
-__device__ __forceinline__ void gq_select(const MolLaunch& lq, int p) {
+__device__ __forceinline__ void gq_select(const MolLaunch& lq, int p, const double2* s_boys) {
   if constexpr (PN == 1) {
-    gq_pass<LA, LB, LC, LD, NPASS, P0, MIXED, BATCH>(lq);
+    gq_pass<LA, LB, LC, LD, NPASS, P0, MIXED, BATCH>(lq, s_boys);
   } else {
-    if (p == P0) gq_pass<LA, LB, LC, LD, NPASS, P0, MIXED, BATCH>(lq);
-    else gq_select<LA, LB, LC, LD, NPASS, P0 + 1, PN - 1, MIXED, BATCH>(lq, p);
+    if (p == P0) gq_pass<LA, LB, LC, LD, NPASS, P0, MIXED, BATCH>(lq, s_boys);
+    else gq_select<LA, LB, LC, LD, NPASS, P0 + 1, PN - 1, MIXED, BATCH>(lq, p, s_boys);
   }
 }
 
 // Passes P0 .. P0 + PN - 1; blockIdx.y is the position among the live ones (bits of live).
 template <int LA, int LB, int LC, int LD, int NPASS, int P0, int PN, bool MIXED, bool BATCH>
-__global__ void __launch_bounds__(128, GqOccupancy<LA, LB, LC, LD>::blocks)
+__global__ void __launch_bounds__(GqOccupancy<LA, LB, LC, LD>::threads, GqOccupancy<LA, LB, LC, LD>::blocks)
     k_gq(const __grid_constant__ MolLaunch lq, unsigned int live) {
+  extern __shared__ double2 s_boys[];
+  if constexpr (DownSmem<LA + LB + LC + LD>::use) {   // once per resident block
+    down_stage<LA + LB + LC + LD>(lq.down, s_boys);
+    __syncthreads();
+  }
   unsigned int m = live;
   for (int y = blockIdx.y; y > 0; --y) m &= m - 1;
-  gq_select<LA, LB, LC, LD, NPASS, P0, PN, MIXED, BATCH>(lq, P0 + __ffs(m) - 1);
+  gq_select<LA, LB, LC, LD, NPASS, P0, PN, MIXED, BATCH>(lq, P0 + __ffs(m) - 1, s_boys);
 }
 
 using LaunchFn = void (*)(const MolLaunch&, int grid, cudaStream_t);
@@ -511,8 +540,19 @@ using LaunchFn = void (*)(const MolLaunch&, int grid, cudaStream_t);
 template <int LA, int LB, int LC, int LD, int NPASS, int P0, bool MIXED, bool BATCH>
 void launch_groups(const MolLaunch& ql, unsigned long long live, int grid, cudaStream_t s) {
   constexpr int PN = NPASS - P0 < kPassGroup ? NPASS - P0 : kPassGroup;
+  using O = GqOccupancy<LA, LB, LC, LD>;
   const unsigned int m = (unsigned int)(live >> P0) & ((1u << PN) - 1);
-  if (m) k_gq<LA, LB, LC, LD, NPASS, P0, PN, MIXED, BATCH><<<dim3(grid, __builtin_popcount(m)), 128, 0, s>>>(ql, m);
+  if (m) {
+    auto kern = k_gq<LA, LB, LC, LD, NPASS, P0, PN, MIXED, BATCH>;
+    constexpr size_t bytes = DownSmem<O::LT>::BYTES;
+    // `grid` counts blocks of four warps
+    int g = grid;
+    if constexpr (O::staged) {
+      cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes);
+      g = std::max(1, std::min((grid * 128 + O::threads - 1) / O::threads, O::blocks * ql.num_sms));
+    }
+    kern<<<dim3(g, __builtin_popcount(m)), O::threads, bytes, s>>>(ql, m);
+  }
   if constexpr (P0 + PN < NPASS) launch_groups<LA, LB, LC, LD, NPASS, P0 + PN, MIXED, BATCH>(ql, live, grid, s);
 }
 
