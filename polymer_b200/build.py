@@ -15,7 +15,8 @@ CSRC = os.path.join(HERE, 'csrc')
 OUT = os.path.join(HERE, '_build')
 LIB = os.path.join(OUT, 'libpolymer_fock.so')
 # the largest units first: the pool starts them before the small ones
-SOURCES = ['pfe_mol_big2.cu', 'pfe_mol_big6.cu', 'pfe_mol_big4.cu', 'pfe_mol_big8.cu', 'pfe_mol_big3.cu',
+SOURCES = ['pfe_mol_big2.cu', 'pfe_mol_kept2.cu', 'pfe_mol_kept3.cu', 'pfe_mol_kept1.cu', 'pfe_mol_kept4.cu',
+           'pfe_mol_kept5.cu', 'pfe_mol_big6.cu', 'pfe_mol_big4.cu', 'pfe_mol_big8.cu', 'pfe_mol_big3.cu',
            'pfe_mol_big7.cu', 'pfe_mol_big1.cu', 'pfe_mol_big5.cu', 'pfe_mol.cu', 'pfe_mol_batch.cu',
            'pfe_mol_mixed.cu', 'pfe_mol_batch_mixed.cu', 'pfe_mol_wide.cu', 'pfe_mol_digest.cu', 'pfe_api.cu', 'pfe_eri.cu', 'pfe_lattice.cu', 'pfe_lattice_sl.cu', 'pfe_lattice_sl2.cu', 'pfe_lattice_sl3.cu', 'pfe_lattice_wide.cu',
            'pfe_grad.cu', 'pfe_onee.cu',

@@ -198,8 +198,8 @@ struct ClassLaunch {
   int wide_wpb, wide_per_warp, wide_vmax, wide_xmax;
   size_t smem_wide;
   int* queue;                // device work queue: one chunk counter per launch (pass), zeroed before each
-  int npass;                 // register passes of the straight-line variant
-  unsigned long long live;   // of which some component has a coefficient (live_passes)
+  int npass;                 // register passes of the straight-line variant (general; see pass_variant)
+  unsigned long long live;   // the passes launched: those with a component that has a coefficient
   int launches_live;         // its kernel launches: pass groups with a component that has a coefficient, digestion
   int gmul = 32;             // straight-line variant: persistent grid of up to gmul blocks per SM
 };

@@ -954,8 +954,13 @@ static void set_passes(ClassLaunch& cl, int bits) {
   cl.launches_live = 1;
   cl.live = 0;
   if (!cl.has_straight) return;
-  cl.live = live_passes(kCL[cl.cb][0], kCL[cl.cb][1], kCL[cl.ck][0], kCL[cl.ck][1], cl.npass, bits);
-  cl.launches_live = pass_groups(cl.npass, cl.live) + (cl.cb > 0 ? 1 : 0);
+  const int la = kCL[cl.cb][0], lb = kCL[cl.cb][1], lc = kCL[cl.ck][0], ld = kCL[cl.ck][1];
+  const int kept = pass_variant(la, lb, lc, ld, bits);
+  const int n = variant_passes(la, lb, lc, ld, kept, cl.npass);
+  // (every pass of a variant of kept components is live)
+  cl.live = kept == class_bits(la, lb, lc, ld) ? live_passes(la, lb, lc, ld, cl.npass, bits)
+                                               : (n < 64 ? (1ull << n) - 1 : ~0ull);
+  cl.launches_live = pass_groups(n, cl.live) + (cl.cb > 0 ? 1 : 0);
 }
 
 static int size_wide(ClassLaunch& cl, const int kept_max[3], const bool lower_kept[3]) {

@@ -1,0 +1,11 @@
+// The pass variants of kept components only of (21|21), single molecules and batches,
+// compiled apart so the build runs them in parallel.
+
+#define PFE_KEPT_UNIT
+#include "pfe_mol_kernels.cuh"
+
+namespace pfe {
+
+PFE_KEPT(2, 1, 2, 1, )
+
+}  // namespace pfe

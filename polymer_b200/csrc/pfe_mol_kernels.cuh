@@ -256,7 +256,35 @@ __host__ __device__ constexpr void pass_range(int LA, int LB, int LC, int LD, in
   ab1 = lsplit ? (pass == 0 ? nlow : NAB) : ((ab0 + abp < NAB) ? ab0 + abp : NAB);
 }
 
-// The register passes of a class that keep a bra component pair that can carry a
+// The angular momenta a class has, as lower_kept bits: KEPT of its general variant, which
+// keeps every component.
+__host__ __device__ constexpr int class_bits(int LA, int LB, int LC, int LD) {
+  return ((LA == 1 || LB == 1 || LC == 1 || LD == 1) ? 2 : 0) | ((LA == 2 || LB == 2 || LC == 2 || LD == 2) ? 4 : 0);
+}
+
+// The variant of a class's passes for a molecule's lower_kept bits: where the d shells (or,
+// without d shells in the class, the p shells) are pure, one that holds only the kept
+// components of all four shells in X, so that more integrals fit a pass and the recursion
+// runs less often ((21|21) of 6-31G**: 12 passes of 48 kept integrals for 24 of 40 with the
+// ket's ghosts among them); else the general one.
+__host__ __device__ constexpr int pass_variant(int LA, int LB, int LC, int LD, int bits) {
+  const int mask = class_bits(LA, LB, LC, LD), r = bits & mask;
+  return (mask & 4) ? ((r & 4) ? mask : r) : r;
+}
+
+// Register passes of a variant: kPassIntegrals kept integrals each.
+constexpr int kPassIntegrals = 48;
+__host__ __device__ constexpr int kept_pairs_per_pass(int LC, int LD, int KEPT) {
+  return kPassIntegrals / (kept_n(LC, KEPT) * kept_n(LD, KEPT)) > 0
+             ? kPassIntegrals / (kept_n(LC, KEPT) * kept_n(LD, KEPT)) : 1;
+}
+__host__ __device__ constexpr int variant_passes(int LA, int LB, int LC, int LD, int KEPT, int npass_general) {
+  if (KEPT == class_bits(LA, LB, LC, LD)) return npass_general;
+  const int per = kept_pairs_per_pass(LC, LD, KEPT);
+  return (kept_n(LA, KEPT) * kept_n(LB, KEPT) + per - 1) / per;
+}
+
+// The register passes of a class's general variant that keep a bra component pair that can carry a
 // coefficient (bit p of the mask): a component below its shell's top level has none
 // unless bit L of lower_kept_bits is set (the kernel skips such chunks anyway; a pass
 // that keeps none of them is not launched at all).
@@ -295,19 +323,38 @@ struct GqOccupancy {
   static constexpr int blocks = staged ? 2 : (LT <= 4 ? 3 : 1);
 };
 
-template <int LA, int LB, int LC, int LD, int NPASS, int PASS, bool MIXED, bool BATCH>
+template <int LA, int LB, int LC, int LD, int KEPT, int NPASS, int PASS, bool MIXED, bool BATCH>
 __device__ __forceinline__ void gq_pass(const MolLaunch& lq, const double2* s_boys) {
   constexpr int NA = ncum(LA), NB = ncum(LB), NC = ncum(LC), ND = ncum(LD);
   constexpr int NI = NA * NB * NC * ND;
-  constexpr int NAB = NA * NB;
   constexpr int NCD = NC * ND;
   constexpr int LT = LA + LB + LC + LD;
+  constexpr bool GENERAL = KEPT == class_bits(LA, LB, LC, LD);
   constexpr AbOrder<LA, LB> ORD{};
-  constexpr int AB0 = [] { int a = 0, b = 0; pass_range(LA, LB, LC, LD, NPASS, PASS, a, b); return a; }();
-  constexpr int AB1 = [] { int a = 0, b = 0; pass_range(LA, LB, LC, LD, NPASS, PASS, a, b); return b; }();
-  constexpr int XN = (AB1 - AB0) * NCD;
-  static_assert(AB0 < NAB, "every pass keeps at least one bra component pair");
-  // the pass keeps the pairs ab at positions [AB0, AB1) of ORD; X(k, cd) is pair ORD.ab[AB0 + k]
+  // the kept bra component pairs are the last of AbOrder (both shells' top levels, or the
+  // d shell's with all of the other's)
+  constexpr int NKP = kept_n(LA, KEPT) * kept_n(LB, KEPT), KP0 = NA * NB - NKP;
+  constexpr int FC = kept_first(LC, KEPT), FD = kept_first(LD, KEPT);
+  constexpr int NDK = kept_n(LD, KEPT), NCDK = kept_n(LC, KEPT) * NDK;
+  // the pass keeps the kept pairs [AB0, AB1); X(k, cd) is that of pair AB0 + k
+  constexpr int AB0 = [] {
+    int a = PASS * kept_pairs_per_pass(LC, LD, KEPT), b = 0;
+    if (GENERAL) pass_range(LA, LB, LC, LD, NPASS, PASS, a, b);
+    return a;
+  }();
+  constexpr int AB1 = [] {
+    int a = 0, b = (PASS + 1) * kept_pairs_per_pass(LC, LD, KEPT);
+    if (GENERAL) pass_range(LA, LB, LC, LD, NPASS, PASS, a, b);
+    return b < NKP ? b : NKP;
+  }();
+  constexpr int XN = (AB1 - AB0) * NCDK;
+  static_assert(AB0 < NKP, "every pass keeps at least one bra component pair");
+  // pair k's component pair, and the kept position of ket component pair (cc, d), or -1
+  auto ab_of = [&](int k) { return ORD.ab[KP0 + k]; };
+  auto cd_at = [&](int cc, int d) {
+    const int rc = comp_rank(LC, cc) - FC, rd = comp_rank(LD, d) - FD;
+    return (rc < 0 || rd < 0) ? -1 : rc * NDK + rd;
+  };
   const int lane = threadIdx.x & 31;
   const int nchunks = *lq.nchunks;
   const double c2pi = 2.0 / sqrt(REF_PI);
@@ -342,7 +389,7 @@ __device__ __forceinline__ void gq_pass(const MolLaunch& lq, const double2* s_bo
       bool live = false;
 #pragma unroll
       for (int k = AB0; k < AB1; ++k)
-        live = live || (stidx[ijg.x * MAXCOMP + ORD.ab[k] / NB] >= 0 && stidx[ijg.y * MAXCOMP + ORD.ab[k] % NB] >= 0);
+        live = live || (stidx[ijg.x * MAXCOMP + ab_of(k) / NB] >= 0 && stidx[ijg.y * MAXCOMP + ab_of(k) % NB] >= 0);
       if (!live) continue;
     }
     const int li = ch.first + lane;
@@ -379,8 +426,8 @@ __device__ __forceinline__ void gq_pass(const MolLaunch& lq, const double2* s_bo
       const int K = kq.si, L = kq.sj;
       const double wKL = (K != L) ? 2.0 : 1.0;
       // ket coefficients: products held when small, factors otherwise
-      constexpr bool HOLD = NCD <= 16;
-      double ccd[HOLD ? NCD : 1];
+      constexpr bool HOLD = NCDK <= 16;
+      double ccd[HOLD ? NCDK : 1];
       double sK[NC], sL[ND];
 #pragma unroll
       for (int cc = 0; cc < NC; ++cc) sK[cc] = scoef[K * MAXCOMP + cc];
@@ -390,7 +437,8 @@ __device__ __forceinline__ void gq_pass(const MolLaunch& lq, const double2* s_bo
 #pragma unroll
         for (int cc = 0; cc < NC; ++cc)
 #pragma unroll
-          for (int d = 0; d < ND; ++d) ccd[cc * ND + d] = wKL * sK[cc] * sL[d];
+          for (int d = 0; d < ND; ++d)
+            if (cd_at(cc, d) >= 0) ccd[cd_at(cc, d)] = wKL * sK[cc] * sL[d];
       }
       for (int p = g0 + ch.p0; p < g0 + ch.p1; ++p) {
         const PairView bp = load_pair(rec, p);
@@ -439,7 +487,7 @@ __device__ __forceinline__ void gq_pass(const MolLaunch& lq, const double2* s_bo
         const double w = ((I != J) ? 2.0 : 1.0) * ((p != q) ? 2.0 : 1.0);
 #pragma unroll
         for (int k = AB0; k < AB1; ++k) {
-          const double ca = w * scoef[I * MAXCOMP + ORD.ab[k] / NB] * scoef[J * MAXCOMP + ORD.ab[k] % NB];
+          const double ca = w * scoef[I * MAXCOMP + ab_of(k) / NB] * scoef[J * MAXCOMP + ab_of(k) % NB];
 #pragma unroll
           for (int cc = 0; cc < NC; ++cc) {
             double cb;
@@ -447,8 +495,11 @@ __device__ __forceinline__ void gq_pass(const MolLaunch& lq, const double2* s_bo
             else cb = ca * (wKL * sK[cc]);
 #pragma unroll
             for (int d = 0; d < ND; ++d) {
-              const double c4 = HOLD ? cb * ccd[cc * ND + d] : cb * sL[d];
-              X[(k - AB0) * NCD + cc * ND + d] = fma(c4, out[ORD.ab[k] * NCD + cc * ND + d], X[(k - AB0) * NCD + cc * ND + d]);
+              const int j = cd_at(cc, d);
+              if (j < 0) continue;
+              const double c4 = HOLD ? cb * ccd[HOLD ? j : 0] : cb * sL[d];
+              const int x = (k - AB0) * NCDK + j;
+              X[x] = fma(c4, out[ab_of(k) * NCD + cc * ND + d], X[x]);
             }
           }
         }
@@ -478,22 +529,22 @@ __device__ __forceinline__ void gq_pass(const MolLaunch& lq, const double2* s_bo
     } else {
       // this pass's part of X to the digestion kernel: the kept components, one
       // coalesced 256-byte row per integral
-      const int bits = lq.lower_kept_bits;
+      const int bits = GENERAL ? lq.lower_kept_bits : KEPT;
       const int fa = kept_first(LA, bits), fb = kept_first(LB, bits), fc = kept_first(LC, bits),
                 fd = kept_first(LD, bits);
       const int nb = NB - fb, nc = NC - fc, nd = ND - fd;
       double* __restrict__ xb = lq.xbuf + (size_t)t * ((size_t)(NA - fa) * nb * nc * nd * 32) + lane;
 #pragma unroll
       for (int k = AB0; k < AB1; ++k) {
-        const int ra = comp_rank(LA, ORD.ab[k] / NB) - fa, rb = comp_rank(LB, ORD.ab[k] % NB) - fb;
+        const int ra = comp_rank(LA, ab_of(k) / NB) - fa, rb = comp_rank(LB, ab_of(k) % NB) - fb;
         if (ra < 0 || rb < 0) continue;
 #pragma unroll
         for (int cc = 0; cc < NC; ++cc)
 #pragma unroll
           for (int d = 0; d < ND; ++d) {
             const int rc = comp_rank(LC, cc) - fc, rd = comp_rank(LD, d) - fd;
-            if (rc < 0 || rd < 0) continue;
-            xb[(((ra * nb + rb) * nc + rc) * nd + rd) * 32] = X[(k - AB0) * NCD + cc * ND + d];
+            if (rc < 0 || rd < 0 || cd_at(cc, d) < 0) continue;
+            xb[(((ra * nb + rb) * nc + rc) * nd + rd) * 32] = X[(k - AB0) * NCDK + cd_at(cc, d)];
           }
       }
       if (lane == 0) lq.xlive[t] = 1;
@@ -511,18 +562,18 @@ void launch_digest(int cb, int ck, const MolLaunch& ql, int num_sms, cudaStream_
 // launch-bound.
 constexpr int kPassGroup = 8;
 
-template <int LA, int LB, int LC, int LD, int NPASS, int P0, int PN, bool MIXED, bool BATCH>
+template <int LA, int LB, int LC, int LD, int KEPT, int NPASS, int P0, int PN, bool MIXED, bool BATCH>
 __device__ __forceinline__ void gq_select(const MolLaunch& lq, int p, const double2* s_boys) {
   if constexpr (PN == 1) {
-    gq_pass<LA, LB, LC, LD, NPASS, P0, MIXED, BATCH>(lq, s_boys);
+    gq_pass<LA, LB, LC, LD, KEPT, NPASS, P0, MIXED, BATCH>(lq, s_boys);
   } else {
-    if (p == P0) gq_pass<LA, LB, LC, LD, NPASS, P0, MIXED, BATCH>(lq, s_boys);
-    else gq_select<LA, LB, LC, LD, NPASS, P0 + 1, PN - 1, MIXED, BATCH>(lq, p, s_boys);
+    if (p == P0) gq_pass<LA, LB, LC, LD, KEPT, NPASS, P0, MIXED, BATCH>(lq, s_boys);
+    else gq_select<LA, LB, LC, LD, KEPT, NPASS, P0 + 1, PN - 1, MIXED, BATCH>(lq, p, s_boys);
   }
 }
 
 // Passes P0 .. P0 + PN - 1; blockIdx.y is the position among the live ones (bits of live).
-template <int LA, int LB, int LC, int LD, int NPASS, int P0, int PN, bool MIXED, bool BATCH>
+template <int LA, int LB, int LC, int LD, int KEPT, int NPASS, int P0, int PN, bool MIXED, bool BATCH>
 __global__ void __launch_bounds__(GqOccupancy<LA, LB, LC, LD>::threads, GqOccupancy<LA, LB, LC, LD>::blocks)
     k_gq(const __grid_constant__ MolLaunch lq, unsigned int live) {
   extern __shared__ double2 s_boys[];
@@ -532,18 +583,18 @@ __global__ void __launch_bounds__(GqOccupancy<LA, LB, LC, LD>::threads, GqOccupa
   }
   unsigned int m = live;
   for (int y = blockIdx.y; y > 0; --y) m &= m - 1;
-  gq_select<LA, LB, LC, LD, NPASS, P0, PN, MIXED, BATCH>(lq, P0 + __ffs(m) - 1, s_boys);
+  gq_select<LA, LB, LC, LD, KEPT, NPASS, P0, PN, MIXED, BATCH>(lq, P0 + __ffs(m) - 1, s_boys);
 }
 
 using LaunchFn = void (*)(const MolLaunch&, int grid, cudaStream_t);
 
-template <int LA, int LB, int LC, int LD, int NPASS, int P0, bool MIXED, bool BATCH>
+template <int LA, int LB, int LC, int LD, int KEPT, int NPASS, int P0, bool MIXED, bool BATCH>
 void launch_groups(const MolLaunch& ql, unsigned long long live, int grid, cudaStream_t s) {
   constexpr int PN = NPASS - P0 < kPassGroup ? NPASS - P0 : kPassGroup;
   using O = GqOccupancy<LA, LB, LC, LD>;
   const unsigned int m = (unsigned int)(live >> P0) & ((1u << PN) - 1);
   if (m) {
-    auto kern = k_gq<LA, LB, LC, LD, NPASS, P0, PN, MIXED, BATCH>;
+    auto kern = k_gq<LA, LB, LC, LD, KEPT, NPASS, P0, PN, MIXED, BATCH>;
     constexpr size_t bytes = DownSmem<O::LT>::BYTES;
     // `grid` counts blocks of four warps
     int g = grid;
@@ -553,13 +604,41 @@ void launch_groups(const MolLaunch& ql, unsigned long long live, int grid, cudaS
     }
     kern<<<dim3(g, __builtin_popcount(m)), O::threads, bytes, s>>>(ql, m);
   }
-  if constexpr (P0 + PN < NPASS) launch_groups<LA, LB, LC, LD, NPASS, P0 + PN, MIXED, BATCH>(ql, live, grid, s);
+  if constexpr (P0 + PN < NPASS) launch_groups<LA, LB, LC, LD, KEPT, NPASS, P0 + PN, MIXED, BATCH>(ql, live, grid, s);
 }
+
+// A variant that holds the kept components only (KEPT: 0 or 2); those of the large
+// classes are instantiated in units of their own (pfe_mol_kept*.cu).
+template <int LA, int LB, int LC, int LD, int KEPT, bool MIXED, bool BATCH>
+void launch_kept(const MolLaunch& ql, int grid, cudaStream_t s) {
+  launch_groups<LA, LB, LC, LD, KEPT, variant_passes(LA, LB, LC, LD, KEPT, 0), 0, MIXED, BATCH>(ql, ql.live, grid, s);
+}
+#define PFE_KEPT(A, B, C, D, WORD)                                                            \
+  WORD template void launch_kept<A, B, C, D, 0, false, false>(const MolLaunch&, int, cudaStream_t); \
+  WORD template void launch_kept<A, B, C, D, 0, false, true>(const MolLaunch&, int, cudaStream_t);  \
+  WORD template void launch_kept<A, B, C, D, 2, false, false>(const MolLaunch&, int, cudaStream_t); \
+  WORD template void launch_kept<A, B, C, D, 2, false, true>(const MolLaunch&, int, cudaStream_t);
+#ifndef PFE_KEPT_UNIT
+PFE_KEPT(2, 1, 1, 1, extern)
+PFE_KEPT(2, 1, 2, 0, extern)
+PFE_KEPT(2, 1, 2, 1, extern)
+PFE_KEPT(2, 2, 1, 0, extern)
+PFE_KEPT(2, 2, 1, 1, extern)
+PFE_KEPT(2, 2, 2, 0, extern)
+#endif
 
 template <int LA, int LB, int LC, int LD, int NPASS, bool MIXED, bool BATCH = false>
 void launch_q(const MolLaunch& ql, int grid, cudaStream_t s) {
   static_assert(NPASS <= 64, "a bit per pass");
-  launch_groups<LA, LB, LC, LD, NPASS, 0, MIXED, BATCH>(ql, ql.live, grid, s);
+  constexpr int ALL = class_bits(LA, LB, LC, LD);
+  const int kept = pass_variant(LA, LB, LC, LD, ql.lower_kept_bits);
+  if constexpr (ALL != 0) {
+    if (kept == 0) return launch_kept<LA, LB, LC, LD, 0, MIXED, BATCH>(ql, grid, s);
+  }
+  if constexpr (ALL == 6) {
+    if (kept == 2) return launch_kept<LA, LB, LC, LD, 2, MIXED, BATCH>(ql, grid, s);
+  }
+  launch_groups<LA, LB, LC, LD, ALL, NPASS, 0, MIXED, BATCH>(ql, ql.live, grid, s);
 }
 
 // Kernels launch_q launches for a class (groups with a live pass).
@@ -569,7 +648,7 @@ inline int pass_groups(int npass, unsigned long long live) {
   return n;
 }
 
-// Register passes per straight-line class; must match the table below.
+// Register passes per straight-line class's general variant; must match the table below.
 static inline int straight_npass(int cb, int ck) {
   static const int np[6][6] = {{1, 0, 0, 0, 0, 0}, {1, 1, 0, 0, 0, 0}, {1, 2, 8, 0, 0, 0},
                                {2, 2, 5, 3, 0, 0}, {1, 4, 14, 10, 40, 0}, {3, 10, 50, 25, 0, 0}};
