@@ -963,6 +963,14 @@ static void set_passes(ClassLaunch& cl, int bits) {
   cl.launches_live = pass_groups(n, cl.live) + (cl.cb > 0 ? 1 : 0);
 }
 
+// The table of group quartets whose bra shells keep their top-level components only.  For
+// (dd|dp) of a basis of pure d shells it drops the lower components of the ket's d shell
+// too (3079 operations in 1233 slots instead of 3827 in 1809 where the ket's p shell is an
+// sp shell, C20H42 6-31G**).
+static const OpTableHost* bra_table(int cb, int ck, bool lower_d) {
+  return (cb == 5 && ck == 4 && !lower_d) ? host_optable_topd(cb, ck) : host_optable_pure(cb, ck);
+}
+
 static int size_wide(ClassLaunch& cl, const int kept_max[3], const bool lower_kept[3]) {
   cl.has_wide = false;
   const WideVariant wv = wide_variant(cl.cb, cl.ck);
@@ -1314,6 +1322,7 @@ int molecular_setup(pfe_context* ctx, const pfe_args* a) {
     PFE_CUDA(cudaGetLastError());
     PFE_CUDA(cudaStreamSynchronize(s));
   }
+  free_pairs(ctx, &raw);   // gathered: free before the records and tiles are made
   PFE_CUDA(ctx->alloc((void**)&ctx->d_prec, sizeof(PairRec) * npairs));
   k_pack_pairs<<<nb256, 256, 0, s>>>(ctx->pairs, (PairRec*)ctx->d_prec, npairs);
   PFE_CUDA(cudaGetLastError());
@@ -1472,7 +1481,7 @@ int molecular_setup(pfe_context* ctx, const pfe_args* a) {
         cl.nlevels = d.nlevels; cl.nout = d.nout; cl.nslots = d.nslots;
         cl.ops_p = nullptr; cl.levels_p = nullptr; cl.out_p = nullptr; cl.nlevels_p = 0;
         cl.nslots_p = cl.nslots_p2 = 0;
-        if (const OpTableHost* hp = host_optable_pure(cb, ck)) {
+        if (const OpTableHost* hp = bra_table(cb, ck, ctx->lower_kept[2])) {
           OpTableDev dp{};
           if ((rc = upload_optable(ctx, hp, &dp)) != PFE_OK) return rc;
           if (dp.nslots <= d.nslots) {   // runs inside the full table's shared-memory layout
@@ -1539,7 +1548,6 @@ int molecular_setup(pfe_context* ctx, const pfe_args* a) {
     free_raw(ctx);
   }
   ctx->free_now(d_count);
-  free_pairs(ctx, &raw);
   for (void* p : {(void*)gbits, (void*)k_sch, (void*)k_gmax, (void*)k64, (void*)perm_a, (void*)perm_b, (void*)k32,
                   (void*)k32b, (void*)k8, (void*)k8b, (void*)head, (void*)gix, (void*)gr_cls, (void*)bkey,
                   (void*)bkey_sorted, (void*)giota})
@@ -1934,6 +1942,13 @@ int batch_setup(pfe_batch* b) {
         int bits = 0;
         for (pfe_context* c : b->inst) bits |= lower_kept_bits(c);
         set_passes(cl, bits);
+        if (cl.has_table && cl.ops_p && ((bits >> 2) & 1)) {   // some instance's d shells keep lower components
+          OpTableDev dp{};
+          const int rc = upload_optable(b->inst[0], bra_table(cb, ck, true), &dp);
+          if (rc != PFE_OK) return rc;
+          cl.ops_p = dp.ops; cl.levels_p = dp.levels; cl.out_p = dp.out; cl.nlevels_p = dp.nlevels;
+          cl.nslots_p = dp.nslots;
+        }
       }
       if (cl.has_wide) {   // the wide variant's working set must cover every instance
         int km[3] = {1, 1, 1};
