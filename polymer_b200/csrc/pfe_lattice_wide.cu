@@ -12,8 +12,9 @@
 // do the whole class.  Besides, every lane evaluates the Boys values and the geometry
 // itself, tickets are single (bra, ket) pairs instead of 32 kets, and the output slots are
 // listed once per ticket for all image cells.
-// Measured (B200), helical polyethylene 6-31G**, CUTOFF1/2 = 1/2: see the table at
-// lattice_wide_launcher.
+// Measured (B200), helical polyethylene 6-31G**, CUTOFF1/2 = 1/2, both orders of the
+// classes, against the interpreter of every component: (22|21) 7.8 -> 0.28 ms, (22|11) 3.4
+// -> 0.35, (21|11) 4.1 -> 1.9, (22|22) 1.8 -> 0.21; the build 39.8 -> 14.5 ms.
 
 #include <algorithm>
 

@@ -14,7 +14,9 @@
 //     lanes along the elements of a block;
 //   * the bra is the warp's, so J'(ab) is summed over the lanes first.
 // The multiply-adds (six per integral) run per lane from registers.
-// Measured, C20H42 6-31G** (B200): see the figures at launch_digest.
+// Measured, C20H42 6-31G** (B200): (21|11) 2.9 ms inside its nine passes, 0.7 ms here;
+// (11|10) 2.4 and 0.9 ms; all classes 17 and 8 ms, of which the stored integrals' traffic
+// (written and read once) is about 1 ms.
 
 #include <algorithm>
 
