@@ -237,6 +237,9 @@ static void reset_context(pfe_context* ctx) {
   ctx->tuned = false;
 }
 
+// Every copy, clear and kernel of a set-up is issued on the context's stream, which a build
+// stream does not wait for (both are non-blocking, and so is the legacy stream to them): the
+// wait at the end orders them.
 static int setup_impl(pfe_context* ctx, const pfe_args* a, const HostShells& hs, uint64_t key) {
   int rc;
   PFE_CUDA(cudaSetDevice(ctx->device));
@@ -303,14 +306,16 @@ static int setup_impl(pfe_context* ctx, const pfe_args* a, const HostShells& hs,
     for (int p = 0; p < a->npgs; ++p)
       for (int r = 0; r < a->ncgs; ++r) maxc[p] = std::max(maxc[p], std::fabs(a->cc[r + (size_t)a->ncgs * p]));
     PFE_CUDA(ctx->alloc((void**)&ctx->d_maxc, sizeof(double) * a->npgs));
-    PFE_CUDA(cudaMemcpy(ctx->d_maxc, maxc.data(), sizeof(double) * a->npgs, cudaMemcpyHostToDevice));
+    PFE_CUDA(cudaMemcpyAsync(ctx->d_maxc, maxc.data(), sizeof(double) * a->npgs, cudaMemcpyHostToDevice, s));
     PFE_CUDA(ctx->alloc((void**)&ctx->d_cc, sizeof(double) * (size_t)a->ncgs * a->npgs));
-    PFE_CUDA(cudaMemcpy(ctx->d_cc, a->cc, sizeof(double) * (size_t)a->ncgs * a->npgs, cudaMemcpyHostToDevice));
+    PFE_CUDA(cudaMemcpyAsync(ctx->d_cc, a->cc, sizeof(double) * (size_t)a->ncgs * a->npgs, cudaMemcpyHostToDevice,
+                             s));
   }
   if (a->helix != 0.0) {
     const int nq = 2 * (a->cel2[0] + a->cel1[0]) + 1;
     PFE_CUDA(ctx->alloc((void**)&ctx->d_c2h, sizeof(double) * (size_t)a->ncgs * a->ncgs * nq));
-    PFE_CUDA(cudaMemcpy(ctx->d_c2h, a->c2h, sizeof(double) * (size_t)a->ncgs * a->ncgs * nq, cudaMemcpyHostToDevice));
+    PFE_CUDA(cudaMemcpyAsync(ctx->d_c2h, a->c2h, sizeof(double) * (size_t)a->ncgs * a->ncgs * nq,
+                             cudaMemcpyHostToDevice, s));
   }
   // digestion targets and contracted blocks
   {
@@ -391,15 +396,15 @@ static int setup_impl(pfe_context* ctx, const pfe_args* a, const HostShells& hs,
       }
       PFE_CUDA(ctx->alloc((void**)&ctx->d_scoef, sizeof(double) * scoef.size()));
       PFE_CUDA(ctx->alloc((void**)&ctx->d_stidx, sizeof(int) * stidx.size()));
-      PFE_CUDA(cudaMemcpy(ctx->d_scoef, scoef.data(), sizeof(double) * scoef.size(), cudaMemcpyHostToDevice));
-      PFE_CUDA(cudaMemcpy(ctx->d_stidx, stidx.data(), sizeof(int) * stidx.size(), cudaMemcpyHostToDevice));
+      PFE_CUDA(cudaMemcpyAsync(ctx->d_scoef, scoef.data(), sizeof(double) * scoef.size(), cudaMemcpyHostToDevice, s));
+      PFE_CUDA(cudaMemcpyAsync(ctx->d_stidx, stidx.data(), sizeof(int) * stidx.size(), cudaMemcpyHostToDevice, s));
     }
     PFE_CUDA(ctx->alloc((void**)&ctx->d_tidx, sizeof(int) * a->npgs));
     PFE_CUDA(ctx->alloc((void**)&ctx->d_tcoef, sizeof(double) * a->npgs));
     PFE_CUDA(ctx->alloc((void**)&ctx->d_blk, sizeof(int) * a->npshell));
-    PFE_CUDA(cudaMemcpy(ctx->d_tidx, tidx.data(), sizeof(int) * a->npgs, cudaMemcpyHostToDevice));
-    PFE_CUDA(cudaMemcpy(ctx->d_tcoef, tcoef.data(), sizeof(double) * a->npgs, cudaMemcpyHostToDevice));
-    PFE_CUDA(cudaMemcpy(ctx->d_blk, blk.data(), sizeof(int) * a->npshell, cudaMemcpyHostToDevice));
+    PFE_CUDA(cudaMemcpyAsync(ctx->d_tidx, tidx.data(), sizeof(int) * a->npgs, cudaMemcpyHostToDevice, s));
+    PFE_CUDA(cudaMemcpyAsync(ctx->d_tcoef, tcoef.data(), sizeof(double) * a->npgs, cudaMemcpyHostToDevice, s));
+    PFE_CUDA(cudaMemcpyAsync(ctx->d_blk, blk.data(), sizeof(int) * a->npshell, cudaMemcpyHostToDevice, s));
     // representative primitive of every target (largest |coefficient|): P_C(mu,nu) is read
     // off P_P at the representatives of mu and nu
     std::vector<int> rep(ctx->nt, -1);
@@ -416,16 +421,16 @@ static int setup_impl(pfe_context* ctx, const pfe_args* a, const HostShells& hs,
         if (t >= 0) tblk[t] = blk[sh];
       }
     PFE_CUDA(ctx->alloc((void**)&ctx->d_tblk, sizeof(int) * ctx->nt));
-    PFE_CUDA(cudaMemcpy(ctx->d_tblk, tblk.data(), sizeof(int) * ctx->nt, cudaMemcpyHostToDevice));
+    PFE_CUDA(cudaMemcpyAsync(ctx->d_tblk, tblk.data(), sizeof(int) * ctx->nt, cudaMemcpyHostToDevice, s));
     PFE_CUDA(ctx->alloc((void**)&ctx->d_bmax, sizeof(double) * (size_t)ctx->nblk * ctx->nblk));
     PFE_CUDA(ctx->alloc((void**)&ctx->d_n32, sizeof(unsigned long long)));
-    PFE_CUDA(cudaMemset(ctx->d_n32, 0, sizeof(unsigned long long)));
+    PFE_CUDA(cudaMemsetAsync(ctx->d_n32, 0, sizeof(unsigned long long), s));
     PFE_CUDA(ctx->alloc((void**)&ctx->d_rep, sizeof(int) * ctx->nt));
     PFE_CUDA(ctx->alloc((void**)&ctx->d_repc, sizeof(double) * ctx->nt));
     PFE_CUDA(ctx->alloc((void**)&ctx->d_pt, sizeof(double) * (size_t)ctx->nt * ctx->nt));
     PFE_CUDA(ctx->alloc((void**)&ctx->d_flag, sizeof(unsigned int)));
-    PFE_CUDA(cudaMemcpy(ctx->d_rep, rep.data(), sizeof(int) * ctx->nt, cudaMemcpyHostToDevice));
-    PFE_CUDA(cudaMemcpy(ctx->d_repc, repc.data(), sizeof(double) * ctx->nt, cudaMemcpyHostToDevice));
+    PFE_CUDA(cudaMemcpyAsync(ctx->d_rep, rep.data(), sizeof(int) * ctx->nt, cudaMemcpyHostToDevice, s));
+    PFE_CUDA(cudaMemcpyAsync(ctx->d_repc, repc.data(), sizeof(double) * ctx->nt, cudaMemcpyHostToDevice, s));
   }
   // accumulators and GEMM scratch
   const size_t pp = (size_t)a->npgs * a->npgs * ctx->ncell1;
@@ -435,6 +440,8 @@ static int setup_impl(pfe_context* ctx, const pfe_args* a, const HostShells& hs,
   PFE_CUDA(ctx->alloc((void**)&ctx->d_w2, sizeof(double) * (size_t)a->ncgs * a->ncgs * ctx->ncell1));
   rc = ctx->molecular ? molecular_setup(ctx, a) : lattice_setup(ctx, a);
   if (rc != PFE_OK) return rc;
+  // builds run on other streams: nothing of the set-up may still be on its way
+  PFE_CUDA(cudaStreamSynchronize(s));
   ctx->key = key;
   ctx->ready = true;
   return PFE_OK;

@@ -234,10 +234,13 @@ int upload_optable(pfe_context* ctx, const OpTableHost* h, OpTableDev* d) {
     std::vector<unsigned short> rec((size_t)8 * (h->nops + 1), 0);
     for (int o = 0; o < h->nops; ++o)
       for (int k = 0; k < 7; ++k) rec[(size_t)8 * o + k] = h->ops[(size_t)7 * o + k];
-    PFE_CUDA(cudaMemcpy(ops, rec.data(), sizeof(unsigned short) * rec.size(), cudaMemcpyHostToDevice));
+    PFE_CUDA(cudaMemcpyAsync(ops, rec.data(), sizeof(unsigned short) * rec.size(), cudaMemcpyHostToDevice,
+                             ctx->stream));
   }
-  PFE_CUDA(cudaMemcpy(out, h->out, sizeof(unsigned short) * h->nout, cudaMemcpyHostToDevice));
-  PFE_CUDA(cudaMemcpy(lev, h->levels, sizeof(int) * (h->nlevels + 1), cudaMemcpyHostToDevice));
+  PFE_CUDA(cudaMemcpyAsync(out, h->out, sizeof(unsigned short) * h->nout, cudaMemcpyHostToDevice, ctx->stream));
+  PFE_CUDA(cudaMemcpyAsync(lev, h->levels, sizeof(int) * (h->nlevels + 1), cudaMemcpyHostToDevice,
+                           ctx->stream));
+  PFE_CUDA(cudaStreamSynchronize(ctx->stream));   // the kernels that read them run on any stream
   d->ops = ops;
   d->out = out;
   d->levels = lev;

@@ -555,7 +555,7 @@ int lattice_setup(pfe_context* ctx, const pfe_args* a) {
   PFE_CUDA(ctx->alloc((void**)&L->d_queue, sizeof(int) * 64 * kLatQueueSlots));
   if (!ctx->d_n32) {   // FP32 quartet counter of the mixed-precision path
     PFE_CUDA(ctx->alloc((void**)&ctx->d_n32, sizeof(unsigned long long)));
-    PFE_CUDA(cudaMemset(ctx->d_n32, 0, sizeof(unsigned long long)));
+    PFE_CUDA(cudaMemsetAsync(ctx->d_n32, 0, sizeof(unsigned long long), s));
   }
   const LatGeom g = make_geom(ctx);
   const int n = ctx->npshell;
@@ -576,7 +576,8 @@ int lattice_setup(pfe_context* ctx, const pfe_args* a) {
     return (qx + ctx->rc1[0]) + nx * ((qy + ctx->rc1[1]) + ny * (qz + ctx->rc1[2]));
   };
   PFE_CUDA(ctx->alloc((void**)&L->d_qcell, sizeof(int) * L->qcell.size()));
-  PFE_CUDA(cudaMemcpy(L->d_qcell, L->qcell.data(), sizeof(int) * L->qcell.size(), cudaMemcpyHostToDevice));
+  PFE_CUDA(cudaMemcpyAsync(L->d_qcell, L->qcell.data(), sizeof(int) * L->qcell.size(), cudaMemcpyHostToDevice,
+                           s));
   int rc;
   PairArrays raw{};
   if ((rc = alloc_pairs(ctx, &raw, ntot)) != PFE_OK) return rc;
@@ -629,7 +630,8 @@ int lattice_setup(pfe_context* ctx, const pfe_args* a) {
     std::vector<int> cnt(6, 0);
     std::vector<int> L_sh(n);
     for (int i = 0; i < n; ++i) L_sh[i] = 0;
-    PFE_CUDA(cudaMemcpy(L_sh.data(), ctx->shells.L, sizeof(int) * n, cudaMemcpyDeviceToHost));
+    PFE_CUDA(cudaMemcpyAsync(L_sh.data(), ctx->shells.L, sizeof(int) * n, cudaMemcpyDeviceToHost, s));
+    PFE_CUDA(cudaStreamSynchronize(s));
     for (int I = 0; I < n; ++I)
       for (int J = 0; J < n; ++J) {
         const int la = std::max(L_sh[I], L_sh[J]), lb = std::min(L_sh[I], L_sh[J]);
@@ -660,7 +662,7 @@ int lattice_setup(pfe_context* ctx, const pfe_args* a) {
   }
   if (L->ntk == 0) { L->nlaunch = 0; return PFE_OK; }
   PFE_CUDA(ctx->alloc((void**)&L->d_tickets, sizeof(int4) * L->ntk));
-  PFE_CUDA(cudaMemcpy(L->d_tickets, L->h_tickets.data(), sizeof(int4) * L->ntk, cudaMemcpyHostToDevice));
+  PFE_CUDA(cudaMemcpyAsync(L->d_tickets, L->h_tickets.data(), sizeof(int4) * L->ntk, cudaMemcpyHostToDevice, s));
   // the reference's bra bounds per ticket
   {
     const long long nj = (long long)L->ntk * L->npl;

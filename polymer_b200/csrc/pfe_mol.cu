@@ -1042,7 +1042,7 @@ static PanelView panel_view(const pfe_context* c) {
 
 // The block panels of a molecule whose shells of top L keep their lower components
 // where bit L of `bits` says so (a batch: where any of its molecules needs them).
-static int build_panels(pfe_context* ctx, int bits) {
+static int build_panels(pfe_context* ctx, int bits, cudaStream_t s) {
   const int nblk = ctx->nblk;
   std::vector<int> first(nblk + 1, 0);
   for (int b = 0; b < nblk; ++b) first[b + 1] = first[b] + kept_n(ctx->h_blk_L[b], bits);
@@ -1058,7 +1058,7 @@ static int build_panels(pfe_context* ctx, int bits) {
       rown[p] = first[b + 1] - first[b];
     }
   }
-  for (int s = 0; s < ctx->npshell; ++s) poff[s] = first[ctx->h_blk[s]];
+  for (int sh = 0; sh < ctx->npshell; ++sh) poff[sh] = first[ctx->h_blk[sh]];
   for (int p = 0; p < np; ++p)
     if (tgt[p] >= 0) ++inv[tgt[p] + 1];
   for (int t = 0; t < ctx->nt; ++t) inv[t + 1] += inv[t];
@@ -1070,7 +1070,8 @@ static int build_panels(pfe_context* ctx, int bits) {
   }
   auto put = [&](auto** d, const auto& v) -> cudaError_t {
     cudaError_t e = ctx->alloc((void**)d, sizeof(v[0]) * v.size());
-    return e != cudaSuccess ? e : cudaMemcpy(*d, v.data(), sizeof(v[0]) * v.size(), cudaMemcpyHostToDevice);
+    return e != cudaSuccess ? e
+                            : cudaMemcpyAsync(*d, v.data(), sizeof(v[0]) * v.size(), cudaMemcpyHostToDevice, s);
   };
   PFE_CUDA(put(&ctx->d_poff, poff));
   PFE_CUDA(put(&ctx->d_ptgt, tgt));
@@ -1098,7 +1099,7 @@ static int kept_integrals(int cb, int ck, int bits) {
 // do not show, and the buffer's traffic (written and read once, at HBM rate) is a tenth
 // of what the digestion inside every pass cost.
 template <typename Owner>
-static int alloc_integrals(Owner* own, ClassLaunch* launches, int nlaunch, int bits) {
+static int alloc_integrals(Owner* own, ClassLaunch* launches, int nlaunch, int bits, cudaStream_t s) {
   constexpr size_t kTileBytes = (size_t)1 << 30, kTogetherBytes = (size_t)1 << 30;
   auto bytes_per = [&](const ClassLaunch& cl) {
     return sizeof(double) * 32 * (size_t)kept_integrals(cl.cb, cl.ck, bits);
@@ -1121,7 +1122,7 @@ static int alloc_integrals(Owner* own, ClassLaunch* launches, int nlaunch, int b
     const size_t flags = own->concurrent ? sum_flags : most_flags;
     PFE_CUDA(own->alloc_kept((void**)&x, own->concurrent ? sum : most));
     PFE_CUDA(own->alloc((void**)&f, flags));
-    PFE_CUDA(cudaMemset(f, 0, flags));
+    PFE_CUDA(cudaMemsetAsync(f, 0, flags, s));
   }
   size_t xo = 0, fo = 0;
   for (int i = 0; i < nlaunch; ++i) {
@@ -1327,7 +1328,8 @@ int molecular_setup(pfe_context* ctx, const pfe_args* a) {
   k_pack_pairs<<<nb256, 256, 0, s>>>(ctx->pairs, (PairRec*)ctx->d_prec, npairs);
   PFE_CUDA(cudaGetLastError());
   int hcount[8] = {0};
-  PFE_CUDA(cudaMemcpy(hcount, d_count, sizeof(int) * 8, cudaMemcpyDeviceToHost));
+  PFE_CUDA(cudaMemcpyAsync(hcount, d_count, sizeof(int) * 8, cudaMemcpyDeviceToHost, s));
+  PFE_CUDA(cudaStreamSynchronize(s));
   int off = 0;
   for (int c = 0; c < 6; ++c) {
     ctx->class_off[c] = off;
@@ -1542,9 +1544,9 @@ int molecular_setup(pfe_context* ctx, const pfe_args* a) {
   if (!ctx->in_batch) {
     pfe_context* const self = ctx;
     if ((rc = finish_chunks(ctx, &self, 1, ctx->launches, ctx->nlaunch, s)) != PFE_OK) return rc;
-    if ((rc = build_panels(ctx, lower_kept_bits(ctx))) != PFE_OK) return rc;
+    if ((rc = build_panels(ctx, lower_kept_bits(ctx), s)) != PFE_OK) return rc;
     if ((rc = ensure_side(ctx)) != PFE_OK) return rc;
-    if ((rc = alloc_integrals(ctx, ctx->launches, ctx->nlaunch, lower_kept_bits(ctx))) != PFE_OK) return rc;
+    if ((rc = alloc_integrals(ctx, ctx->launches, ctx->nlaunch, lower_kept_bits(ctx), s)) != PFE_OK) return rc;
     free_raw(ctx);
   }
   ctx->free_now(d_count);
@@ -1971,17 +1973,17 @@ int batch_setup(pfe_batch* b) {
   for (pfe_context* c : b->inst) bits |= lower_kept_bits(c);
   for (pfe_context* c : b->inst) {
     free_raw(c);   // the joined lists replace them
-    const int rc = build_panels(c, bits);
+    const int rc = build_panels(c, bits, st);
     if (rc != PFE_OK) return rc;
   }
   {
-    int rc = alloc_integrals(b, b->launches, b->nlaunch, bits);
+    int rc = alloc_integrals(b, b->launches, b->nlaunch, bits, st);
     if (rc == PFE_OK) rc = ensure_side(b->inst[0]);
     if (rc != PFE_OK) return rc;
   }
   PFE_CUDA(b->alloc(&b->d_insts, (sizeof(MolLaunch) + sizeof(PanelView)) * b->inst.size()));
   PFE_CUDA(b->alloc((void**)&b->d_off, sizeof(long long) * b->off.size()));
-  PFE_CUDA(cudaMemcpy(b->d_off, b->off.data(), sizeof(long long) * b->off.size(), cudaMemcpyHostToDevice));
+  PFE_CUDA(cudaMemcpyAsync(b->d_off, b->off.data(), sizeof(long long) * b->off.size(), cudaMemcpyHostToDevice, st));
   b->all_contracted = true;
   for (pfe_context* c : b->inst) b->all_contracted = b->all_contracted && c->contracted;
   PFE_CUDA(cudaMallocHost(&b->h_insts, (sizeof(MolLaunch) + sizeof(PanelView)) * b->inst.size()));
