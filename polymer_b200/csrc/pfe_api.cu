@@ -952,8 +952,18 @@ int32_t pfe_fourindex_eri_gradient(const pfe_args* a, const int32_t* pgs_atom, i
     ctx->pp_bytes = npp * sizeof(double);
   }
   PFE_CUDA(cudaMemcpyAsync(ctx->d_pp, a->p_p, npp * sizeof(double), cudaMemcpyHostToDevice, s));
-  int* d_satom = nullptr;
-  double* d_g = nullptr;
+  struct Scratch {   // given back on every way out, after a wait for the work on it
+    pfe_context* ctx;
+    int* d_satom = nullptr;
+    double* d_g = nullptr;
+    ~Scratch() {
+      cudaStreamSynchronize(ctx->stream);
+      ctx->free_now(d_satom);
+      ctx->free_now(d_g);
+    }
+  } scratch{ctx};
+  int*& d_satom = scratch.d_satom;
+  double*& d_g = scratch.d_g;
   PFE_CUDA(ctx->alloc((void**)&d_satom, sizeof(int) * a->npshell));
   PFE_CUDA(ctx->alloc((void**)&d_g, sizeof(double) * 6 * (size_t)natom));
   PFE_CUDA(cudaMemcpyAsync(d_satom, satom.data(), sizeof(int) * a->npshell, cudaMemcpyHostToDevice, s));
@@ -968,11 +978,8 @@ int32_t pfe_fourindex_eri_gradient(const pfe_args* a, const int32_t* pgs_atom, i
     PFE_CUDA(cudaMemcpyAsync(grad_j, d_g, sizeof(double) * 3 * (size_t)natom, cudaMemcpyDeviceToHost, s));
     PFE_CUDA(cudaMemcpyAsync(grad_k, d_g + 3 * (size_t)natom, sizeof(double) * 3 * (size_t)natom,
                              cudaMemcpyDeviceToHost, s));
-    PFE_CUDA(cudaStreamSynchronize(s));
   }
   PFE_CUDA(cudaStreamSynchronize(s));
-  ctx->free_now(d_satom);
-  ctx->free_now(d_g);
   return rc;
 }
 

@@ -8,7 +8,9 @@
 #include <cuda_runtime.h>
 
 #include <cstdint>
+#include <map>
 #include <memory>
+#include <unordered_map>
 #include <vector>
 
 #include "pfe_common.cuh"
@@ -46,23 +48,33 @@ int acquire_boys(int device, const double* igamma, cudaStream_t s, std::shared_p
 // Device memory of a context or batch.  Requests of up to kSmall bytes are cut from
 // blocks that are kept from one set-up to the next (a set-up makes over a hundred, and
 // cudaMalloc and cudaFree were most of a small molecule's: 1.1 of 2.6 ms); larger ones,
-// and small ones beyond kBlocks blocks, are allocations of their own, but for one buffer
-// of up to kKept bytes (`kept`) that also stays.  All of it is freed with the owner.  A block's memory may still be read by a build in flight when the
-// next set-up begins, so release_all waits for the device, as cudaFree does.
+// and small ones that no block has room for, are allocations of their own, but for one
+// buffer of up to kKept bytes (`kept`) that also stays.  A piece that free_now gives back
+// is cut again for the requests that follow, so scratch does not add up: the work on it
+// must be ordered before theirs (a set-up's work is all on one stream; other callers wait
+// first).  Kept at most: 13.5 MiB of blocks (512 KiB, 1 MiB, then 2 MiB each; one water
+// molecule takes the first two) and the 64 MiB buffer; all of it is freed with the owner.  A block's memory may
+// still be read by a build in flight when the next set-up begins, so release_all waits
+// for the device, as cudaFree does.
 struct DeviceMemory {
-  static constexpr size_t kSmall = 256 << 10, kBlock = 2 << 20;
+  static constexpr size_t kSmall = 256 << 10, kFirst = 512 << 10, kBlock = 2 << 20, kKept = 64 << 20;
   static constexpr int kBlocks = 8;
+  struct Block {
+    char* p;
+    size_t n;
+  };
   std::vector<void*> owned;    // allocations of their own
-  std::vector<char*> blocks;
-  size_t block = 0, offset = 0;   // the next small request: blocks[block] + offset
-  static constexpr size_t kKept = 64 << 20;
+  std::vector<Block> blocks;
+  size_t block = 0, offset = 0;             // the next uncut byte: blocks[block].p + offset
+  std::unordered_map<void*, size_t> cut;    // pieces in use
+  std::multimap<size_t, char*> spare;       // pieces to cut from first, by size
   void* kept = nullptr;
   size_t kept_bytes = 0;
   DeviceMemory() = default;
   DeviceMemory(const DeviceMemory&) = delete;
   DeviceMemory& operator=(const DeviceMemory&) = delete;
   ~DeviceMemory() {
-    for (char* b : blocks) cudaFree(b);
+    for (const Block& b : blocks) cudaFree(b.p);
     cudaFree(kept);
   }
 
@@ -70,19 +82,31 @@ struct DeviceMemory {
     if (cudaError_t f = injected_alloc_failure()) return f;
     const size_t n = (std::max<size_t>(bytes, 1) + 255) & ~size_t(255);
     if (n <= kSmall) {
-      if (block < blocks.size() && offset + n > kBlock) {
+      const auto it = spare.lower_bound(n);
+      if (it != spare.end()) {
+        char* q = it->second;
+        const size_t left = it->first - n;
+        spare.erase(it);
+        if (left > 0) spare.emplace(left, q + n);
+        cut[q] = n;
+        *p = q;
+        return cudaSuccess;
+      }
+      if (block < blocks.size() && offset + n > blocks[block].n) {
+        if (offset < blocks[block].n) spare.emplace(blocks[block].n - offset, blocks[block].p + offset);
         ++block;
         offset = 0;
       }
       if (block == blocks.size() && blocks.size() < (size_t)kBlocks) {
-        char* b = nullptr;
-        const cudaError_t e = cudaMalloc((void**)&b, kBlock);
+        Block b{nullptr, std::min(kBlock, kFirst << blocks.size())};
+        const cudaError_t e = cudaMalloc((void**)&b.p, b.n);
         if (e != cudaSuccess) return e;
         blocks.push_back(b);
       }
       if (block < blocks.size()) {
-        *p = blocks[block] + offset;
+        *p = blocks[block].p + offset;
         offset += n;
+        cut[*p] = n;
         return cudaSuccess;
       }
     }
@@ -105,9 +129,15 @@ struct DeviceMemory {
     *p = kept;
     return cudaSuccess;
   }
-  // (memory cut from a block stays taken until release_all)
   void free_now(void* p) {
-    for (size_t i = 0; p && i < owned.size(); ++i)
+    if (!p) return;
+    const auto it = cut.find(p);
+    if (it != cut.end()) {
+      spare.emplace(it->second, (char*)p);
+      cut.erase(it);
+      return;
+    }
+    for (size_t i = 0; i < owned.size(); ++i)
       if (owned[i] == p) {
         owned.erase(owned.begin() + i);
         cudaFree(p);
@@ -118,6 +148,8 @@ struct DeviceMemory {
     if (block > 0 || offset > 0 || kept) cudaDeviceSynchronize();
     for (void* p : owned) cudaFree(p);
     owned.clear();
+    cut.clear();
+    spare.clear();
     block = offset = 0;
   }
 };
