@@ -424,6 +424,41 @@ inline bool ensure_blas(pfe_context* ctx) {
   return true;
 }
 int ensure_side(pfe_context* ctx);
+
+// Work of a build on the context's side streams (bit k of `used`: side[k]), forked from
+// stream s and joined back to it on every way out: after an error too, later work on s
+// waits for what was launched, and a stream capture ends with no stream unjoined.
+class SideFork {
+ public:
+  SideFork(pfe_context* cx, cudaStream_t s) : cx_(cx), s_(s) {}
+  ~SideFork() { join(); }
+  cudaError_t fork(unsigned int used) {
+    if (!used) return cudaSuccess;
+    cudaError_t e = cudaEventRecord(cx_->ev_fork, s_);
+    for (int k = 0; k < pfe_context::kSide && e == cudaSuccess; ++k) {
+      if (!((used >> k) & 1)) continue;
+      e = cudaStreamWaitEvent(cx_->side[k], cx_->ev_fork, 0);
+      if (e == cudaSuccess) forked_ |= 1u << k;
+    }
+    return e;
+  }
+  cudaError_t join() {
+    cudaError_t first = cudaSuccess;
+    for (int k = 0; k < pfe_context::kSide; ++k) {
+      if (!((forked_ >> k) & 1)) continue;
+      cudaError_t e = cudaEventRecord(cx_->ev_join[k], cx_->side[k]);
+      if (e == cudaSuccess) e = cudaStreamWaitEvent(s_, cx_->ev_join[k], 0);
+      if (first == cudaSuccess) first = e;
+    }
+    forked_ = 0;
+    return first;
+  }
+
+ private:
+  pfe_context* cx_;
+  cudaStream_t s_;
+  unsigned int forked_ = 0;
+};
 int batch_setup(pfe_batch* b);
 int batch_fock_pc(pfe_batch* b, const double* d_pc, double* d_cc, double* d_xc, cudaStream_t s);
 int batch_refresh(pfe_batch* b, const double* d_pc);

@@ -227,6 +227,7 @@ int upload_optable(pfe_context* ctx, const OpTableHost* h, OpTableDev* d) {
   }
   unsigned short *ops = nullptr, *out = nullptr;
   int* lev = nullptr;
+  if (cudaError_t f = injected_alloc_failure()) PFE_CUDA(f);
   PFE_CUDA(cudaMalloc((void**)&ops, sizeof(unsigned short) * 8 * (h->nops + 1)));
   PFE_CUDA(cudaMalloc((void**)&out, sizeof(unsigned short) * (h->nout ? h->nout : 1)));
   PFE_CUDA(cudaMalloc((void**)&lev, sizeof(int) * (h->nlevels + 1)));

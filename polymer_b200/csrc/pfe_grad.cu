@@ -353,52 +353,65 @@ GradClass grad_class(int cb, int ck) {
 // (overwritten).  satom: shell -> atom on the device.
 int molecular_gradient(pfe_context* ctx, const double* d_dt, const int* d_satom, int natom, double* d_gj,
                        double* d_gk, cudaStream_t s) {
+  // what can fail comes first: the tables' uploads, the launch shapes and the attributes
+  struct Launch {
+    GradFn fn;
+    GradTables t;
+    const ClassLaunch* cl;
+    int vmax, per_team, grid, threads, side;
+    size_t smem;
+  };
+  Launch launch[64];
+  int n = 0;
+  for (int i = ctx->nlaunch - 1; i >= 0; --i) {   // the classes of the longest quartets first
+    const ClassLaunch& cl = ctx->launches[i];
+    const GradClass gc = grad_class(cl.cb, cl.ck);
+    if (!gc.warp) { set_error("no gradient kernel for a quartet class"); return PFE_EUNSUPPORTED; }
+    Launch& g = launch[n++];
+    g = Launch{};
+    for (int k = 0; k < 3; ++k) {
+      const int rc = upload_optable(ctx, gc.tab[k], &g.t.t[k]);
+      if (rc != PFE_OK) return rc;
+      g.vmax = std::max(g.vmax, gc.tab[k]->nslots);
+    }
+    // a warp per quartet where at least kWarpTeams fit an SM's shared memory, else a block
+    constexpr int kWarpTeams = 8;
+    g.per_team = g.vmax + gc.np;
+    const size_t one = sizeof(double) * (size_t)g.per_team, sm = 220 * 1024;
+    const bool warp = one * kWarpTeams <= sm;
+    const long long tickets = 32ll * cl.nchunks_host;
+    int teams = 1;   // per block
+    if (warp) teams = (int)std::min<size_t>(8, std::max<size_t>(1, sm / 4 / one));
+    g.smem = one * teams;
+    if (g.smem > 227 * 1024) { set_error("gradient op table exceeds shared memory"); return PFE_EUNSUPPORTED; }
+    PFE_CUDA((warp ? gc.allow_warp : gc.allow_block)(g.smem));
+    g.threads = warp ? 32 * teams : 256;
+    const int per_sm = std::max(1, std::min(2048 / g.threads, (int)((228 * 1024) / (g.smem + 2048))));
+    g.grid = (int)std::max<long long>(
+        1, std::min<long long>((tickets + teams - 1) / teams, (long long)ctx->num_sms * std::min(per_sm, 8)));
+    g.fn = warp ? gc.warp : gc.block;
+    g.cl = &cl;
+    g.side = i % pfe_context::kSide;
+  }
+  {
+    const int rc = ensure_side(ctx);
+    if (rc != PFE_OK) return rc;
+  }
   PFE_CUDA(cudaMemsetAsync(d_gj, 0, sizeof(double) * 3 * (size_t)natom, s));
   PFE_CUDA(cudaMemsetAsync(d_gk, 0, sizeof(double) * 3 * (size_t)natom, s));
   MolLaunch ql = molecular_launch(ctx, d_dt);
   GradOut go{d_gj, d_gk, natom, d_satom, ctx->shells.zeta};
   // the classes side by side on the context's streams: their launches end on few teams
-  {
-    const int rc = ensure_side(ctx);
-    if (rc != PFE_OK) return rc;
+  SideFork sides(ctx, s);
+  PFE_CUDA(sides.fork((1u << pfe_context::kSide) - 1));
+  for (int i = 0; i < n; ++i) {
+    const Launch& g = launch[i];
+    ql.chunks = g.cl->chunks;
+    ql.nchunks = g.cl->d_nchunks;
+    g.fn(ql, g.t, go, g.vmax, g.per_team, g.grid, g.threads, g.smem, ctx->side[g.side]);
   }
-  PFE_CUDA(cudaEventRecord(ctx->ev_fork, s));
-  for (int k = 0; k < pfe_context::kSide; ++k) PFE_CUDA(cudaStreamWaitEvent(ctx->side[k], ctx->ev_fork, 0));
-  for (int i = ctx->nlaunch - 1; i >= 0; --i) {   // the classes of the longest quartets first
-    const ClassLaunch& cl = ctx->launches[i];
-    const GradClass gc = grad_class(cl.cb, cl.ck);
-    if (!gc.warp) { set_error("no gradient kernel for a quartet class"); return PFE_EUNSUPPORTED; }
-    GradTables t{};
-    int vmax = 0;
-    for (int k = 0; k < 3; ++k) {
-      const int rc = upload_optable(ctx, gc.tab[k], &t.t[k]);
-      if (rc != PFE_OK) return rc;
-      vmax = std::max(vmax, gc.tab[k]->nslots);
-    }
-    ql.chunks = cl.chunks;
-    ql.nchunks = cl.d_nchunks;
-    // a warp per quartet where at least kWarpTeams fit an SM's shared memory, else a block
-    constexpr int kWarpTeams = 8;
-    const int per_team = vmax + gc.np;
-    const size_t one = sizeof(double) * (size_t)per_team, sm = 220 * 1024;
-    const bool warp = one * kWarpTeams <= sm;
-    const long long tickets = 32ll * cl.nchunks_host;
-    int teams = 1;   // per block
-    if (warp) teams = (int)std::min<size_t>(8, std::max<size_t>(1, sm / 4 / one));
-    const size_t smem = one * teams;
-    if (smem > 227 * 1024) { set_error("gradient op table exceeds shared memory"); return PFE_EUNSUPPORTED; }
-    PFE_CUDA((warp ? gc.allow_warp : gc.allow_block)(smem));
-    const int threads = warp ? 32 * teams : 256;
-    const int per_sm = std::max(1, std::min(2048 / threads, (int)((228 * 1024) / (smem + 2048))));
-    const int grid = (int)std::max<long long>(
-        1, std::min<long long>((tickets + teams - 1) / teams, (long long)ctx->num_sms * std::min(per_sm, 8)));
-    (warp ? gc.warp : gc.block)(ql, t, go, vmax, per_team, grid, threads, smem, ctx->side[i % pfe_context::kSide]);
-    PFE_CUDA(cudaGetLastError());
-  }
-  for (int k = 0; k < pfe_context::kSide; ++k) {
-    PFE_CUDA(cudaEventRecord(ctx->ev_join[k], ctx->side[k]));
-    PFE_CUDA(cudaStreamWaitEvent(s, ctx->ev_join[k], 0));
-  }
+  PFE_CUDA(cudaGetLastError());
+  PFE_CUDA(sides.join());
   return PFE_OK;
 }
 

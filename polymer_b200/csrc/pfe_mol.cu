@@ -1787,7 +1787,7 @@ static int launch_classes(pfe_context* cx, const ClassLaunch* launches, int nlau
   cudaStream_t on[64];
   int order[64];
   double load[pfe_context::kSide + 1] = {0.0};
-  bool used[pfe_context::kSide + 1] = {false};
+  unsigned int used = 0;   // side streams
   auto straight = [&](int i) { return (launches[i].variant == 0 && launches[i].has_straight) || !launches[i].has_table; };
   // the interpreters run at about a fifth of the straight-line classes' rate
   auto work = [&](int i) {
@@ -1808,24 +1808,17 @@ static int launch_classes(pfe_context* cx, const ClassLaunch* launches, int nlau
     } else if (fork && !ql.insts && !straight(order[j])) {
       k = 1;
     }
-    used[k] = true;
+    if (k > 0) used |= 1u << (k - 1);
     on[order[j]] = k == 0 ? s : cx->side[k - 1];
   }
-  bool any = false;
-  for (int k = 1; k <= pfe_context::kSide; ++k) any = any || used[k];
-  if (any) PFE_CUDA(cudaEventRecord(cx->ev_fork, s));
-  for (int k = 1; k <= pfe_context::kSide; ++k)
-    if (used[k]) PFE_CUDA(cudaStreamWaitEvent(cx->side[k - 1], cx->ev_fork, 0));
+  SideFork sides(cx, s);
+  PFE_CUDA(sides.fork(used));
   for (int j = 0; j < nlaunch; ++j) {
     const ClassLaunch& cl = launches[order[j]];
     launch_class(cx, cl, ql, cl.variant, on[order[j]], mixed);
   }
   PFE_CUDA(cudaGetLastError());
-  for (int k = 1; k <= pfe_context::kSide; ++k)
-    if (used[k]) {
-      PFE_CUDA(cudaEventRecord(cx->ev_join[k - 1], cx->side[k - 1]));
-      PFE_CUDA(cudaStreamWaitEvent(s, cx->ev_join[k - 1], 0));
-    }
+  PFE_CUDA(sides.join());
   return PFE_OK;
 }
 

@@ -118,3 +118,44 @@ def test_batch_setup_recovers_from_allocation_failure(waters, after):
     finally:
         L.pfe_debug_fail_allocation(-1)
         L.pfe_batch_destroy(h)
+
+
+GRADIENT = '''
+import ctypes, sys
+import numpy as np
+from polymer_b200 import capi, fock, geometry, system
+L = capi.lib()
+s, other = [system.build_system(geometry.water_deck(1, seed=k), fock.onee) for k in (80, 81)]
+def density(t):
+    return (t.basis.cc.T @ np.eye(t.basis.ncgs) @ t.basis.cc)[None]
+def gradient():
+    return np.concatenate(fock.fourindex_eri_gradient(s, density(s)))
+j0, k0 = fock.fourindex_eri(s, density(s))          # the set-up of this geometry
+L.pfe_debug_fail_allocation(int(sys.argv[1]))
+try:
+    gradient()
+    raise SystemExit('the failure was not reported')
+except capi.FockError as e:
+    assert e.code == -5, e
+L.pfe_debug_fail_allocation(-1)
+j1, k1 = fock.fourindex_eri(s, density(s))
+g1 = gradient()
+fock.fourindex_eri(other, density(other))           # another geometry, then this one set up again
+g2 = gradient()
+for a, b in ((j1, j0), (k1, k0), (g1, g2)):
+    assert np.abs(a - b).max() <= 1e-11 * np.abs(b).max()
+'''
+
+
+@pytest.mark.parametrize('after', [0, 1, 2, 12, 40])
+def test_gradient_recovers_from_allocation_failure(after):
+    """The gradient's scratch (0, 1) and the upload of one of its tables (2 and up: in a process of its own,
+    since tables are uploaded once) fail: nothing has been launched, the status is PFE_ENOMEM, and later builds
+    and gradients on the same context are those of an undisturbed one."""
+    import os
+    import subprocess
+    import sys
+    root = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
+    r = subprocess.run([sys.executable, '-c', GRADIENT, str(after)], cwd=root, capture_output=True, text=True,
+                       timeout=300)
+    assert r.returncode == 0, r.stdout + r.stderr
