@@ -2079,6 +2079,15 @@ __global__ void k_batch_symmetrize(const MolLaunch* __restrict__ insts, const Pa
   }
 }
 
+// What a batch's launches take from all of its instances: the kept components (a pass is
+// skipped only if dead everywhere), and whether one copy of the Boys rows serves them all.
+static void join_launch(const pfe_batch* b, MolLaunch* lq) {
+  for (pfe_context* c : b->inst) {
+    lq->lower_kept_bits |= lower_kept_bits(c);
+    if (c->boys != b->inst[0]->boys) lq->own_boys = 1;
+  }
+}
+
 // One build of every instance from the packed contracted densities d_pc.
 int batch_fock_pc(pfe_batch* b, const double* d_pc, double* d_cc, double* d_xc, cudaStream_t s) {
   const size_t n = b->inst.size();
@@ -2116,7 +2125,7 @@ int batch_fock_pc(pfe_batch* b, const double* d_pc, double* d_cc, double* d_xc, 
   pfe_context* c0 = b->inst[0];
   MolLaunch lq = make_launch(c0, c0->d_pt);
   lq.insts = di;
-  for (pfe_context* c : b->inst) lq.lower_kept_bits |= lower_kept_bits(c);   // a pass is skipped only if dead everywhere
+  join_launch(b, &lq);
   {
     const int rc = launch_classes(c0, b->launches, b->nlaunch, lq, s, b->mixed, b->concurrent, false);
     if (rc != PFE_OK) return rc;
@@ -2150,7 +2159,7 @@ int batch_autotune(pfe_batch* b, const double* d_pc, cudaStream_t s) {
   pfe_context* c0 = b->inst[0];
   MolLaunch lq = make_launch(c0, c0->d_pt);
   lq.insts = static_cast<const MolLaunch*>(b->d_insts);
-  for (pfe_context* c : b->inst) lq.lower_kept_bits |= lower_kept_bits(c);
+  join_launch(b, &lq);
   cudaEvent_t e0, e1;
   PFE_CUDA(cudaEventCreate(&e0));
   PFE_CUDA(cudaEventCreate(&e1));

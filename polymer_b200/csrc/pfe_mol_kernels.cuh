@@ -92,6 +92,7 @@ struct MolLaunch {
   int nt;
   int myid, numprocs;
   const MolLaunch* insts;   // batches: the launch record of every instance (Chunk::inst), else null
+  int own_boys;             // batches: the instances' Boys tables differ (set up with different IGAMMA)
   int lower_kept_bits;      // bit L: some shell of top L has a coefficient on a lower component
   // block panels (see Panels): the density and the J', K' accumulators of the
   // digestion kernels, and the panel row where a shell's block begins
@@ -315,15 +316,17 @@ inline unsigned long long live_passes(int LA, int LB, int LC, int LD, int npass,
 // (10|00) gains 5 % at five blocks, (10|10) and (11|00) lose 10-20 % there.  The classes up
 // to a total of 2 hold the same warps in two blocks, each with its copy of the Boys rows in
 // shared memory, on a grid of resident blocks.
-template <int LA, int LB, int LC, int LD>
+// OWN: a batch whose instances were set up with different IGAMMA, for which no one copy is
+// right, reads each instance's rows from global memory.
+template <int LA, int LB, int LC, int LD, bool OWN = false>
 struct GqOccupancy {
   static constexpr int LT = LA + LB + LC + LD;
-  static constexpr bool staged = DownSmem<LT>::use;
+  static constexpr bool staged = DownSmem<LT>::use && !OWN;
   static constexpr int threads = staged ? (LT <= 1 ? 320 : 256) : 128;
   static constexpr int blocks = staged ? 2 : (LT <= 4 ? 3 : 1);
 };
 
-template <int LA, int LB, int LC, int LD, int KEPT, int NPASS, int PASS, bool MIXED, bool BATCH>
+template <int LA, int LB, int LC, int LD, int KEPT, int NPASS, int PASS, bool MIXED, bool BATCH, bool OWN>
 __device__ __forceinline__ void gq_pass(const MolLaunch& lq, const double2* s_boys) {
   constexpr int NA = ncum(LA), NB = ncum(LB), NC = ncum(LC), ND = ncum(LD);
   constexpr int NI = NA * NB * NC * ND;
@@ -462,7 +465,7 @@ __device__ __forceinline__ void gq_pass(const MolLaunch& lq, const double2* s_bo
         if constexpr (MIXED && LT > 0) f32 = __all_sync(__activemask(), sp * sq * pmax < mcut);
         n32 += f32 ? 1u : 0u;
         double F[LT + 1];
-        boys_down<LT, DownSmem<LT>::use>(T, f32 ? 1.0 : pref, down, F, s_boys);
+        boys_down<LT, GqOccupancy<LA, LB, LC, LD, OWN>::staged>(T, f32 ? 1.0 : pref, down, F, s_boys);
         double out[NI];
         if constexpr (LT == 0) {
           out[0] = F[0];
@@ -562,40 +565,43 @@ void launch_digest(int cb, int ck, const MolLaunch& ql, int num_sms, cudaStream_
 // launch-bound.
 constexpr int kPassGroup = 8;
 
-template <int LA, int LB, int LC, int LD, int KEPT, int NPASS, int P0, int PN, bool MIXED, bool BATCH>
+template <int LA, int LB, int LC, int LD, int KEPT, int NPASS, int P0, int PN, bool MIXED, bool BATCH, bool OWN>
 __device__ __forceinline__ void gq_select(const MolLaunch& lq, int p, const double2* s_boys) {
   if constexpr (PN == 1) {
-    gq_pass<LA, LB, LC, LD, KEPT, NPASS, P0, MIXED, BATCH>(lq, s_boys);
+    gq_pass<LA, LB, LC, LD, KEPT, NPASS, P0, MIXED, BATCH, OWN>(lq, s_boys);
   } else {
-    if (p == P0) gq_pass<LA, LB, LC, LD, KEPT, NPASS, P0, MIXED, BATCH>(lq, s_boys);
-    else gq_select<LA, LB, LC, LD, KEPT, NPASS, P0 + 1, PN - 1, MIXED, BATCH>(lq, p, s_boys);
+    if (p == P0) gq_pass<LA, LB, LC, LD, KEPT, NPASS, P0, MIXED, BATCH, OWN>(lq, s_boys);
+    else gq_select<LA, LB, LC, LD, KEPT, NPASS, P0 + 1, PN - 1, MIXED, BATCH, OWN>(lq, p, s_boys);
   }
 }
 
 // Passes P0 .. P0 + PN - 1; blockIdx.y is the position among the live ones (bits of live).
-template <int LA, int LB, int LC, int LD, int KEPT, int NPASS, int P0, int PN, bool MIXED, bool BATCH>
-__global__ void __launch_bounds__(GqOccupancy<LA, LB, LC, LD>::threads, GqOccupancy<LA, LB, LC, LD>::blocks)
+template <int LA, int LB, int LC, int LD, int KEPT, int NPASS, int P0, int PN, bool MIXED, bool BATCH, bool OWN>
+__global__ void __launch_bounds__(GqOccupancy<LA, LB, LC, LD, OWN>::threads, GqOccupancy<LA, LB, LC, LD, OWN>::blocks)
     k_gq(const __grid_constant__ MolLaunch lq, unsigned int live) {
   extern __shared__ double2 s_boys[];
-  if constexpr (DownSmem<LA + LB + LC + LD>::use) {   // once per resident block
+  if constexpr (GqOccupancy<LA, LB, LC, LD, OWN>::staged) {   // once per resident block
     down_stage<LA + LB + LC + LD>(lq.down, s_boys);
     __syncthreads();
   }
   unsigned int m = live;
   for (int y = blockIdx.y; y > 0; --y) m &= m - 1;
-  gq_select<LA, LB, LC, LD, KEPT, NPASS, P0, PN, MIXED, BATCH>(lq, P0 + __ffs(m) - 1, s_boys);
+  gq_select<LA, LB, LC, LD, KEPT, NPASS, P0, PN, MIXED, BATCH, OWN>(lq, P0 + __ffs(m) - 1, s_boys);
 }
 
 using LaunchFn = void (*)(const MolLaunch&, int grid, cudaStream_t);
 
-template <int LA, int LB, int LC, int LD, int KEPT, int NPASS, int P0, bool MIXED, bool BATCH>
+template <int LA, int LB, int LC, int LD, int KEPT, int NPASS, int P0, bool MIXED, bool BATCH, bool OWN = false>
 void launch_groups(const MolLaunch& ql, unsigned long long live, int grid, cudaStream_t s) {
   constexpr int PN = NPASS - P0 < kPassGroup ? NPASS - P0 : kPassGroup;
-  using O = GqOccupancy<LA, LB, LC, LD>;
+  using O = GqOccupancy<LA, LB, LC, LD, OWN>;
+  if constexpr (BATCH && O::staged) {
+    if (ql.own_boys) return launch_groups<LA, LB, LC, LD, KEPT, NPASS, P0, MIXED, BATCH, true>(ql, live, grid, s);
+  }
   const unsigned int m = (unsigned int)(live >> P0) & ((1u << PN) - 1);
   if (m) {
-    auto kern = k_gq<LA, LB, LC, LD, KEPT, NPASS, P0, PN, MIXED, BATCH>;
-    constexpr size_t bytes = DownSmem<O::LT>::BYTES;
+    auto kern = k_gq<LA, LB, LC, LD, KEPT, NPASS, P0, PN, MIXED, BATCH, OWN>;
+    constexpr size_t bytes = O::staged ? DownSmem<O::LT>::BYTES : 0;
     // `grid` counts blocks of four warps
     int g = grid;
     if constexpr (O::staged) {
@@ -604,7 +610,8 @@ void launch_groups(const MolLaunch& ql, unsigned long long live, int grid, cudaS
     }
     kern<<<dim3(g, __builtin_popcount(m)), O::threads, bytes, s>>>(ql, m);
   }
-  if constexpr (P0 + PN < NPASS) launch_groups<LA, LB, LC, LD, KEPT, NPASS, P0 + PN, MIXED, BATCH>(ql, live, grid, s);
+  if constexpr (P0 + PN < NPASS)
+    launch_groups<LA, LB, LC, LD, KEPT, NPASS, P0 + PN, MIXED, BATCH, OWN>(ql, live, grid, s);
 }
 
 // A variant that holds the kept components only (KEPT: 0 or 2); those of the large

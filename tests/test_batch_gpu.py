@@ -10,6 +10,7 @@ over the work of every molecule in the batch.
   the per-molecule builds the same way;
 * the census of a batch sums its molecules' quartets while the class launches
   do not grow with the number of molecules;
+* each molecule is built with the Boys table (IGAMMA) of its own set-up;
 * after the batch autotuner has timed every variant of every class, builds
   still match the per-molecule ones;
 * a set-up refused for one instance leaves no half-built batch: later calls
@@ -90,6 +91,22 @@ def test_batch_matches_single_builds(name):
     got2 = [(b.view(oc, k), b.view(ox, k)) for k in range(len(b))]
     _check(got2, _singles(systems, pcs2), name + '/second')
     b.close()
+
+
+def test_instances_read_their_own_boys_table():
+    """IGAMMA is an input of each instance: one that differs (here by a factor, so that its integrals differ by
+    it wherever the table is read) changes its own molecule's J and K and no other's, in every class."""
+    systems = [_sys(geometry.water_deck(1, seed=3150)), _sys(geometry.alkane_deck(1)),
+               _sys(geometry.water_deck(2, seed=3151))]
+    systems[1].igamma = systems[1].igamma * 1.001
+    pcs = [_pc(s, 30 + k) for k, s in enumerate(systems)]
+    ref = _singles(systems, pcs)
+    for order in ([0, 1, 2], [1, 2, 0]):
+        b = fock.DeviceBatch([systems[k] for k in order])
+        got = b([torch.tensor(pcs[k], device='cuda') for k in order])
+        torch.cuda.synchronize()
+        _check(got, [ref[k] for k in order], 'own table')
+        b.close()
 
 
 def test_batch_screening_matches_single_builds():
