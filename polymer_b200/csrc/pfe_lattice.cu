@@ -45,7 +45,7 @@ struct LatticeLaunch {
   OpTableDev tab_top;    // its table with the d shells' top level only
   LatWideFn wide;        // kernel of that table, or null
   int nx;                // kept integrals of its largest quartet
-  int per_warp, wpb;
+  int per_warp, wpb, resident;   // of the interpreter; resident: blocks per SM
   size_t smem;
   double quartets;
 };
@@ -248,7 +248,12 @@ __global__ void __launch_bounds__(256) k_lattice(LatticeRun R, OpTableDev tab, i
   const double c2pi = 2.0 / sqrt(REF_PI);
   const int h3 = g.c2[0] + g.c1[0];
   const bool helix = R.pph != nullptr;
-  for (int c = blockIdx.x * wpb + wid; c < nchunks; c += gridDim.x * wpb) {
+  // chunks from the class's second work-queue counter (the first is k_lat_wide's)
+  for (;;) {
+    int c = 0;
+    if (lane == 0) c = atomicAdd(R.queue + 1, 1);
+    c = __shfl_sync(0xffffffffu, c, 0);
+    if (c >= nchunks) break;
     const int4 ch = R.chunks[c];
     const int p = ch.x;
     const int4 tk = R.tickets[ch.w];
@@ -413,7 +418,7 @@ __global__ void __launch_bounds__(256) k_lattice(LatticeRun R, OpTableDev tab, i
 // ---------------------------------------------------------------- host side
 
 using LatFn = void (*)(const LatticeRun&, const OpTableDev&, int grid, int wpb, int per_warp, size_t smem, cudaStream_t);
-using LatAllow = cudaError_t (*)(size_t);
+using LatAllow = cudaError_t (*)(size_t smem, int threads, int* resident);
 
 template <int LA, int LB, int LC, int LD, bool SW>
 static void launch_lat(const LatticeRun& r, const OpTableDev& t, int grid, int wpb, int per_warp, size_t smem,
@@ -421,8 +426,10 @@ static void launch_lat(const LatticeRun& r, const OpTableDev& t, int grid, int w
   k_lattice<LA, LB, LC, LD, SW><<<grid, 32 * wpb, smem, s>>>(r, t, per_warp);
 }
 template <int LA, int LB, int LC, int LD, bool SW>
-static cudaError_t allow_lat(size_t smem) {
-  return cudaFuncSetAttribute(k_lattice<LA, LB, LC, LD, SW>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+static cudaError_t allow_lat(size_t smem, int threads, int* resident) {
+  auto kern = k_lattice<LA, LB, LC, LD, SW>;
+  const cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+  return e != cudaSuccess ? e : cudaOccupancyMaxActiveBlocksPerMultiprocessor(resident, kern, threads, smem);
 }
 
 struct LatVariant {
@@ -749,7 +756,7 @@ int lattice_setup(pfe_context* ctx, const pfe_args* a) {
       ll.wpb = (int)std::max<size_t>(1, std::min<size_t>(8, (200 * 1024) / (sizeof(double) * ll.per_warp)));
       ll.smem = sizeof(double) * (size_t)ll.per_warp * ll.wpb;
       (void)nbra;
-      PFE_CUDA(lat_variant(e1, e2, cb < ck).allow(ll.smem));
+      PFE_CUDA(lat_variant(e1, e2, cb < ck).allow(ll.smem, 32 * ll.wpb, &ll.resident));
       PFE_CUDA(cudaStreamSynchronize(s));
       L->quartets += ll.quartets;
       L->flops += ll.quartets * class_flops(e1, e2);
@@ -824,8 +831,11 @@ int lattice_fock(pfe_context* ctx, const double* d_pp, const double* d_pph, doub
         const int rc = ll.wide(R, ll.tab_top, ll.nx, ll.ncells_chunks, ctx->num_sms, s);
         if (rc != PFE_OK) return rc;
       }
-      // (a block per SM where the launch is only the fallback of the above)
-      const int grid = std::min((ll.ncells_chunks + ll.wpb - 1) / ll.wpb, ctx->num_sms * (R.ghost ? 1 : 8));
+      // Resident blocks taking chunks from the queue: where the launch is only the fallback of
+      // the above, it ends as soon as one block a slot has started.  A build with ghost
+      // densities, helical polyethylene 6-31G** at CUTOFF1/2 = 1/2 and 2/2 (B200): 34.9 and
+      // 44.7 ms with one block per SM and a static share of the chunks each, 32.1 and 38.3 here.
+      const int grid = std::min((ll.ncells_chunks + ll.wpb - 1) / ll.wpb, ctx->num_sms * std::max(1, ll.resident));
       lat_variant(e1, e2, ll.cb < ll.ck).fn(R, ll.tab, std::max(grid, 1), ll.wpb, ll.per_warp, ll.smem, s);
     }
     PFE_CUDA(cudaGetLastError());

@@ -10,7 +10,7 @@ import pytest
 import torch
 
 import oracle
-from polymer_b200 import fock, inputdeck, scf, system
+from polymer_b200 import fock, geometry, inputdeck, scf, system
 
 pytestmark = pytest.mark.gpu
 
@@ -41,3 +41,34 @@ def test_d_shells_match_the_oracle(shells, helix, ghosts):
     got = fock.fourindex_eri(s, pp, ph)
     for g, r in zip(got, ref):
         assert np.abs(g - r).max() <= 1e-11 * np.abs(ref[0]).max() + 1e-13
+
+
+def test_builds_with_ghost_densities_are_no_slower_than_the_interpreter_alone():
+    """Where ghosts carry density the d classes fall back to the interpreter.  With the far-cell cutoff set and no
+    cell outside the CUTOFF1 box the same kernels do the same FP64 work without the attempt before them: the
+    fallback may cost its empty launches and the check (here some 2 %), no more."""
+    deck = geometry.polyethylene_deck('6-31Gss', cutoff1=1, cutoff2=1, kpoints=2, inttol=1e-10)
+    s = system.build_system(deck, fock.onee)
+    rng = np.random.default_rng(4)
+    pp = torch.tensor(0.05 * rng.normal(size=(s.ncell1, s.basis.npgs, s.basis.npgs)), device='cuda')
+    ph = scf.rotate(scf.HostState(s), pp.cpu()).to('cuda')
+    df = fock.DeviceFock(s)
+
+    def best():
+        times = []
+        for _ in range(7):
+            e0, e1 = torch.cuda.Event(enable_timing=True), torch.cuda.Event(enable_timing=True)
+            e0.record()
+            out = df(pp, ph)
+            e1.record()
+            torch.cuda.synchronize()
+            times.append(e0.elapsed_time(e1))
+        return min(times), out
+
+    fallback, a = best()
+    df.set_screening(mixed_cutoff=1e-30)
+    alone, b = best()
+    df.close()
+    for x, y in zip(a, b):
+        assert float((x - y).abs().max()) <= 1e-11 * float(b[0].abs().max())
+    assert fallback <= 1.05 * alone, (fallback, alone)
