@@ -178,7 +178,8 @@ typedef struct pfe_census {
   double flops;             /* FP64/FP32 recursion + digestion flops per build        */
   double quartets_fp32;     /* quartets routed to FP32 recursion (mixed mode)          */
   int64_t pairs;            /* significant primitive-shell pairs kept                 */
-  int32_t kernel_launches;  /* kernels launched by one pfe_context_fock call          */
+  int32_t kernel_launches;  /* this library's kernels that one pfe_context_fock call
+                               launches (contractions by cuBLAS not counted)          */
 } pfe_census;
 int32_t pfe_context_census(pfe_context *ctx, pfe_census *out);
 /* The same summed over a batch's instances (kernel_launches: one batched build). */

@@ -731,9 +731,10 @@ int32_t pfe_batch_census(pfe_batch* b, pfe_census* out) {
     tot.flops += ci.flops;
     tot.pairs += ci.pairs;
   }
-  int n = 0;
-  for (int i = 0; i < b->nlaunch; ++i)
-    n += (b->launches[i].variant == 0 && b->launches[i].has_straight) ? b->launches[i].launches_live : 1;
+  // class kernels, the beginning of every instance and its block maxima, and the end: one
+  // launch, or three for every instance where some has primitive targets
+  int n = b->nlaunch > 0 ? 2 + (b->all_contracted ? 1 : 3 * (int)b->inst.size()) : 0;
+  for (int i = 0; i < b->nlaunch; ++i) n += class_launches(b->launches[i], 1);
   tot.kernel_launches = n;
   *out = tot;
   return PFE_OK;
@@ -762,15 +763,14 @@ int32_t pfe_context_census(pfe_context* ctx, pfe_census* out) {
   }
   out->pairs = ctx->npairs;
   if (ctx->molecular) {
-    // class kernels (pass groups and digestion), the target-space density and its check,
-    // the panels' beginning and end, the block maxima under density screening or mixed precision
-    int n = 0;
-    for (int i = 0; i < ctx->nlaunch; ++i)
-      n += (ctx->launches[i].variant == 0 && ctx->launches[i].has_straight) ? ctx->launches[i].launches_live : 1;
-    n += (ctx->contracted ? 2 : 0) + 2 + ((ctx->dtol > 0.0 || ctx->mcut > 0.0) ? 1 : 0);
+    // class kernels, the panels' beginning and end, the target-space density and its check or
+    // the two symmetrisations after the contraction, the block maxima under density screening
+    // or mixed precision
+    int n = 4 + ((ctx->dtol > 0.0 || ctx->mcut > 0.0) ? 1 : 0);
+    for (int i = 0; i < ctx->nlaunch; ++i) n += class_launches(ctx->launches[i], ctx->numprocs);
     out->kernel_launches = n;
   } else {
-    out->kernel_launches = lattice_class_launches(ctx) + 3;
+    out->kernel_launches = lattice_launches(ctx);
   }
   return PFE_OK;
 }

@@ -232,9 +232,18 @@ struct ClassLaunch {
   int* queue;                // device work queue: one chunk counter per launch (pass), zeroed before each
   int npass;                 // register passes of the straight-line variant (general; see pass_variant)
   unsigned long long live;   // the passes launched: those with a component that has a coefficient
-  int launches_live;         // its kernel launches: pass groups with a component that has a coefficient, digestion
+  int launches_live;         // kernel launches of a tile: pass groups with a component that has a coefficient, digestion
   int gmul = 32;             // straight-line variant: persistent grid of up to gmul blocks per SM
 };
+
+// Kernel launches of one class of a build (launch_class): those of its tiles, or one.
+// (An instance of a batch has no launches of its own: no chunks, no memory for a tile.)
+inline int class_launches(const ClassLaunch& cl, int numprocs) {
+  if (cl.has_table && !(cl.variant == 0 && cl.has_straight)) return 1;
+  const int work = (cl.nchunks_host + numprocs - 1) / numprocs;
+  if (work <= 0) return 0;
+  return (cl.cb > 0 ? (work + cl.xcap - 1) / std::max(1, cl.xcap) : 1) * cl.launches_live;
+}
 
 }  // namespace pfe
 
@@ -487,7 +496,7 @@ int lattice_fock(pfe_context* ctx, const double* d_pp, const double* d_pph, doub
                  cudaStream_t s);
 void lattice_release(pfe_context* ctx);
 void lattice_force_interpreter(pfe_context* ctx, bool on);
-int lattice_class_launches(pfe_context* ctx);
+int lattice_launches(pfe_context* ctx);
 int molecular_gradient_pp(pfe_context* ctx, const double* d_pp, const int* d_satom, int natom, double* d_gj,
                           double* d_gk, cudaStream_t s);
 const char* last_error_cstr();

@@ -774,6 +774,11 @@ int lattice_setup(pfe_context* ctx, const pfe_args* a) {
   return PFE_OK;
 }
 
+// The kernels of kept components are FP64 in every cell.
+static bool wide_allowed(const pfe_context* ctx, const LatticeState* L) {
+  return !L->interpret_only && !(ctx->mcut > 0.0);
+}
+
 int lattice_fock(pfe_context* ctx, const double* d_pp, const double* d_pph, double* d_cc, double* d_xc,
                  cudaStream_t s) {
   LatticeState* L = (LatticeState*)ctx->lattice;
@@ -803,7 +808,7 @@ int lattice_fock(pfe_context* ctx, const double* d_pp, const double* d_pph, doub
   // ghost has a density; decided on the device
   bool wide = false;
   for (int i = 0; i < L->nlaunch; ++i) wide = wide || L->launches[i].wide != nullptr;
-  wide = wide && !L->interpret_only && !R.far32;
+  wide = wide && wide_allowed(ctx, L);
   if (wide) {
     PFE_CUDA(cudaMemsetAsync(L->d_ghost, 0, sizeof(int), s));
     lattice_ghost_check(d_pp, (long long)pp, ctx->npgs, ctx->d_tidx, L->d_ghost, ctx->num_sms, s);
@@ -861,18 +866,23 @@ int lattice_fock(pfe_context* ctx, const double* d_pp, const double* d_pph, doub
   return PFE_OK;
 }
 
-// Class kernel launches of one lattice build: a straight-line class's register
-// passes, one launch for an interpreted class.
-int lattice_class_launches(pfe_context* ctx) {
+// Kernel launches of one lattice build: a straight-line class's register passes, one for an
+// interpreted class, two where the kernels of kept components come before it, and then the
+// checks for ghost densities.  (The contraction after them is cuBLAS's.)
+int lattice_launches(pfe_context* ctx) {
   const LatticeState* L = (const LatticeState*)ctx->lattice;
   if (!L) return 0;
   int n = 0;
+  bool wide = false;
   for (int i = 0; i < L->nlaunch; ++i) {
     const LatticeLaunch& ll = L->launches[i];
     const int e1 = std::max(ll.cb, ll.ck), e2 = std::min(ll.cb, ll.ck);
-    n += L->interpret_only ? 1 : std::max(1, lattice_sl_passes(e1, e2, ll.cb < ll.ck));
+    const int passes = L->interpret_only ? 0 : lattice_sl_passes(e1, e2, ll.cb < ll.ck);
+    const bool w = ll.wide != nullptr && passes == 0 && wide_allowed(ctx, L);
+    n += passes > 0 ? passes : 1 + w;
+    wide = wide || w;
   }
-  return n;
+  return n + (wide ? (ctx->helix != 0.0 ? 2 : 1) : 0);
 }
 
 void lattice_force_interpreter(pfe_context* ctx, bool on) {
