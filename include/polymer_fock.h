@@ -280,6 +280,13 @@ const char *pfe_version(void);
  * Process-wide; nothing is attempted on the device. */
 int32_t pfe_debug_fail_allocation(int32_t after);
 
+/* Testing aid, no reference counterpart: the limits of the memory for stored
+ * integrals that later set-ups work to.  A class stores at most tile_bytes at a
+ * time (at least one chunk) and runs in as many tiles as that takes; classes run
+ * side by side, each with its own memory, where all of them together need no more
+ * than together_bytes.  Either <= 0: its default, 1 GiB.  Process-wide. */
+int32_t pfe_debug_integral_memory(int64_t tile_bytes, int64_t together_bytes);
+
 #ifdef __cplusplus
 }
 #endif

@@ -479,6 +479,11 @@ int32_t pfe_debug_fail_allocation(int32_t after) {
   return PFE_OK;
 }
 
+int32_t pfe_debug_integral_memory(int64_t tile_bytes, int64_t together_bytes) {
+  pfe::debug_integral_memory(tile_bytes, together_bytes);
+  return PFE_OK;
+}
+
 int32_t pfe_last_error(char* buf, int32_t len) {
   const char* m = last_error_cstr();
   const int32_t n = (int32_t)strlen(m);

@@ -433,6 +433,7 @@ inline bool ensure_blas(pfe_context* ctx) {
   return true;
 }
 int ensure_side(pfe_context* ctx);
+void debug_integral_memory(long long tile, long long together);
 
 // Work of a build on the context's side streams (bit k of `used`: side[k]), forked from
 // stream s and joined back to it on every way out: after an error too, later work on s

@@ -1091,6 +1091,15 @@ static int kept_integrals(int cb, int ck, int bits) {
   return kept_n(kCL[cb][0], bits) * kept_n(kCL[cb][1], bits) * kept_n(kCL[ck][0], bits) * kept_n(kCL[ck][1], bits);
 }
 
+// Limits of the memory for stored integrals (settable for tests).
+static constexpr long long kTileBytes = 1LL << 30, kTogetherBytes = 1LL << 30;
+static std::atomic<long long> g_tile_bytes{kTileBytes}, g_together_bytes{kTogetherBytes};
+
+void debug_integral_memory(long long tile, long long together) {
+  g_tile_bytes.store(tile > 0 ? tile : kTileBytes);
+  g_together_bytes.store(together > 0 ? together : kTogetherBytes);
+}
+
 // Memory for the stored integrals of the straight-line classes.  Where all classes fit
 // kTogetherBytes together, each has a buffer of its own and the classes run side by
 // side (launch_classes); otherwise they use one buffer after another, of the largest
@@ -1100,7 +1109,7 @@ static int kept_integrals(int cb, int ck, int bits) {
 // of what the digestion inside every pass cost.
 template <typename Owner>
 static int alloc_integrals(Owner* own, ClassLaunch* launches, int nlaunch, int bits, cudaStream_t s) {
-  constexpr size_t kTileBytes = (size_t)1 << 30, kTogetherBytes = (size_t)1 << 30;
+  const size_t tile = (size_t)g_tile_bytes.load(), together = (size_t)g_together_bytes.load();
   auto bytes_per = [&](const ClassLaunch& cl) {
     return sizeof(double) * 32 * (size_t)kept_integrals(cl.cb, cl.ck, bits);
   };
@@ -1109,13 +1118,13 @@ static int alloc_integrals(Owner* own, ClassLaunch* launches, int nlaunch, int b
     ClassLaunch& cl = launches[i];
     cl.xcap = 0;
     if (!cl.has_straight || cl.cb == 0) continue;
-    cl.xcap = (int)std::max<size_t>(1, std::min<size_t>(kTileBytes / bytes_per(cl), (size_t)cl.nchunks_host));
+    cl.xcap = (int)std::max<size_t>(1, std::min<size_t>(tile / bytes_per(cl), (size_t)cl.nchunks_host));
     most = std::max(most, bytes_per(cl) * cl.xcap);
     most_flags = std::max(most_flags, (size_t)cl.xcap);
     sum += bytes_per(cl) * (size_t)cl.nchunks_host;
     sum_flags += (size_t)cl.nchunks_host;
   }
-  own->concurrent = sum <= kTogetherBytes;
+  own->concurrent = sum <= together;
   double* x = nullptr;
   unsigned char* f = nullptr;
   if (most > 0) {
