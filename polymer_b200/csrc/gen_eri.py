@@ -465,7 +465,8 @@ def main():
             big.append(emit_optable(LA, LB, LC, LD))   # every class can run interpreted
             if LA >= 1:
                 big.append(emit_optable(LA, LB, LC, LD, pure_bra=True))
-            if LA == 2:
+            # the classes of the lattice kernels of kept components (pfe_lattice_wide.cu)
+            if LB == 2 or (LA, LB) == (2, 1) and (LC, LD) >= (1, 1):
                 big.append(emit_optable(LA, LB, LC, LD, top_d=True))
             if LA >= 1 and LC >= 1 and pure_ket_gains(LA, LB, LC, LD):
                 big.append(emit_optable(LA, LB, LC, LD, pure_bra=True, pure_ket=True))

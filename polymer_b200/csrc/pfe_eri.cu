@@ -132,15 +132,10 @@ const OpTableHost* host_optable_pure2(int cb, int ck) {
   }
 }
 
-// The class's table with the top-level components of d shells only, all of s and p shells.
+// The class's table with the top-level components of d shells only, all of s and p shells
+// (the classes of pfe_lattice_wide.cu).
 const OpTableHost* host_optable_topd(int cb, int ck) {
   switch (cb * 8 + ck) {
-    case 3 * 8 + 0: return &op_2000_topd;
-    case 3 * 8 + 1: return &op_2010_topd;
-    case 3 * 8 + 2: return &op_2011_topd;
-    case 3 * 8 + 3: return &op_2020_topd;
-    case 4 * 8 + 0: return &op_2100_topd;
-    case 4 * 8 + 1: return &op_2110_topd;
     case 4 * 8 + 2: return &op_2111_topd;
     case 4 * 8 + 3: return &op_2120_topd;
     case 4 * 8 + 4: return &op_2121_topd;

@@ -1707,8 +1707,9 @@ static bool variant_ok(const ClassLaunch& cl, int v) {
 }
 
 // Time every execution variant of one class -- and, for the straight-line
-// variant, its persistent grid (4, 8, 16 or 32 blocks per SM) -- and keep the
-// fastest (best of two launches after one warm-up each).
+// variant, its persistent grid (4, 8, 16 or 32 blocks per SM, but one of resident
+// blocks in the classes that stage their Boys rows) -- and keep the fastest (best of
+// two launches after one warm-up each).
 static int tune_class(pfe_context* ctx, ClassLaunch& cl, const MolLaunch& ql, cudaStream_t s, bool mixed,
                       cudaEvent_t e0, cudaEvent_t e1) {
   float best = 1e30f;
@@ -1720,10 +1721,11 @@ static int tune_class(pfe_context* ctx, ClassLaunch& cl, const MolLaunch& ql, cu
     // not timed there, which keeps the autotuner to seconds
     if ((v == 1 || v == 2) && cl.has_straight) continue;
     static const int kGmul[4] = {4, 8, 16, 32};
-    const int ng = v == 0 ? 4 : 1;
+    const bool staged = kCL[cl.cb][0] + kCL[cl.cb][1] + kCL[cl.ck][0] + kCL[cl.ck][1] <= 2;
+    const int ng = (v == 0 && !staged) ? 4 : 1;
     float tv = 1e30f;
     for (int gi = 0; gi < ng; ++gi) {
-      if (v == 0) cl.gmul = kGmul[gi];
+      if (ng > 1) cl.gmul = kGmul[gi];
       auto once = [&]() {
         cudaMemsetAsync(cl.queue, 0, sizeof(int) * 64, s);
         launch_class(ctx, cl, ql, v, s, mixed);
@@ -1790,9 +1792,8 @@ int ensure_side(pfe_context* ctx) {
 //     single molecule the interpreter classes (few resident warps, bound by shared
 //     memory or barriers) beside them on one side stream: C20H42 34.0 -> 32.0 ms; the
 //     32-cluster water batch was 2 % slower split that way.
-// Serial on s when `serial` (per-class timing).
 static int launch_classes(pfe_context* cx, const ClassLaunch* launches, int nlaunch, const MolLaunch& ql,
-                          cudaStream_t s, bool mixed, bool together, bool serial) {
+                          cudaStream_t s, bool mixed, bool together) {
   cudaStream_t on[64];
   int order[64];
   double load[pfe_context::kSide + 1] = {0.0};
@@ -1803,18 +1804,17 @@ static int launch_classes(pfe_context* cx, const ClassLaunch* launches, int nlau
     return launches[i].quartets * class_flops(launches[i].cb, launches[i].ck) * (straight(i) ? 1.0 : 5.0);
   };
   for (int i = 0; i < nlaunch; ++i) order[i] = i;
-  const bool fork = !serial && cx->ev_fork != nullptr;
-  if (fork && together)   // the interpreter classes first: their longest pieces take longest
+  if (together)   // the interpreter classes first: their longest pieces take longest
     std::sort(order, order + nlaunch, [&](int a, int b) {
       return straight(a) != straight(b) ? !straight(a) : work(a) > work(b);
     });
   for (int j = 0; j < nlaunch; ++j) {
     int k = 0;
-    if (fork && together) {
+    if (together) {
       for (int x = 1; x <= pfe_context::kSide; ++x)
         if (load[x] < load[k]) k = x;
       load[k] += work(order[j]);
-    } else if (fork && !ql.insts && !straight(order[j])) {
+    } else if (!ql.insts && !straight(order[j])) {
       k = 1;
     }
     if (k > 0) used |= 1u << (k - 1);
@@ -1842,7 +1842,7 @@ static int run_build(pfe_context* ctx, const double* d_dt, double* d_cc, double*
     PFE_CUDA(cudaEventRecord(ctx->ev[0], s));
   }
   if (!ctx->profile) {
-    const int rc2 = launch_classes(ctx, ctx->launches, ctx->nlaunch, ql, s, ctx->mcut > 0.0, ctx->concurrent, false);
+    const int rc2 = launch_classes(ctx, ctx->launches, ctx->nlaunch, ql, s, ctx->mcut > 0.0, ctx->concurrent);
     if (rc2 != PFE_OK) return rc2;
   }
   for (int i = 0; i < ctx->nlaunch && ctx->profile; ++i) {
@@ -2136,7 +2136,7 @@ int batch_fock_pc(pfe_batch* b, const double* d_pc, double* d_cc, double* d_xc, 
   lq.insts = di;
   join_launch(b, &lq);
   {
-    const int rc = launch_classes(c0, b->launches, b->nlaunch, lq, s, b->mixed, b->concurrent, false);
+    const int rc = launch_classes(c0, b->launches, b->nlaunch, lq, s, b->mixed, b->concurrent);
     if (rc != PFE_OK) return rc;
   }
   if (b->all_contracted) {

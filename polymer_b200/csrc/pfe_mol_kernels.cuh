@@ -94,7 +94,7 @@ struct MolLaunch {
   const MolLaunch* insts;   // batches: the launch record of every instance (Chunk::inst), else null
   int own_boys;             // batches: the instances' Boys tables differ (set up with different IGAMMA)
   int lower_kept_bits;      // bit L: some shell of top L has a coefficient on a lower component
-  // block panels (see Panels): the density and the J', K' accumulators of the
+  // block panels (pfe_context): the density and the J', K' accumulators of the
   // digestion kernels, and the panel row where a shell's block begins
   const double* pd;
   double* pj;
@@ -238,11 +238,6 @@ __host__ __device__ constexpr int lower_pairs(int LA, int LB) {
       if (comp_tot(LA, a) < LA || comp_tot(LB, b) < LB) ++c;
   return c;
 }
-
-template <int LA, int LB>
-struct LowerPairs {
-  static constexpr int n = lower_pairs(LA, LB);
-};
 
 // The bra component pairs [ab0, ab1) (positions in AbOrder) register pass `pass`
 // of `npass` keeps.  Two-pass (d s| classes split at the level boundary: the
