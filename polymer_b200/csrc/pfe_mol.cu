@@ -1092,7 +1092,7 @@ static int kept_integrals(int cb, int ck, int bits) {
 }
 
 // Limits of the memory for stored integrals (settable for tests).
-static constexpr long long kTileBytes = 1LL << 30, kTogetherBytes = 1LL << 30;
+static constexpr long long kTileBytes = 1LL << 30, kTogetherBytes = 1LL << 30, kLeastTileBytes = 4 << 20;
 static std::atomic<long long> g_tile_bytes{kTileBytes}, g_together_bytes{kTogetherBytes};
 
 void debug_integral_memory(long long tile, long long together) {
@@ -1103,35 +1103,46 @@ void debug_integral_memory(long long tile, long long together) {
 // Memory for the stored integrals of the straight-line classes.  Where all classes fit
 // kTogetherBytes together, each has a buffer of its own and the classes run side by
 // side (launch_classes); otherwise they use one buffer after another, of the largest
-// class's size up to kTileBytes, and larger classes run in tiles of that size.
+// class's size up to kTileBytes, and larger classes run in tiles of that size.  Where
+// the device has no room for that (a program may keep hundreds of contexts), one buffer
+// and tiles of a quarter, down to kLeastTileBytes, do: more launches, the same work.
 // Measured on B200: a tile's passes last long enough (milliseconds) that their tails
 // do not show, and the buffer's traffic (written and read once, at HBM rate) is a tenth
 // of what the digestion inside every pass cost.
 template <typename Owner>
 static int alloc_integrals(Owner* own, ClassLaunch* launches, int nlaunch, int bits, cudaStream_t s) {
-  const size_t tile = (size_t)g_tile_bytes.load(), together = (size_t)g_together_bytes.load();
+  size_t tile = (size_t)g_tile_bytes.load(), together = (size_t)g_together_bytes.load();
   auto bytes_per = [&](const ClassLaunch& cl) {
     return sizeof(double) * 32 * (size_t)kept_integrals(cl.cb, cl.ck, bits);
   };
-  size_t most = 0, most_flags = 0, sum = 0, sum_flags = 0;
-  for (int i = 0; i < nlaunch; ++i) {
-    ClassLaunch& cl = launches[i];
-    cl.xcap = 0;
-    if (!cl.has_straight || cl.cb == 0) continue;
-    cl.xcap = (int)std::max<size_t>(1, std::min<size_t>(tile / bytes_per(cl), (size_t)cl.nchunks_host));
-    most = std::max(most, bytes_per(cl) * cl.xcap);
-    most_flags = std::max(most_flags, (size_t)cl.xcap);
-    sum += bytes_per(cl) * (size_t)cl.nchunks_host;
-    sum_flags += (size_t)cl.nchunks_host;
-  }
-  own->concurrent = sum <= together;
   double* x = nullptr;
   unsigned char* f = nullptr;
-  if (most > 0) {
+  for (;;) {
+    size_t most = 0, most_flags = 0, sum = 0, sum_flags = 0;
+    for (int i = 0; i < nlaunch; ++i) {
+      ClassLaunch& cl = launches[i];
+      cl.xcap = 0;
+      if (!cl.has_straight || cl.cb == 0) continue;
+      cl.xcap = (int)std::max<size_t>(1, std::min<size_t>(tile / bytes_per(cl), (size_t)cl.nchunks_host));
+      most = std::max(most, bytes_per(cl) * cl.xcap);
+      most_flags = std::max(most_flags, (size_t)cl.xcap);
+      sum += bytes_per(cl) * (size_t)cl.nchunks_host;
+      sum_flags += (size_t)cl.nchunks_host;
+    }
+    own->concurrent = sum <= together;
+    if (most == 0) break;
     const size_t flags = own->concurrent ? sum_flags : most_flags;
-    PFE_CUDA(own->alloc_kept((void**)&x, own->concurrent ? sum : most));
+    const cudaError_t e = own->alloc_kept((void**)&x, own->concurrent ? sum : most);
+    if (e == cudaErrorMemoryAllocation && (own->concurrent || tile > kLeastTileBytes)) {
+      (void)cudaGetLastError();   // not an error: less memory will do
+      if (own->concurrent) together = 0;
+      else tile /= 4;
+      continue;
+    }
+    PFE_CUDA(e);
     PFE_CUDA(own->alloc((void**)&f, flags));
     PFE_CUDA(cudaMemsetAsync(f, 0, flags, s));
+    break;
   }
   size_t xo = 0, fo = 0;
   for (int i = 0; i < nlaunch; ++i) {

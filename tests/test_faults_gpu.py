@@ -159,3 +159,45 @@ def test_gradient_recovers_from_allocation_failure(after):
     r = subprocess.run([sys.executable, '-c', GRADIENT, str(after)], cwd=root, capture_output=True, text=True,
                        timeout=300)
     assert r.returncode == 0, r.stdout + r.stderr
+
+
+@pytest.mark.parametrize('tile, together', [(0, 0), (16 << 20, 1)])
+def test_setup_without_room_for_the_stored_integrals_takes_less(waters, tile, together):
+    """The failure moved through every allocation of a set-up: PFE_ENOMEM, but at the memory of the stored
+    integrals, of which a set-up then takes less (instead of a buffer per class one for all, whose build has the
+    same launches; instead of tiles of 16 MiB ones of 4, whose build has more) and builds the same."""
+    L = capi.lib()
+    sysm = waters[1]
+    pc = _pc(sysm)
+    ref = fock.DeviceFock(sysm)
+    c_ref, x_ref = ref.from_pc(pc)
+    ref.close()
+    absorbed = []   # (position, launches) of the set-ups that succeeded
+    L.pfe_debug_integral_memory(tile, together)
+    try:
+        for after in range(1000):
+            h = ctypes.c_void_p()
+            capi.check(L, L.pfe_context_create(0, ctypes.byref(h)))
+            a, keep = sysm.pfe_args(None, None)
+            L.pfe_debug_fail_allocation(after)
+            rc = L.pfe_context_setup(h, ctypes.byref(a))
+            L.pfe_debug_fail_allocation(-1)
+            if rc == 0:
+                c = capi.PfeCensus()
+                capi.check(L, L.pfe_context_census(h, ctypes.byref(c)))
+                rc, oc, ox = _build(L, h, sysm, pc)
+                assert rc == 0, capi.last_error(L)
+                _close(oc.t(), c_ref)
+                _close(ox.t(), x_ref)
+                absorbed.append((after, c.kernel_launches))
+            else:
+                assert rc == -5, (after, rc, capi.last_error(L))
+            L.pfe_context_destroy(h)
+            if len(absorbed) == 2:   # the second lies beyond the set-up's last allocation
+                break
+    finally:
+        L.pfe_debug_fail_allocation(-1)
+        L.pfe_debug_integral_memory(0, 0)
+    (first, less), (last, whole) = absorbed
+    assert last == first + 2   # one allocation, that of the chunk flags, comes after the integrals'
+    assert less > whole if tile else less == whole
