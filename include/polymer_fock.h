@@ -209,8 +209,8 @@ int32_t pfe_batch_schedule(pfe_batch *b, pfe_kernel_stat *out, int32_t cap);
 
 /* Schedule autotuning (no counterpart in the reference): time every execution
  * variant of every quartet class on this context's screened work lists with the
- * device density d_p_p, keep the fastest for later builds.  Synchronous.  The
- * host entry point pfe_fourindex_eri runs it on its first call after a set-up. */
+ * device density d_p_p, keep the fastest for later builds.  Synchronous.  Without
+ * it (and in pfe_fourindex_eri) builds run the measured default schedule. */
 int32_t pfe_context_autotune(pfe_context *ctx, const double *d_p_p, const double *d_p_p_helix, void *stream);
 
 /* Force execution variant v (0..3 as in pfe_kernel_stat) on every quartet

@@ -53,9 +53,9 @@ int acquire_boys(int device, const double* igamma, cudaStream_t s, std::shared_p
 // is cut again for the requests that follow, so scratch does not add up: the work on it
 // must be ordered before theirs (a set-up's work is all on one stream; other callers wait
 // first).  Kept at most: 13.5 MiB of blocks (512 KiB, 1 MiB, then 2 MiB each; one water
-// molecule takes the first two) and the 64 MiB buffer; all of it is freed with the owner.  A block's memory may
-// still be read by a build in flight when the next set-up begins, so release_all waits
-// for the device, as cudaFree does.
+// molecule takes the first two) and the 64 MiB buffer; all of it is freed with the owner.
+// A block's memory may still be read by a build in flight when the next set-up begins, so
+// release_all waits for the device, as cudaFree does.
 struct DeviceMemory {
   static constexpr size_t kSmall = 256 << 10, kFirst = 512 << 10, kBlock = 2 << 20, kKept = 64 << 20;
   static constexpr int kBlocks = 8;

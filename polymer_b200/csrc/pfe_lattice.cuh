@@ -38,18 +38,19 @@ struct LatticeRun {
   // the recursion in FP32, the rest in FP64; n32 counts the FP32 quartets
   int far32;
   unsigned long long* n32;
-  int* queue;          // chunk counter of the straight-line kernels, zero at launch
+  int* queue;          // the class's chunk counters, zero at launch
   const int* tidx;     // primitive -> contracted function (-1: a ghost)
   // set where P_P or P_P_HELIX has a non-zero element of a ghost; null where the
   // interpreter runs a class in any case
   const int* ghost;
 };
 
-// The straight-line kernel of evaluated class (e1|e2) (e1 >= e2, swap: the
-// chunk's bra class is e2) on `grid` blocks of 128 threads, or null where the
-// class has more than 64 integrals (it keeps the op-table interpreter).
-// work-queue counters per lattice class launch (one per register pass)
+// Work-queue counters per lattice class: one per register pass of the straight-line
+// kernels, or one for k_lat_wide and one for the interpreter after it.
 constexpr int kLatQueueSlots = 8;
+// The straight-line kernel of evaluated class (e1|e2) (e1 >= e2, swap: the chunk's bra
+// class is e2) on `grid` blocks of 128 threads, in one launch or a launch per register
+// pass, or null for the classes that run one quartet per warp.
 using LatSlFn = void (*)(const LatticeRun&, int grid, cudaStream_t);
 LatSlFn lattice_sl_launcher(int e1, int e2, bool sw);
 // The warp-per-quartet kernel of a class with d shells for bases whose d shells are all

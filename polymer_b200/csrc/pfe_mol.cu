@@ -28,8 +28,10 @@
 //     symmetry weight, into X(abcd) of the group quartet; X is then digested
 //     once against the target-space density into J'/K' (FP64 atomics; the
 //     bra's J' warp-reduced first).  Straight-line code with one group quartet
-//     per lane, or the op-table interpreter with one (warp) or all (block)
-//     threads per primitive quartet and X in shared memory;
+//     per lane, whose X goes to memory and through a digestion kernel over block
+//     panels (pfe_mol_digest.cu), or the op-table interpreter with one (warp) or
+//     all (block) threads per primitive quartet and X in shared memory, digested
+//     in place;
 //   * C_C = J' + J'^T and X_C = K' + K'^T (contracted targets), or the cuBLAS
 //     contraction CC (J'+J'^T) CC^T for primitive targets.
 
@@ -936,11 +938,6 @@ static int exclusive_sum(pfe_context* ctx, const int* in, int* out, int n, cudaS
   return PFE_OK;
 }
 
-// Shared memory of the wide variant (pfe_mol_wide.cu) for this molecule's
-// shells: the slots of the largest op table one of its group quartets can take
-// (the pure-bra or bra-and-ket table when no shell of the bra or ket kind has a
-// target on a lower component) and the kept outputs of its largest group
-// quartet; warps per block chosen for the most resident warps per SM.
 // bit L: some shell of top angular momentum L has a coefficient on a lower component
 static int lower_kept_bits(const pfe_context* ctx) {
   int bits = 0;
@@ -971,6 +968,11 @@ static const OpTableHost* bra_table(int cb, int ck, bool lower_d) {
   return (cb == 5 && ck == 4 && !lower_d) ? host_optable_topd(cb, ck) : host_optable_pure(cb, ck);
 }
 
+// Shared memory of the wide variant (pfe_mol_wide.cu) for this molecule's
+// shells: the slots of the largest op table one of its group quartets can take
+// (the pure-bra or bra-and-ket table when no shell of the bra or ket kind has a
+// target on a lower component) and the kept outputs of its largest group
+// quartet; warps per block chosen for the most resident warps per SM.
 static int size_wide(ClassLaunch& cl, const int kept_max[3], const bool lower_kept[3]) {
   cl.has_wide = false;
   const WideVariant wv = wide_variant(cl.cb, cl.ck);
@@ -1017,10 +1019,7 @@ static GroupView group_view(const pfe_context* ctx) {
   return GroupView{ctx->d_bk_list, ctx->d_gr_start, ctx->d_gr_n, ctx->pairs.schwarz, ctx->inttol};
 }
 
-// The chunk lists the kernels run, from the raw chunks of one molecule or of every
-// instance of a batch (`own`, a context or a batch, holds the memory): chunks much
-// longer than an even share of their class's work are cut into pieces, and every
-// class's pieces are sorted costliest first for its work queue.
+// The longest piece of a class whose chunks walk `steps` steps in all (finish_chunks).
 //
 // Why cut: a lane walks all primitive quartets of its group quartet in turn (up to
 // thousands where both groups are products of long contractions), so in a small
@@ -1158,6 +1157,10 @@ static int alloc_integrals(Owner* own, ClassLaunch* launches, int nlaunch, int b
   return PFE_OK;
 }
 
+// The chunk lists the kernels run, from the raw chunks of one molecule or of every
+// instance of a batch (`own`, a context or a batch, holds the memory): chunks much
+// longer than an even share of their class's work are cut into pieces, and every
+// class's pieces are sorted costliest first for its work queue.
 template <typename Owner>
 static int finish_chunks(Owner* own, pfe_context* const* inst, int ninst, ClassLaunch* launches, int nlaunch,
                          cudaStream_t s) {

@@ -15,8 +15,8 @@
 //   * the bra is the warp's, so J'(ab) is summed over the lanes first.
 // The multiply-adds (six per integral) run per lane from registers.
 // Measured, C20H42 6-31G** (B200): (21|11) 2.9 ms inside its nine passes, 0.7 ms here;
-// (11|10) 2.4 and 0.9 ms; all classes 17 and 8 ms, of which the stored integrals' traffic
-// (written and read once) is about 1 ms.
+// (11|10) 2.4 and 0.9 ms; all classes 17 and 6.9 ms.  A tile's integrals are read once, at
+// a quarter of the DRAM rate: the kernel waits on loads with 16 warps per SM.
 
 #include <algorithm>
 
