@@ -24,6 +24,11 @@ __host__ __device__ constexpr int ncum(int L) { return (L + 1) * (L + 2) * (L + 
 
 void set_error(const std::string& msg);
 
+// Dynamic shared memory a kernel whose blocks' size depends on the molecule is allowed: all a
+// block can have.  The limit belongs to the kernel on its device, not to a context, so one
+// context's set-up must not lower it below what another's launches need.
+constexpr int kMostSmem = 227 * 1024;
+
 #define PFE_CUDA(call)                                                                   \
   do {                                                                                   \
     cudaError_t e_ = (call);                                                             \

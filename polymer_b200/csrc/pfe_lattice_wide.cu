@@ -223,7 +223,7 @@ int launch_wide(const LatticeRun& r, const OpTableDev& t, int nx, int nchunks, i
   const int wpb = (int)std::max<size_t>(1, std::min<size_t>(4, cap / 4 / one));
   const size_t smem = one * wpb;
   auto kern = k_lat_wide<LA, LB, LC, LD, SWAP>;
-  PFE_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+  PFE_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, kMostSmem));
   const int per_sm = std::max(1, std::min(16, (int)(cap / smem)));
   const long long work = (32ll * nchunks + wpb - 1) / wpb;
   const int grid = (int)std::max<long long>(1, std::min<long long>(work, (long long)num_sms * per_sm));

@@ -1001,7 +1001,7 @@ static int size_wide(ClassLaunch& cl, const int kept_max[3], const bool lower_ke
   cl.wide_per_warp = (int)(pw / sizeof(double));
   cl.wide_wpb = best;
   cl.smem_wide = pw * best;
-  PFE_CUDA(wv.allow(cl.smem_wide));
+  PFE_CUDA(wv.allow());
   cl.has_wide = true;
   return PFE_OK;
 }

@@ -278,9 +278,9 @@ void launch_wide(const MolLaunch& ql, const OpTableDev& t, int grid, int wpb, in
 }
 
 template <int LA, int LB, int LC, int LD>
-cudaError_t allow_wide(size_t smem) {
+cudaError_t allow_wide() {
   const cudaError_t e =
-      cudaFuncSetAttribute(k_gq_wide<LA, LB, LC, LD>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+      cudaFuncSetAttribute(k_gq_wide<LA, LB, LC, LD>, cudaFuncAttributeMaxDynamicSharedMemorySize, kMostSmem);
   if (e != cudaSuccess) return e;
   // ask for no more shared memory than the blocks use: the rest of the SM's
   // 256 KB is L1, where the op table the warps read stays resident

@@ -12,7 +12,7 @@ struct WideVariant {
   // vmax hold the op-table slots and xmax the kept outputs of a group quartet
   void (*launch)(const MolLaunch&, const OpTableDev&, int grid, int wpb, int per_warp, int vmax, int xmax,
                  size_t smem, cudaStream_t);
-  cudaError_t (*allow)(size_t smem);
+  cudaError_t (*allow)();
   int (*doubles)(int vmax, int xmax);
 };
 
