@@ -29,10 +29,27 @@ void set_error(const std::string& msg);
 // context's set-up must not lower it below what another's launches need.
 constexpr int kMostSmem = 227 * 1024;
 
+// Launches that return no status (launchers behind function pointers): a launch refused by
+// the runtime shows in cudaGetLastError only until the next call that succeeds (CUDA 12.9),
+// so every launch is followed by note_launch(), and whoever called them by
+// PFE_CUDA(launch_status()).  Each thread has its own.
+inline thread_local cudaError_t t_launch = cudaSuccess;   // the first failure not yet reported
+inline void note(cudaError_t e) {
+  if (e != cudaSuccess && t_launch == cudaSuccess) t_launch = e;
+}
+inline void note_launch() { note(cudaGetLastError()); }
+inline cudaError_t launch_status() {
+  note_launch();
+  const cudaError_t e = t_launch;
+  t_launch = cudaSuccess;
+  return e;
+}
+
 #define PFE_CUDA(call)                                                                   \
   do {                                                                                   \
     cudaError_t e_ = (call);                                                             \
     if (e_ != cudaSuccess) {                                                             \
+      ::pfe::t_launch = cudaSuccess;                                                     \
       ::pfe::set_error(std::string(#call) + ": " + cudaGetErrorString(e_));             \
       return (e_ == cudaErrorMemoryAllocation) ? PFE_ENOMEM : PFE_ECUDA;               \
     }                                                                                    \

@@ -50,10 +50,12 @@ __global__ void k_select_class_impl(const unsigned char* __restrict__ cls, int w
 void launch_symmetrize(const double* a, double* out, int n, int ncell, cudaStream_t s) {
   const long long t = (long long)n * n * ncell;
   k_symmetrize_impl<<<(unsigned)((t + 255) / 256), 256, 0, s>>>(a, out, n, ncell);
+  note_launch();
 }
 
 void launch_select_class(const unsigned char* cls, int want, int* list, int* count, long long n, cudaStream_t s) {
   k_select_class_impl<<<(unsigned)((n + 255) / 256), 256, 0, s>>>(cls, want, list, count, n);
+  note_launch();
 }
 
 const OpTableHost* host_optable(int cb, int ck) {
@@ -267,7 +269,7 @@ int contract_outputs(pfe_context* ctx, const double* jp, const double* kp, doubl
     if (st != CUBLAS_STATUS_SUCCESS) { set_error("cublasDgemmStridedBatched (W.CC^T) failed"); return PFE_ECUDA; }
     if (symmetrize) {
       launch_symmetrize(ctx->d_w2, dst[o], nc, ncell, s);
-      PFE_CUDA(cudaGetLastError());
+      PFE_CUDA(launch_status());
     }
   }
   return PFE_OK;
@@ -300,10 +302,12 @@ int measure_fp64_peak(int device, double* tflops) {
   PFE_CUDA(cudaEventCreate(&e0));
   PFE_CUDA(cudaEventCreate(&e1));
   k_dfma_peak<<<blocks, threads>>>(d, 64, 0.999999, 1e-7);  // warm-up
+  PFE_CUDA(cudaGetLastError());
   float best = 1e30f;
   for (int r = 0; r < 5; ++r) {
     PFE_CUDA(cudaEventRecord(e0));
     k_dfma_peak<<<blocks, threads>>>(d, iters, 0.999999, 1e-7);
+    PFE_CUDA(cudaGetLastError());
     PFE_CUDA(cudaEventRecord(e1));
     PFE_CUDA(cudaEventSynchronize(e1));
     float ms = 0.f;

@@ -298,6 +298,7 @@ template <int LA, int LB, int LC, int LD, bool BLOCK>
 void launch_grad(const MolLaunch& ql, const GradTables& t, const GradOut& go, int vmax, int per_team, int grid,
                  int threads, size_t smem, cudaStream_t s) {
   k_grad<LA, LB, LC, LD, BLOCK><<<grid, threads, smem, s>>>(ql, t, go, vmax, per_team);
+  note_launch();
 }
 
 template <int LA, int LB, int LC, int LD, bool BLOCK>
@@ -410,7 +411,7 @@ int molecular_gradient(pfe_context* ctx, const double* d_dt, const int* d_satom,
     ql.nchunks = g.cl->d_nchunks;
     g.fn(ql, g.t, go, g.vmax, g.per_team, g.grid, g.threads, g.smem, ctx->side[g.side]);
   }
-  PFE_CUDA(cudaGetLastError());
+  PFE_CUDA(launch_status());
   PFE_CUDA(sides.join());
   return PFE_OK;
 }

@@ -424,6 +424,7 @@ template <int LA, int LB, int LC, int LD, bool SW>
 static void launch_lat(const LatticeRun& r, const OpTableDev& t, int grid, int wpb, int per_warp, size_t smem,
                        cudaStream_t s) {
   k_lattice<LA, LB, LC, LD, SW><<<grid, 32 * wpb, smem, s>>>(r, t, per_warp);
+  note_launch();
 }
 template <int LA, int LB, int LC, int LD, bool SW>
 static cudaError_t allow_lat(size_t smem, int threads, int* resident) {
@@ -490,6 +491,7 @@ static int compute_schwarz(pfe_context* ctx, PairArrays recs, long long n, cudaS
   for (int cls = 4; cls <= 5; ++cls) {
     PFE_CUDA(cudaMemsetAsync(cnt, 0, sizeof(int), s));
     k_select_cls<<<(unsigned)((n + 255) / 256), 256, 0, s>>>(recs.cls, cls, list, cnt, n);
+    PFE_CUDA(cudaGetLastError());
     int hn = 0;
     PFE_CUDA(cudaMemcpyAsync(&hn, cnt, sizeof(int), cudaMemcpyDeviceToHost, s));
     PFE_CUDA(cudaStreamSynchronize(s));
@@ -502,11 +504,12 @@ static int compute_schwarz(pfe_context* ctx, PairArrays recs, long long n, cudaS
     if (cls == 4) {
       PFE_CUDA(cudaFuncSetAttribute(k_schwarz_big<2, 1>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
       k_schwarz_big<2, 1><<<std::min(hn, 4 * ctx->num_sms), 256, smem, s>>>(recs, ctx->shells.prim, ctx->d_maxc, list, hn, d);
+      PFE_CUDA(cudaGetLastError());
     } else {
       PFE_CUDA(cudaFuncSetAttribute(k_schwarz_big<2, 2>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
       k_schwarz_big<2, 2><<<std::min(hn, 4 * ctx->num_sms), 256, smem, s>>>(recs, ctx->shells.prim, ctx->d_maxc, list, hn, d);
+      PFE_CUDA(cudaGetLastError());
     }
-    PFE_CUDA(cudaGetLastError());
     PFE_CUDA(cudaStreamSynchronize(s));
   }
   ctx->free_now(list);
@@ -609,6 +612,7 @@ int lattice_setup(pfe_context* ctx, const pfe_args* a) {
     PFE_CUDA(ctx->alloc((void**)&l1, sizeof(unsigned short) * ntot));
     PFE_CUDA(ctx->alloc((void**)&l2, sizeof(unsigned short) * ntot));
     k_iota_lat<<<(unsigned)((ntot + 255) / 256), 256, 0, s>>>(pa, ntot);
+    PFE_CUDA(cudaGetLastError());
     size_t t1 = 0, t2 = 0, t3 = 0;
     cub::DeviceRadixSort::SortPairs(nullptr, t1, raw.key, kb, pa, pb, (int)ntot, 0, 64, s);
     cub::DeviceRadixSort::SortPairs(nullptr, t2, c1, c2, pb, pa, (int)ntot, 0, 8, s);
@@ -619,10 +623,13 @@ int lattice_setup(pfe_context* ctx, const pfe_args* a) {
     size_t tbb = tb;
     PFE_CUDA(cub::DeviceRadixSort::SortPairs(tmp, tbb, raw.key, kb, pa, pb, (int)ntot, 0, 64, s));
     k_gather_u8_lat<<<(unsigned)((ntot + 255) / 256), 256, 0, s>>>(raw.cls, pb, c1, ntot);
+    PFE_CUDA(cudaGetLastError());
     tbb = tb;
     PFE_CUDA(cub::DeviceRadixSort::SortPairs(tmp, tbb, c1, c2, pb, pa, (int)ntot, 0, 8, s));
     k_lat_listkey<<<(unsigned)((ntot + 255) / 256), 256, 0, s>>>(l2, L->npl, ntot);
+    PFE_CUDA(cudaGetLastError());
     k_gather_u16<<<(unsigned)((ntot + 255) / 256), 256, 0, s>>>(l2, pa, l1, ntot);
+    PFE_CUDA(cudaGetLastError());
     tbb = tb;
     PFE_CUDA(cub::DeviceRadixSort::SortPairs(tmp, tbb, l1, l2, pa, pb, (int)ntot, 0, 16, s));
     k_lat_gather<<<(unsigned)((ntot + 127) / 128), 128, 0, s>>>(raw, sw_raw, L->pairs, L->swp, pb, ntot);
@@ -817,7 +824,7 @@ int lattice_fock(pfe_context* ctx, const double* d_pp, const double* d_pph, doub
                           (long long)ctx->npgs * ctx->npgs * (2 * ctx->cel2[0] + 1) *
                               (2 * (ctx->cel2[0] + ctx->cel1[0]) + 1),
                           ctx->npgs, ctx->d_tidx, L->d_ghost, ctx->num_sms, s);
-    PFE_CUDA(cudaGetLastError());
+    PFE_CUDA(launch_status());
   }
   for (int i = 0; i < L->nlaunch; ++i) {
     const LatticeLaunch& ll = L->launches[i];
@@ -843,7 +850,7 @@ int lattice_fock(pfe_context* ctx, const double* d_pp, const double* d_pph, doub
       const int grid = std::min((ll.ncells_chunks + ll.wpb - 1) / ll.wpb, ctx->num_sms * std::max(1, ll.resident));
       lat_variant(e1, e2, ll.cb < ll.ck).fn(R, ll.tab, std::max(grid, 1), ll.wpb, ll.per_warp, ll.smem, s);
     }
-    PFE_CUDA(cudaGetLastError());
+    PFE_CUDA(launch_status());
   }
   int rc = contract_outputs(ctx, ctx->d_jp, ctx->d_kp, d_cc, d_xc, /*symmetrize=*/false, ctx->ncell1, s);
   if (rc != PFE_OK) return rc;

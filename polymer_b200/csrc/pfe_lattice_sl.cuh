@@ -276,6 +276,7 @@ __global__ void __launch_bounds__(128) k_lat_sl(LatticeRun R) {
 template <int LA, int LB, int LC, int LD, bool SW>
 void launch_sl(const LatticeRun& r, int grid, cudaStream_t s) {
   k_lat_sl<LA, LB, LC, LD, SW><<<grid, 128, 0, s>>>(r);
+  note_launch();
 }
 
 // The register passes of a class, one launch each on its own work-queue counter
@@ -286,6 +287,7 @@ void launch_sl_passes(const LatticeRun& r, int grid, cudaStream_t s) {
   LatticeRun rp = r;
   rp.queue = r.queue + PASS;
   k_lat_sl<LA, LB, LC, LD, SW, NPASS, PASS><<<grid, 128, 0, s>>>(rp);
+  note_launch();
   if constexpr (PASS + 1 < NPASS) launch_sl_passes<LA, LB, LC, LD, SW, NPASS, PASS + 1>(r, grid, s);
 }
 

@@ -245,6 +245,7 @@ __global__ void k_ghost_check(const double* __restrict__ p, long long n, int npg
 void lattice_ghost_check(const double* p, long long n, int npgs, const int* tidx, int* flag, int num_sms,
                          cudaStream_t s) {
   k_ghost_check<<<(unsigned)std::min<long long>((n + 255) / 256, 16ll * num_sms), 256, 0, s>>>(p, n, npgs, tidx, flag);
+  note_launch();
 }
 
 // evaluated class (e1 >= e2) and swap flag -> launcher, or null for the classes without a

@@ -859,12 +859,14 @@ using WarpFn = void (*)(const MolLaunch&, const OpTableDev&, int grid, int wpb, 
 template <int LA, int LB, int LC, int LD>
 static void launch_big(const MolLaunch& ql, const OpTableDev& t, double* xg, int grid, size_t smem, cudaStream_t s) {
   k_gq_block<LA, LB, LC, LD><<<grid, 256, smem, s>>>(ql, t, xg);
+  note_launch();
 }
 
 template <int LA, int LB, int LC, int LD>
 static void launch_warp(const MolLaunch& ql, const OpTableDev& t, int grid, int wpb, int per_warp, size_t smem,
                         cudaStream_t s) {
   k_gq_warp<LA, LB, LC, LD><<<grid, 32 * wpb, smem, s>>>(ql, t, per_warp);
+  note_launch();
 }
 
 template <int LA, int LB, int LC, int LD>
@@ -1204,6 +1206,7 @@ static int finish_chunks(Owner* own, pfe_context* const* inst, int ninst, ClassL
       if (c->nraw == 0) continue;
       k_piece_count<<<(c->nraw + 127) / 128, 128, 0, s>>>(c->d_raw, c->d_raw_pair, c->d_raw_steps, c->nraw,
                                                           group_view(c), pm, npiece + o);
+      PFE_CUDA(cudaGetLastError());
       o += c->nraw;
     }
     PFE_CUDA(cudaGetLastError());
@@ -1236,6 +1239,7 @@ static int finish_chunks(Owner* own, pfe_context* const* inst, int ninst, ClassL
       const int n = first[k + 1] - first[k];
       if (n > 0) k_piece_fill<<<(n + 3) / 4, 128, 0, s>>>(c->d_raw, c->d_raw_pair, c->d_raw_steps, c->d_raw_cost, c->nraw,
                                                      group_view(c), pm, k, off + o, pieces, key, d_stat);
+      PFE_CUDA(cudaGetLastError());
       o += c->nraw;
     }
     k_mol_iota<<<(total + 255) / 256, 256, 0, s>>>(iota, total);
@@ -1292,6 +1296,7 @@ int molecular_setup(pfe_context* ctx, const pfe_args* a) {
     for (int cls = 4; cls <= 5; ++cls) {
       PFE_CUDA(cudaMemsetAsync(cnt, 0, sizeof(int), s));
       launch_select_class(raw.cls, cls, list, cnt, npairs, s);
+      PFE_CUDA(launch_status());
       int hn = 0;
       PFE_CUDA(cudaMemcpyAsync(&hn, cnt, sizeof(int), cudaMemcpyDeviceToHost, s));
       PFE_CUDA(cudaStreamSynchronize(s));
@@ -1303,11 +1308,12 @@ int molecular_setup(pfe_context* ctx, const pfe_args* a) {
       if (cls == 4) {
         PFE_CUDA(cudaFuncSetAttribute(k_schwarz_big<2, 1>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
         k_schwarz_big<2, 1><<<std::min(hn, 4 * ctx->num_sms), 256, smem, s>>>(raw, ctx->shells.prim, ctx->d_maxc, list, hn, d);
+        PFE_CUDA(cudaGetLastError());
       } else {
         PFE_CUDA(cudaFuncSetAttribute(k_schwarz_big<2, 2>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
         k_schwarz_big<2, 2><<<std::min(hn, 4 * ctx->num_sms), 256, smem, s>>>(raw, ctx->shells.prim, ctx->d_maxc, list, hn, d);
+        PFE_CUDA(cudaGetLastError());
       }
-      PFE_CUDA(cudaGetLastError());
       PFE_CUDA(cudaStreamSynchronize(s));
     }
     ctx->free_now(list);
@@ -1330,17 +1336,22 @@ int molecular_setup(pfe_context* ctx, const pfe_args* a) {
   PFE_CUDA(ctx->alloc((void**)&k8b, npairs));
   PFE_CUDA(cudaMemsetAsync(gbits, 0, sizeof(unsigned long long) * ngid, s));
   k_mol_groupmax<<<nb256, 256, 0, s>>>(raw.schwarz, raw.gid, gbits, npairs);
+  PFE_CUDA(cudaGetLastError());
   k_mol_keys<<<nb256, 256, 0, s>>>(raw.schwarz, raw.gid, gbits, k_sch, k_gmax, raw.gmax, npairs);
+  PFE_CUDA(cudaGetLastError());
   k_mol_iota<<<nb256, 256, 0, s>>>(perm_a, npairs);
   PFE_CUDA(cudaGetLastError());
   {
     const int n = (int)npairs;
     if ((rc = radix_sort_pairs(ctx, k_sch, k64, perm_a, perm_b, n, 64, s)) != PFE_OK) return rc;
     k_gather_t<int><<<nb256, 256, 0, s>>>(raw.gid, perm_b, k32, npairs);
+    PFE_CUDA(cudaGetLastError());
     if ((rc = radix_sort_pairs(ctx, k32, k32b, perm_b, perm_a, n, 32, s)) != PFE_OK) return rc;
     k_gather_t<unsigned long long><<<nb256, 256, 0, s>>>(k_gmax, perm_a, k_sch, npairs);
+    PFE_CUDA(cudaGetLastError());
     if ((rc = radix_sort_pairs(ctx, k_sch, k64, perm_a, perm_b, n, 64, s)) != PFE_OK) return rc;
     k_gather_t<unsigned char><<<nb256, 256, 0, s>>>(raw.cls, perm_b, k8, npairs);
+    PFE_CUDA(cudaGetLastError());
     if ((rc = radix_sort_pairs(ctx, k8, k8b, perm_b, perm_a, n, 8, s)) != PFE_OK) return rc;
     k_mol_gather<<<(unsigned)((npairs + 127) / 128), 128, 0, s>>>(raw, ctx->pairs, perm_a, npairs);
     PFE_CUDA(cudaGetLastError());
@@ -1364,6 +1375,7 @@ int molecular_setup(pfe_context* ctx, const pfe_args* a) {
   PFE_CUDA(ctx->alloc((void**)&head, sizeof(int) * npairs));
   PFE_CUDA(ctx->alloc((void**)&gix, sizeof(int) * npairs));
   k_group_heads<<<nb256, 256, 0, s>>>(ctx->pairs.gid, head, npairs);
+  PFE_CUDA(cudaGetLastError());
   if ((rc = exclusive_sum(ctx, head, gix, (int)npairs, s)) != PFE_OK) return rc;
   int last_gix = 0, last_head = 0;
   PFE_CUDA(cudaMemcpyAsync(&last_gix, gix + npairs - 1, sizeof(int), cudaMemcpyDeviceToHost, s));
@@ -1383,7 +1395,9 @@ int molecular_setup(pfe_context* ctx, const pfe_args* a) {
   PFE_CUDA(ctx->alloc((void**)&giota, sizeof(int) * ng));
   k_group_fill<<<nb256, 256, 0, s>>>(head, gix, ctx->pairs.schwarz, ctx->pairs.cls, ctx->d_gr_start, ctx->d_gr_max,
                                      gr_cls, npairs);
+  PFE_CUDA(cudaGetLastError());
   k_group_size<<<(ng + 255) / 256, 256, 0, s>>>(ctx->d_gr_start, gr_cls, ng, npairs, ctx->d_gr_n, bkey);
+  PFE_CUDA(cudaGetLastError());
   k_mol_iota<<<(ng + 255) / 256, 256, 0, s>>>(giota, ng);
   PFE_CUDA(cudaGetLastError());
   if ((rc = radix_sort_pairs(ctx, bkey, bkey_sorted, giota, ctx->d_bk_list, ng, 8, s)) != PFE_OK) return rc;
@@ -1473,6 +1487,7 @@ int molecular_setup(pfe_context* ctx, const pfe_args* a) {
       PFE_CUDA(ctx->alloc((void**)&ctx->d_raw_cost, sizeof(unsigned int) * total));
       k_chunk_fill<<<(nrow + 127) / 128, 128, 0, s>>>(ctx->d_gr_max, ctx->d_bk_list, ctx->d_gr_n, rows, ctx->inttol,
                                                       offs, ctx->d_raw, ctx->d_raw_pair);
+      PFE_CUDA(cudaGetLastError());
       k_chunk_census<<<(total + 3) / 4, 128, 0, s>>>(ctx->d_raw, ctx->d_raw_pair, total, group_view(ctx), serial,
                                                      ctx->d_raw_steps, ctx->d_raw_cost, d_stat);
       PFE_CUDA(cudaGetLastError());
@@ -1637,7 +1652,7 @@ static void launch_class(pfe_context* ctx, const ClassLaunch& cl, MolLaunch ql, 
     const bool stored = cl.cb > 0;
     const int cap = stored ? cl.xcap : std::max(work, 1);
     for (int t0 = 0; t0 < work; t0 += cap) {
-      if (t0 > 0) cudaMemsetAsync(cl.queue, 0, sizeof(int) * 64, s);
+      if (t0 > 0) note(cudaMemsetAsync(cl.queue, 0, sizeof(int) * 64, s));
       ql.t0 = t0;
       ql.tn = std::min(cap, work - t0);
       ql.xbuf = cl.xbuf;
@@ -1674,9 +1689,11 @@ static const double* target_density(pfe_context* ctx, const double* d_pp, cudaSt
   const long long nt2 = (long long)ctx->nt * ctx->nt, np2 = (long long)ctx->npgs * ctx->npgs;
   k_target_density<<<(unsigned)((nt2 + 255) / 256), 256, 0, s>>>(d_pp, ctx->npgs, ctx->d_rep, ctx->d_repc, ctx->nt,
                                                                    ctx->d_pt);
-  cudaMemsetAsync(ctx->d_flag, 0, sizeof(unsigned int), s);
+  note_launch();
+  note(cudaMemsetAsync(ctx->d_flag, 0, sizeof(unsigned int), s));
   k_check_density<<<(unsigned)((np2 + 255) / 256), 256, 0, s>>>(d_pp, ctx->npgs, ctx->d_tidx, ctx->d_tcoef,
                                                                   ctx->d_pt, ctx->nt, ctx->d_flag);
+  note_launch();
   return ctx->d_pt;
 }
 
@@ -1741,7 +1758,7 @@ static int tune_class(pfe_context* ctx, ClassLaunch& cl, const MolLaunch& ql, cu
     for (int gi = 0; gi < ng; ++gi) {
       if (ng > 1) cl.gmul = kGmul[gi];
       auto once = [&]() {
-        cudaMemsetAsync(cl.queue, 0, sizeof(int) * 64, s);
+        note(cudaMemsetAsync(cl.queue, 0, sizeof(int) * 64, s));
         launch_class(ctx, cl, ql, v, s, mixed);
       };
       once();
@@ -1755,7 +1772,7 @@ static int tune_class(pfe_context* ctx, ClassLaunch& cl, const MolLaunch& ql, cu
         PFE_CUDA(cudaEventElapsedTime(&ms, e0, e1));
         t = std::min(t, ms);
       }
-      PFE_CUDA(cudaGetLastError());
+      PFE_CUDA(launch_status());
       tv = std::min(tv, t);
       if (t < best) { best = t; bestv = v; bestg = cl.gmul; }
     }
@@ -1768,6 +1785,7 @@ static int tune_class(pfe_context* ctx, ClassLaunch& cl, const MolLaunch& ql, cu
 
 int autotune(pfe_context* ctx, const double* d_pp, cudaStream_t s) {
   const double* d_dt = target_density(ctx, d_pp, s);
+  PFE_CUDA(launch_status());
   const MolLaunch ql = make_launch(ctx, d_dt);
   const int rc0 = begin_build(ctx, d_dt, s);
   if (rc0 != PFE_OK) return rc0;
@@ -1840,7 +1858,7 @@ static int launch_classes(pfe_context* cx, const ClassLaunch* launches, int nlau
     const ClassLaunch& cl = launches[order[j]];
     launch_class(cx, cl, ql, cl.variant, on[order[j]], mixed);
   }
-  PFE_CUDA(cudaGetLastError());
+  PFE_CUDA(launch_status());
   PFE_CUDA(sides.join());
   return PFE_OK;
 }
@@ -1862,7 +1880,7 @@ static int run_build(pfe_context* ctx, const double* d_dt, double* d_cc, double*
   for (int i = 0; i < ctx->nlaunch && ctx->profile; ++i) {
     const ClassLaunch& cl = ctx->launches[i];
     launch_class(ctx, cl, ql, cl.variant, s, ctx->mcut > 0.0);
-    PFE_CUDA(cudaGetLastError());
+    PFE_CUDA(launch_status());
     {
       PFE_CUDA(cudaEventRecord(ctx->ev[i + 1], s));
       ctx->ev_cls[i] = 1000 * kCL[cl.cb][0] + 100 * kCL[cl.cb][1] + 10 * kCL[cl.ck][0] + kCL[cl.ck][1];
@@ -1878,7 +1896,7 @@ static int run_build(pfe_context* ctx, const double* d_dt, double* d_cc, double*
 
 int molecular_fock(pfe_context* ctx, const double* d_pp, double* d_cc, double* d_xc, cudaStream_t s) {
   const double* d_dt = target_density(ctx, d_pp, s);
-  PFE_CUDA(cudaGetLastError());
+  PFE_CUDA(launch_status());
   return run_build(ctx, d_dt, d_cc, d_xc, s);
 }
 
@@ -1911,7 +1929,7 @@ int molecular_gradient(pfe_context* ctx, const double* d_dt, const int* d_satom,
 int molecular_gradient_pp(pfe_context* ctx, const double* d_pp, const int* d_satom, int natom, double* d_gj,
                           double* d_gk, cudaStream_t s) {
   const double* d_dt = target_density(ctx, d_pp, s);
-  PFE_CUDA(cudaGetLastError());
+  PFE_CUDA(launch_status());
   return molecular_gradient(ctx, d_dt, d_satom, natom, d_gj, d_gk, s);
 }
 
@@ -2143,6 +2161,7 @@ int batch_fock_pc(pfe_batch* b, const double* d_pc, double* d_cc, double* d_xc, 
   const dim3 gb(8, (unsigned)n);
   const PanelView* dv = reinterpret_cast<const PanelView*>(di + n);
   k_batch_zero<<<gb, 256, 0, s>>>(di, dv, b->d_queue);
+  PFE_CUDA(cudaGetLastError());
   k_batch_dmax<<<gb, 256, 0, s>>>(di);
   PFE_CUDA(cudaGetLastError());
   pfe_context* c0 = b->inst[0];
@@ -2155,6 +2174,7 @@ int batch_fock_pc(pfe_batch* b, const double* d_pc, double* d_cc, double* d_xc, 
   }
   if (b->all_contracted) {
     k_batch_symmetrize<<<gb, 256, 0, s>>>(di, dv, b->d_off, d_cc, d_xc);
+    PFE_CUDA(cudaGetLastError());
   } else {
     for (size_t k = 0; k < n; ++k) {
       const int rc = finish_build(b->inst[k], d_cc + b->off[k], d_xc + b->off[k], s);

@@ -240,9 +240,10 @@ void run(const MolLaunch& ql, int num_sms, cudaStream_t s) {
   using S = DigestShape<LA, LB, LC, LD, KEPT>;
   constexpr int bytes = S::PER_WARP * S::WARPS * 8;
   auto kern = k_digest<LA, LB, LC, LD, KEPT>;
-  cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
+  note(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes));
   const int grid = std::min((ql.tn + S::WARPS - 1) / S::WARPS, num_sms * S::BLOCKS);
   kern<<<std::max(grid, 1), 32 * S::WARPS, bytes, s>>>(ql);
+  note_launch();
 }
 
 // the kept bits that matter to a class: those of the angular momenta it has

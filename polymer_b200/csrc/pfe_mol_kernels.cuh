@@ -600,10 +600,11 @@ void launch_groups(const MolLaunch& ql, unsigned long long live, int grid, cudaS
     // `grid` counts blocks of four warps
     int g = grid;
     if constexpr (O::staged) {
-      cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes);
+      note(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes));
       g = std::max(1, std::min((grid * 128 + O::threads - 1) / O::threads, O::blocks * ql.num_sms));
     }
     kern<<<dim3(g, __builtin_popcount(m)), O::threads, bytes, s>>>(ql, m);
+    note_launch();
   }
   if constexpr (P0 + PN < NPASS)
     launch_groups<LA, LB, LC, LD, KEPT, NPASS, P0 + PN, MIXED, BATCH, OWN>(ql, live, grid, s);

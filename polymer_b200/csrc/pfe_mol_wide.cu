@@ -275,6 +275,7 @@ template <int LA, int LB, int LC, int LD>
 void launch_wide(const MolLaunch& ql, const OpTableDev& t, int grid, int wpb, int per_warp, int vmax, int xmax,
                  size_t smem, cudaStream_t s) {
   k_gq_wide<LA, LB, LC, LD><<<grid, 32 * wpb, smem, s>>>(ql, t, per_warp, vmax, xmax);
+  note_launch();
 }
 
 template <int LA, int LB, int LC, int LD>

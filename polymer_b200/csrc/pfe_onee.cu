@@ -309,6 +309,7 @@ static void launch_nuclear(const OneeDev& d, const int* list, const int* start, 
     const long long total = (long long)na * nb * cells;
     if (total > 0)
       kern<<<(unsigned)((total + 127) / 128), 128>>>(d, list + start[la], na, list + start[lb], nb, n_p);
+      note_launch();
   };
   run(k_nuclear<2, 2, false>, 2, 2);
   run(k_nuclear<2, 1, false>, 2, 1);
@@ -447,11 +448,12 @@ static int onee_run(const pfe_onee_args* a, double* s_p, double* t_p, double* n_
   PFE_CUDA(cudaMemsetAsync(out0, 0, nout * round256(out_bytes), nullptr));
   if (n_p) {
     launch_nuclear(d, i32(10), start, n1, out0);
+    PFE_CUDA(launch_status());
   } else {
     const long long total = (long long)a->npshell * a->npshell * n1;
     k_overlap_kinetic<<<(unsigned)((total + 127) / 128), 128>>>(d, out0, out1);
+    PFE_CUDA(cudaGetLastError());
   }
-  PFE_CUDA(cudaGetLastError());
   if (n_p) {
     PFE_CUDA(cudaMemcpy(n_p, out0, out_bytes, cudaMemcpyDeviceToHost));
   } else {

@@ -447,6 +447,7 @@ int32_t pfe_scf_fock_assemble(int32_t nb, int32_t n, const double* h, const doub
   cudaStream_t s = (cudaStream_t)stream;
   const int nt = tiles_of(n);
   k_fock_assemble<<<dim3(nt, nb), dim3(TS, 8), 0, s>>>(n, h, d_c, d_x, c_ref, x_ref, p, p_ref, incr, hfx, f, work);
+  PFE_CUDA(cudaGetLastError());
   k_finish_partials<false><<<nb, 32, 0, s>>>(work, nt, e_nuc, energy);
   PFE_CUDA(cudaGetLastError());
   return PFE_OK;
@@ -464,6 +465,7 @@ int32_t pfe_scf_commutator(int32_t nb, int32_t n, int32_t ndiis, const double* a
   cudaStream_t s = (cudaStream_t)stream;
   const int nt = tiles_of(n);
   k_commutator<<<dim3(nt, nb), dim3(TS, 8), 0, s>>>(n, ndiis, a, f_o, slot, hist_e, hist_f, valid, work);
+  PFE_CUDA(cudaGetLastError());
   k_finish_partials<true><<<nb, 32, 0, s>>>(work, nt, nullptr, err_max);
   PFE_CUDA(cudaGetLastError());
   return PFE_OK;
@@ -481,7 +483,9 @@ int32_t pfe_scf_diis(int32_t nb, int32_t n, int32_t ndiis, const double* hist_e,
   cudaStream_t s = (cudaStream_t)stream;
   const int nc = chunks_of(n);
   k_diis_row<<<dim3(nc, nb), 256, 0, s>>>(n, ndiis, hist_e, slot, work);
+  PFE_CUDA(cudaGetLastError());
   k_diis_solve<<<nb, 32, 0, s>>>(ndiis, nc, work, valid, slot, gram, coef);
+  PFE_CUDA(cudaGetLastError());
   k_diis_extrapolate<<<dim3(nc, nb), 256, 0, s>>>(n, ndiis, hist_f, coef, f_x);
   PFE_CUDA(cudaGetLastError());
   return PFE_OK;
@@ -509,6 +513,7 @@ int32_t pfe_scf_sp2_step(int32_t nb, int32_t n, int32_t nocc, double* x, const d
   if (nb == 0) return PFE_OK;
   cudaStream_t s = (cudaStream_t)stream;
   k_sp2_trace<<<nb, 32, 0, s>>>(n, nocc, x, x2, defect, work);
+  PFE_CUDA(cudaGetLastError());
   k_sp2_update<<<dim3(chunks_of(n), nb), 256, 0, s>>>(n, x, x2, work);
   PFE_CUDA(cudaGetLastError());
   return PFE_OK;
@@ -526,6 +531,7 @@ int32_t pfe_scf_finish(int32_t nb, int32_t n, double scale, const double* q, con
   cudaStream_t s = (cudaStream_t)stream;
   const int nc = chunks_of(n);
   k_finish<<<dim3(nc, nb), 256, 0, s>>>(n, scale, q, p, p_new, work);
+  PFE_CUDA(cudaGetLastError());
   k_finish_stats<<<nb, 32, 0, s>>>(n, nc, work, energy, err_max, defect, stats);
   PFE_CUDA(cudaGetLastError());
   return PFE_OK;
